@@ -427,7 +427,7 @@ def _step_bytes(case):
     """Bytes and operations of one timestep: every field value read and written once, a coefficient tuple (or its index)
     per cell, the UPML fluxes, the Mur pairs, the ADE state, the NF2FF samples."""
     n = case["nx"] * case["ny"] * case["nz"]
-    b = n * (48 + (4 if case["coef"] == "table" else 96 if case["coef"] == "unique" else 4))
+    b = n * (48 + (48 if case["coef"] == "unique" else 4))
     grid = (case["nx"], case["ny"], case["nz"])
     u = 0
     if case["pml"]:
