@@ -4,8 +4,8 @@
 // with its own fields, extensions, step counter and parity).  One timestep of
 // the batch is the engines' phase order with every phase issued once for all
 // members:
-//   * the core update is one persistent launch of k_fused_tma_batch (one per
-//     coefficient kind present: material index or dense): every
+//   * the core update is one persistent launch of k_fused_tma_batch per kind of
+//     tile present (material index or dense, with or without UPML / TFSF): every
 //     CTA walks a work-tile list spanning all members (tile = member, 64x8
 //     tile origin, x-chunk) and runs each tile through the same TMA plane
 //     pipeline as the single engine, reading the member's grid, UPML set and
@@ -27,25 +27,31 @@ namespace efs {
 
 // ---- core update over all members ------------------------------------------
 struct BatchMember {            // one member at one step parity (tensor maps first: 64-byte aligned)
-    CUtensorMap tmH, tmE, tmM, tmD;
+    CUtensorMap tmH, tmE, tmM, tmD, tmE1, tmH1;
     FusedGrid g;
     PmlSet ps;
 };
 struct BatchTile { uint32_t m, xs, y0, z0; };
 
 // Persistent: CTA b runs tiles b, b + gridDim.x, ... of a list whose members
-// all use material-index (IDX) or all dense coefficients.
-template <bool IDX>
+// all use material-index (IDX) or all dense coefficients and, if !SOME, whose
+// tiles meet neither a UPML region nor a TFSF face corrected in the update.
+// Tiles with and without that code are separate launches: with both bodies in
+// one kernel it spilled (32 stub filters: 620 us against 535 us a step).
+template <bool IDX, bool SOME>
 __global__ void __launch_bounds__(TT_THREADS, 2)
 k_fused_tma_batch(const BatchMember* __restrict__ mem, const BatchTile* __restrict__ tiles, uint32_t ntiles) {
     TmaSmem& S = tt_smem();
     tt_init(S);
-    uint32_t K = 0;                                    // planes this CTA has consumed
+    TmaRing rg;                                        // pipeline state across the CTA's tiles
     for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const BatchTile w = tiles[t];
         const BatchMember& M = mem[w.m];
-        if (!tma_tile_body<IDX, true, true>(S, &M.tmH, &M.tmE, &M.tmM, &M.tmD, M.g, M.ps, w.xs, w.y0, w.z0, K)) return;
+        if (!tma_tile_body<IDX, SOME, SOME>(S, TmaMaps{&M.tmH, &M.tmE, &M.tmM, &M.tmD, &M.tmE1, &M.tmH1}, M.g, M.ps, w.xs, w.y0,
+                                            w.z0, rg))
+            break;
     }
+    tt_done();
 }
 
 // ---- segmented sparse phases ------------------------------------------------
@@ -167,8 +173,8 @@ struct efs_batch {
     bool planned = false;
     std::vector<int> cur0;
     uint32_t phase = 0;
-    DevBuf members[2], tiles[2];               // tiles[1]: material-index members, tiles[0]: dense members
-    uint32_t ntiles[2] = {0, 0};
+    DevBuf members[2], tiles[4];               // tile lists by tile_class
+    uint32_t ntiles[4] = {0, 0, 0, 0};
     SegLaunch mur_pre[2], mur_post[2], mur_apply[2], exc[2], tfsf_v[2], tfsf_c[2], ade_v[2], ade_c[2], ade_apply_v[2], ade_apply_c[2],
         ring[2], nf_sample[2], nf_flush[2],
         deferred_i[2], deferred_d[2], pml_e_i[2], pml_e_d[2], pml_h_i[2], pml_h_d[2], tfsf_face[2], advance;   // _i / _d: index / dense members
@@ -224,6 +230,26 @@ struct efs_batch {
         }
     }
 
+    // Tile list of a work tile: bit 0: material-index member; bit 1: the tile
+    // meets a UPML region or a TFSF face of the core update (the tests of tma_tile).
+    int tile_class(const efs_engine* e, uint32_t xs, uint32_t y0, uint32_t z0) const {
+        bool some = false;
+        for (uint32_t f = 0; f < e->tf.n; ++f) some |= e->tf.z[f] >= z0 && e->tf.z[f] <= z0 + TT_Z;
+        const uint32_t lo[3] = {xs, y0, z0}, hi[3] = {xs + xchunk, y0 + TT_Y, z0 + TT_Z};
+        for (auto& R : e->pml) {
+            bool hit = true;
+            for (int d = 0; d < 3; ++d) hit = hit && hi[d] >= R->s[d] && lo[d] < R->s[d] + R->n[d];
+            some |= hit;
+        }
+        return (e->indexed ? 1 : 0) + (some ? 2 : 0);
+    }
+    template <bool IDX, bool SOME>
+    void launch_tiles(int t, const BatchMember* bm) {
+        if (ntiles[t])
+            k_fused_tma_batch<IDX, SOME><<<std::min<uint32_t>(ntiles[t], ctas_per_sm * sms), TT_THREADS, TT_SMEM_BYTES, stream>>>(
+                bm, tiles[t].as<BatchTile>(), ntiles[t]);
+    }
+
     void plan() {
         check_members();
         drop_graphs();
@@ -259,11 +285,13 @@ struct efs_batch {
                 // core tile descriptor
                 BatchMember& M = bm[i];
                 memset(&M, 0, sizeof(M));
-                const uint32_t bh[4] = {TT_HZ, TT_HY, 1, 3}, be[4] = {TT_EZ, TT_EY, 1, 3};
+                const uint32_t bh[4] = {TT_HZ, TT_HY, 1, 3}, be[4] = {TT_EZ, TT_EY, 1, 3}, bs[4] = {TT_Z, TT_Y, 1, 3};
                 M.tmH = e->tensor_map(fg.H0, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bh);
                 M.tmE = e->tensor_map(fg.V0, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, be);
                 M.tmM = e->indexed ? e->tensor_map(fg.mat, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, be) : M.tmE;
                 M.tmD = e->tf.n ? e->tf_map() : M.tmE;
+                M.tmE1 = e->tensor_map(fg.V1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs);
+                M.tmH1 = e->tensor_map(fg.H1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs);
                 M.g = fg;
                 M.g.xchunk = xchunk;
                 M.ps = ps;
@@ -350,14 +378,21 @@ struct efs_batch {
         std::vector<size_t> order(E);
         for (size_t i = 0; i < E; ++i) order[i] = i;
         std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return mem[a]->N > mem[b]->N; });
-        std::vector<BatchTile> tl[2];
+        std::vector<BatchTile> tl[4];
         for (size_t i : order) {
             const efs_engine* e = mem[i];
             for (uint32_t xs = 0; xs < e->Nx; xs += xchunk)
                 for (uint32_t y0 = 0; y0 < e->Ny; y0 += TT_Y)
-                    for (uint32_t z0 = 0; z0 < e->Nz; z0 += TT_Z) tl[e->indexed].push_back(BatchTile{(uint32_t)i, xs, y0, z0});
+                    for (uint32_t z0 = 0; z0 < e->Nz; z0 += TT_Z) tl[tile_class(e, xs, y0, z0)].push_back(BatchTile{(uint32_t)i, xs, y0, z0});
         }
-        for (int t = 0; t < 2; ++t) {
+        // a batch of few tiles runs them all in one launch: two short ones leave two half-empty
+        // last waves (16 members of 40-96 lines, 1,100 tiles: 101 us in two, 89 us in one)
+        for (int t : {0, 1})
+            if (!tl[t + 2].empty() && tl[t].size() < 4u * ctas_per_sm * sms) {
+                tl[t + 2].insert(tl[t + 2].end(), tl[t].begin(), tl[t].end());
+                tl[t].clear();
+            }
+        for (int t = 0; t < 4; ++t) {
             ntiles[t] = (uint32_t)tl[t].size();
             upload_raw(tiles[t], tl[t].data(), tl[t].size() * sizeof(BatchTile));
         }
@@ -379,12 +414,10 @@ struct efs_batch {
         launch_seg<OpTfsfFace>(tfsf_face[s], k); // TFSF face values the core update adds
         mark(2);
         const BatchMember* bm = members[s].as<BatchMember>();
-        if (ntiles[1])
-            k_fused_tma_batch<true><<<std::min<uint32_t>(ntiles[1], ctas_per_sm * sms), TT_THREADS, TT_SMEM_BYTES, stream>>>(
-                bm, tiles[1].as<BatchTile>(), ntiles[1]);
-        if (ntiles[0])
-            k_fused_tma_batch<false><<<std::min<uint32_t>(ntiles[0], ctas_per_sm * sms), TT_THREADS, TT_SMEM_BYTES, stream>>>(
-                bm, tiles[0].as<BatchTile>(), ntiles[0]);
+        launch_tiles<true, true>(3, bm);
+        launch_tiles<true, false>(1, bm);
+        launch_tiles<false, true>(2, bm);
+        launch_tiles<false, false>(0, bm);
         mark(3);
         launch_seg<OpPoints<1>>(tfsf_v[s], k);
         launch_seg<OpMurPost>(mur_post[s], k);
@@ -547,10 +580,9 @@ efs_status efs_batch_create(efs_batch** out, efs_engine* const* engines, uint32_
         ck(cudaEventCreateWithFlags(&b->ev_done, cudaEventDisableTiming), "cudaEventCreate");
         static bool attr = false;              // the persistent kernels' dynamic shared memory, once per process
         if (!attr) {
-            ck(cudaFuncSetAttribute(k_fused_tma_batch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT_SMEM_BYTES),
-               "smem attr");
-            ck(cudaFuncSetAttribute(k_fused_tma_batch<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT_SMEM_BYTES),
-               "smem attr");
+            for (const void* f : {(const void*)k_fused_tma_batch<true, true>, (const void*)k_fused_tma_batch<true, false>,
+                                  (const void*)k_fused_tma_batch<false, true>, (const void*)k_fused_tma_batch<false, false>})
+                ck(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT_SMEM_BYTES), "smem attr");
             attr = true;
         }
         b->check_members();

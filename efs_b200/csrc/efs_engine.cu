@@ -380,6 +380,7 @@ struct efs_engine {
         g.status = d_status;
         g.wait_ns = wait_ns;
         g.skip_plane = skip_plane;
+        g.nz = 0x8000000080000000ull;
         g.tf = tf;
         return g;
     }
@@ -807,28 +808,29 @@ struct efs_engine {
         return m;
     }
     template <bool IDX, bool PML>
-    void launch_fused_tma_k(dim3 g, const CUtensorMap& tH, const CUtensorMap& tE, const CUtensorMap& tM, const CUtensorMap& tD,
-                            const FusedGrid& fg, const PmlSet& ps) {
+    void launch_fused_tma_k(dim3 g, const CUtensorMap (&t)[6], const FusedGrid& fg, const PmlSet& ps) {
         static bool attr_set = false;   // per instantiation; the attribute is per kernel, all devices alike
         if (!attr_set) {
             ck(cudaFuncSetAttribute(k_fused_tma<IDX, PML>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT_SMEM_BYTES),
                "smem attr");
             attr_set = true;
         }
-        k_fused_tma<IDX, PML><<<g, TT_THREADS, TT_SMEM_BYTES, stream>>>(tH, tE, tM, tD, fg, ps);
+        k_fused_tma<IDX, PML><<<g, TT_THREADS, TT_SMEM_BYTES, stream>>>(t[0], t[1], t[2], t[3], t[4], t[5], fg, ps);
     }
     void launch_fused_tma(int p) {
         const FusedGrid fg = fused_grid(p);
         const PmlSet ps = pml_set(p);
-        const uint32_t bh[4] = {TT_HZ, TT_HY, 1, 3}, be[4] = {TT_EZ, TT_EY, 1, 3};
-        const CUtensorMap tH = tensor_map(fg.H0, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bh);
+        const uint32_t bh[4] = {TT_HZ, TT_HY, 1, 3}, be[4] = {TT_EZ, TT_EY, 1, 3}, bs[4] = {TT_Z, TT_Y, 1, 3};
         const CUtensorMap tE = tensor_map(fg.V0, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, be);
-        const CUtensorMap tM = indexed ? tensor_map(fg.mat, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, be) : tE;
-        const CUtensorMap tD = tf.n ? tf_map() : tE;   // unused without TFSF faces
-        dim3 g(blocks(Nz, TT_Z), blocks(Ny, TT_Y), blocks(Nx, xchunk));
+        const CUtensorMap t[6] = {tensor_map(fg.H0, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bh), tE,
+                                  indexed ? tensor_map(fg.mat, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, be) : tE,
+                                  tf.n ? tf_map() : tE,      // unused without TFSF faces
+                                  tensor_map(fg.V1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs),
+                                  tensor_map(fg.H1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs)};
+        dim3 g(blocks(Nz, TT_Z), blocks(Ny, TT_Y), blocks(Nx, fg.xchunk));
         const bool hp = !pml.empty();
-        if (indexed) { if (hp) launch_fused_tma_k<true, true>(g, tH, tE, tM, tD, fg, ps); else launch_fused_tma_k<true, false>(g, tH, tE, tM, tD, fg, ps); }
-        else { if (hp) launch_fused_tma_k<false, true>(g, tH, tE, tM, tD, fg, ps); else launch_fused_tma_k<false, false>(g, tH, tE, tM, tD, fg, ps); }
+        if (indexed) { if (hp) launch_fused_tma_k<true, true>(g, t, fg, ps); else launch_fused_tma_k<true, false>(g, t, fg, ps); }
+        else { if (hp) launch_fused_tma_k<false, true>(g, t, fg, ps); else launch_fused_tma_k<false, false>(g, t, fg, ps); }
     }
     // UPML cells are updated by k_pml_e / k_pml_h around the fused kernel
     bool pml_split() const { return !pml.empty(); }

@@ -37,6 +37,7 @@ struct FusedGrid {
     uint32_t* status;                   // device status word (bit 0: a bounded wait ran out)
     uint64_t wait_ns;                   // limit of every bounded mbarrier wait (about 1 s)
     uint32_t skip_plane;                // diagnostics: loads of this x-plane are never issued (~0u: none)
+    unsigned long long nz;              // two packed -0.0f (the packed products of efs_tma.cuh)
     TfsfFace tf;                        // TFSF z faces corrected in the core update (tf.n == 0: none)
 };
 

@@ -4,23 +4,21 @@
 // x-planes of one x-chunk through a TT_S-stage shared-memory pipeline: one
 // thread issues, per plane, three cp.async.bulk.tensor loads (H with its
 // low halos, E_old and the material rows, each a box of the tile plus halos)
-// completing on the stage's mbarrier, TT_S-1 planes ahead of the plane being
-// computed.  The loads run on the copy engine, so the bytes in flight per SM
-// do not depend on how many warps are resident.  The tensor maps span the
-// grid's Nz x Ny x Nx cells over the padded device layout (row pitch Pz, a
-// multiple of 4 floats, so every global stride is a multiple of 16 bytes):
-// box columns at z >= Nz lie outside the map and are zero-filled, so pad
-// cells are never loaded.
+// completing on the stage's mbarrier, about TT_S-1 planes ahead of the plane
+// being computed; another stores E_new and H_new of the tile with
+// cp.async.bulk.tensor from shared memory.  The copies run on the copy engine,
+// so the bytes in flight per SM do not depend on how many warps are resident,
+// and the warps spend no instructions on global addresses or ragged edges:
+// the tensor maps span the grid's Nz x Ny x Nx cells over the padded device
+// layout (row pitch Pz, a multiple of 4 floats, so every global stride is a
+// multiple of 16 bytes), box columns at z >= Nz lie outside the map, are
+// zero-filled on loads and clipped on stores, so pad cells are never touched.
 //
-// At plane x (local index k = x - xs) the CTA
-//   1. computes E_new(x) on the tile plus its high halo row and column from
-//      the staged H and E_old (H_old(x-1) of its cells it keeps in registers),
-//      stores the owned cells and keeps every E_new(x) in plane buffer k % 3,
-//   2. one barrier, after which the stage is refilled with plane x+TT_S,
-//   3. computes H_new(x-1) of the owned cells from E_new(x-1) (plane buffer
-//      (k-1) % 3 and registers) and E_new(x) (registers).
-// Three E_new plane buffers make step 3 of plane x and step 1 of plane x+1
-// independent, so one barrier per plane suffices.
+// Per plane x, between two barriers, a CTA computes E_new(x) on the tile plus
+// its high halo row and column from the staged H and E_old (H_old(x-1) of a
+// thread's cells stays in registers), then H_new(x-1) of the owned cells from
+// E_new(x-1), which the interval before left in the other of two plane
+// buffers, and the thread's own E_new(x).
 //
 // UPML cells are updated by k_pml_e (E, before this kernel: its E_new is
 // staged here in place of E_old and adopted as is) and k_pml_h (H, after it);
@@ -50,11 +48,20 @@ constexpr int TT_HZ = TT_Z + 8;          // H box: z0-4 .. z0+TT_Z+3 (x coordina
 constexpr int TT_HY = TT_Y + 2;          // H box: y0-1 .. y0+TT_Y
 constexpr int TT_EZ = TT_Z + 4;          // E_old / material box: z0 .. z0+TT_Z+3
 constexpr int TT_EY = TT_Y + 1;          // E_old / material box: y0 .. y0+TT_Y
-constexpr int TT_THREADS = 32 * (TT_Y + 1);   // warps 0..TT_Y-1: owned rows; warp TT_Y: halo row + halo column
+constexpr int TT_THREADS = 32 * (TT_Y + 2);   // warps 0..TT_Y-1: owned rows; TT_Y: halo row, loads; TT_Y+1: halo column, stores
 constexpr uint32_t TT_H_BYTES = 3u * TT_HY * TT_HZ * 4u;
 constexpr uint32_t TT_E_BYTES = 3u * TT_EY * TT_EZ * 4u;
 constexpr uint32_t TT_M_BYTES = 1u * TT_EY * TT_EZ * 4u;
 static_assert(TT_H_BYTES + TT_E_BYTES + TT_M_BYTES < (1u << 20), "mbarrier transaction count");
+
+// E_new of one plane: the owned cells [component][row][z] as the store box has
+// them, then the halo row and the halo column at the same component stride, so
+// every neighbour of a cell is one index plus a constant per component.
+constexpr int TT_EC = TT_Y * TT_Z;               // component stride
+constexpr int TT_EROW = 3 * TT_EC;               // halo row (Ex, Ez used)
+constexpr int TT_ECOL = TT_EROW + TT_Z;          // halo column, one cell per row (Ex, Ey)
+constexpr int TT_ENEW = TT_EROW + 2 * TT_EC + TT_Z;   // floats of one E_new plane
+static_assert(TT_Z + TT_Y <= TT_EC, "halo row and column fit one component stride");
 
 struct TmaStage {
     alignas(128) float H[3][TT_HY][TT_HZ];
@@ -64,10 +71,16 @@ struct TmaStage {
 };
 struct TmaSmem {
     TmaStage st[TT_S];
-    float En[3][3][TT_EY][TT_EZ];        // E_new of planes k % 3, tile + halo row/column
+    alignas(128) float En[2][TT_ENEW];   // E_new of planes x and x-1
+    alignas(128) float Hn[2][3 * TT_EC]; // H_new of planes x-1 and x-2, as the store box has them
     alignas(8) unsigned long long full[TT_S];
 };
 constexpr size_t TT_SMEM_BYTES = sizeof(TmaSmem) + 128;   // + slack to align the base to 128 B
+static_assert(2 * (TT_SMEM_BYTES + 1024) <= 228 * 1024, "two CTAs per SM");
+
+// What a CTA keeps across the tiles it runs back to back: the stage and its
+// mbarrier phase of the next plane, and the E_new / H_new buffer it writes.
+struct TmaRing { uint32_t s = 0, ph = 0, b = 0; };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -109,20 +122,33 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         : "memory");
 }
 
+// Store one plane of the tile (its owned cells, [component][row][z]) from
+// shared memory; cells beyond the grid are clipped by the tensor map.
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* src, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(src))
+                 : "memory");
+}
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// Every store issued by this thread has read its shared memory.
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
+// The tensor maps of one parity: loads (H_old, E_old, material, TFSF faces) and stores (E_new, H_new).
+struct TmaMaps { const CUtensorMap *H, *E, *M, *D, *E1, *H1; };
+
 // Issue the loads of plane x into stage s (one thread); dbytes > 0: also the
 // plane's TFSF face corrections (rows y0 .. y0+TF_DY-1 of every face).
 template <bool IDX>
-__device__ __forceinline__ void tt_issue(TmaSmem& S, int s, const CUtensorMap* tmH, const CUtensorMap* tmE,
-                                         const CUtensorMap* tmM, const CUtensorMap* tmD, uint32_t dbytes, int x, int y0,
-                                         int z0) {
+__device__ __forceinline__ void tt_issue(TmaSmem& S, uint32_t s, const TmaMaps& tm, uint32_t dbytes, int x, int y0, int z0) {
     const uint32_t bar = smem_u32(&S.full[s]);
     const uint32_t bytes = TT_H_BYTES + TT_E_BYTES + (IDX ? TT_M_BYTES : 0u) + dbytes;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // earlier generic reads of the stage before the refill
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    tma_load_4d(&S.st[s].H[0][0][0], tmH, z0 - 4, y0 - 1, x, 0, bar);
-    tma_load_4d(&S.st[s].E[0][0][0], tmE, z0, y0, x, 0, bar);
-    if (IDX) tma_load_3d(&S.st[s].M[0][0], tmM, z0, y0, x, bar);
-    if (dbytes) tma_load_4d(&S.st[s].D[0][0][0], tmD, y0, x, 0, 0, bar);
+    tma_load_4d(&S.st[s].H[0][0][0], tm.H, z0 - 4, y0 - 1, x, 0, bar);
+    tma_load_4d(&S.st[s].E[0][0][0], tm.E, z0, y0, x, 0, bar);
+    if (IDX) tma_load_3d(&S.st[s].M[0][0], tm.M, z0, y0, x, bar);
+    if (dbytes) tma_load_4d(&S.st[s].D[0][0][0], tm.D, y0, x, 0, 0, bar);
 }
 
 // The CTA's shared working area: 128-byte aligned, addressed from the shared
@@ -142,249 +168,370 @@ __device__ __forceinline__ void tt_init(TmaSmem& S) {
     __syncthreads();
 }
 
+// ---------------------------------------------------------------------------
+// Two z-adjacent cells per thread, as one packed f32x2 value: shared-memory
+// accesses are 64 bits wide and adds, subtractions and products one
+// instruction for both (each half rounded like the scalar instruction, and
+// products and sums stay separate), so a warp covers the 64 cells of a row.
+// ---------------------------------------------------------------------------
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// a * b as a*b + nz with nz = (-0, -0), which is a*b for every product, signed
+// zeros included.  The compiler contracts a packed multiply followed by a
+// packed add into one rounding (also when nz is a constant it can see), so nz
+// comes from the launch's arguments (FusedGrid).
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b, f32x2 nz) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
+    return r;
+}
+// curl4 and upd of both cells
+__device__ __forceinline__ f32x2 curl4_2(f32x2 a, f32x2 b, f32x2 c, f32x2 d) { return add2(sub2(sub2(a, b), c), d); }
+__device__ __forceinline__ f32x2 upd_2(f32x2 vold, f32x2 cv, f32x2 ci, f32x2 curl, f32x2 nz) {
+    return add2(mul2(vold, cv, nz), mul2(ci, curl, nz));
+}
+__device__ __forceinline__ f32x2 ld2(const float* p) { return *reinterpret_cast<const f32x2*>(p); }
+__device__ __forceinline__ f32x2 ldg2(const float* p) { return __ldg(reinterpret_cast<const f32x2*>(p)); }
+__device__ __forceinline__ f32x2 ldg2_once(const float* p) {   // read once: no L1 line
+    f32x2 r;
+    asm("ld.global.nc.L1::no_allocate.b64 %0, [%1];" : "=l"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ void st2(float* p, f32x2 v) { *reinterpret_cast<f32x2*>(p) = v; }
+// The halves of b that m selects (bit 0: low, bit 1: high) in place of a's.
+__device__ __forceinline__ f32x2 pick2(f32x2 a, f32x2 b, uint32_t m) {
+    return pk2(m & 1u ? lo2(b) : lo2(a), m & 2u ? hi2(b) : hi2(a));
+}
+// Coefficients of a pair: E side (BASE 0) or H side (BASE 6) of two table rows
+// (a 48-byte row is three float4: [vv0 vv1 vv2 vi0][vi1 vi2 ii0 ii1][ii2 iv0 iv1 iv2]).
+struct PairCoef { f32x2 v[3], i[3]; };
+template <int BASE>
+__device__ __forceinline__ PairCoef pair_rows(const float* table, uint2 m) {
+    const float4* t0 = reinterpret_cast<const float4*>(table) + (size_t)m.x * 3 + (BASE ? 1 : 0);
+    const float4* t1 = reinterpret_cast<const float4*>(table) + (size_t)m.y * 3 + (BASE ? 1 : 0);
+    const float4 a0 = __ldg(t0), b0 = __ldg(t0 + 1), a1 = __ldg(t1), b1 = __ldg(t1 + 1);
+    PairCoef k;
+    if (BASE == 0) {
+        k.v[0] = pk2(a0.x, a1.x); k.v[1] = pk2(a0.y, a1.y); k.v[2] = pk2(a0.z, a1.z);
+        k.i[0] = pk2(a0.w, a1.w); k.i[1] = pk2(b0.x, b1.x); k.i[2] = pk2(b0.y, b1.y);
+    } else {
+        k.v[0] = pk2(a0.z, a1.z); k.v[1] = pk2(a0.w, a1.w); k.v[2] = pk2(b0.x, b1.x);
+        k.i[0] = pk2(b0.y, b1.y); k.i[1] = pk2(b0.z, b1.z); k.i[2] = pk2(b0.w, b1.w);
+    }
+    return k;
+}
+// Dense coefficients of the pair at cell c (component stride N); zero for a
+// pair outside the grid.  Pad cells of a padded row hold zeros.
+__device__ __forceinline__ PairCoef pair_dense(const float* v, const float* i, size_t N, size_t c, bool in) {
+    PairCoef k;
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+        k.v[n] = in ? ldg2_once(v + n * N + c) : 0ull;
+        k.i[n] = in ? ldg2_once(i + n * N + c) : 0ull;
+    }
+    return k;
+}
+
 // One tile of the streaming update: the x-chunk starting at xs of the tile at
-// (y0, z0), called by every thread of the CTA.  K counts the planes the CTA
-// consumed before this tile (it selects the stage, the mbarrier phase and the
-// E_new buffer, so one CTA can run tiles back to back); every load the tile
-// issues is consumed before it returns.  Returns false after a wait ran out.
-// TF: the tile may meet a TFSF face corrected here (tested per tile; the single
-// engine runs tiles that meet none through the instantiation without that code).
+// (y0, z0), called by every thread of the CTA; `rg` carries the pipeline state
+// from one tile of a CTA to its next.  Every load the tile issues is consumed
+// before it returns; its last stores may still be reading shared memory (the
+// next plane's barrier, or tt_done, waits for them).  Returns false after a
+// wait ran out.
+// PML, TF: the tile may meet a UPML region, a TFSF face corrected here; the
+// single engine tests the second per tile (tma_tile), the batch sorts its tiles.
+//
+// Warp r < TT_Y owns tile row r, lane l the cells z0+2l and z0+2l+1.  Two more
+// warps compute the E_new that their H needs beyond the tile and run the
+// copies: warp TT_Y the halo row (Ex, Ez) and the loads, warp TT_Y+1 the halo
+// column (Ex, Ey; one cell per lane 0..TT_Y-1) and the stores.  Per plane x,
+// between two barriers:
+//   E(x) of the pair from the stage; its E_new to the plane buffer;
+//   H(x-1) of the pair, from the neighbours' E_new(x-1) of the interval before
+//   and the thread's own E(x); its H_new to the plane buffer;
+//   the refill of the stage of plane x-1 and the stores of E_new(x-1), H_new(x-2).
+// A pair's coefficients stay in registers while its material does not change
+// along x.
+//
 template <bool IDX, bool PML, bool TF>
-__device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const CUtensorMap* tmH, const CUtensorMap* tmE, const CUtensorMap* tmM,
-                                              const CUtensorMap* tmD, const FusedGrid& g, const PmlSet& ps, uint32_t xs,
-                                              uint32_t y0, uint32_t z0, uint32_t& K) {
+__device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, const FusedGrid& g, const PmlSet& ps, uint32_t xs,
+                                              uint32_t y0, uint32_t z0, TmaRing& rg) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t xe = min(xs + g.xchunk, g.Nx);
     const uint32_t xl = xe < g.Nx ? xe : g.Nx - 1;           // last plane whose E this CTA computes
     const int nk = (int)(xl - xs) + 1;                       // planes streamed
-    const uint32_t N = (uint32_t)g.N, NyNz = (uint32_t)g.NyNz, Ny = g.Ny, Nz = g.Nz, Pz = g.Pz;   // 3*N < 2^32
-    const uint64_t WAIT_NS = g.wait_ns;
+    const uint32_t Ny = g.Ny, Nz = g.Nz, Pz = g.Pz;
+    const size_t N = g.N, NyNz = g.NyNz;
     constexpr int HPL = TT_HY * TT_HZ;                       // one component of a staged H box
-    constexpr int EPL = TT_EY * TT_EZ;                       // one component of a staged E box / E_new plane
+    constexpr int EPL = TT_EY * TT_EZ;                       // one component of a staged E box
 
-    // ---- E cells of this thread: slots 0, 1 = (row, lane / lane+32); slot 2 = halo column (warp TT_Y, lanes 0..TT_Y)
-    const bool own = warp < TT_Y;                            // slots 0, 1 are owned cells (E stored, H updated)
-    const bool has2 = (warp == TT_Y) && (lane <= TT_Y);
-    const int sr[3] = {warp, warp, has2 ? lane : 0};
-    const int sc[3] = {lane, lane + 32, TT_Z};
-    uint32_t sy[3], sz[3], off[3];
-    int hi[3], ei[3], dym[3], dzm[3];
-    bool sin[3], core[3];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        sy[q] = y0 + sr[q]; sz[q] = z0 + sc[q];
-        sin[q] = sy[q] < Ny && sz[q] < Nz && (q < 2 || has2);
-        core[q] = sy[q] + 1 < Ny && sz[q] + 1 < Nz;
-        off[q] = sy[q] * Pz + sz[q];                         // offset inside a plane (used when sin)
-        hi[q] = (sr[q] + 1) * TT_HZ + sc[q] + 4;             // index in a staged H component
-        ei[q] = sr[q] * TT_EZ + sc[q];                       // index in a staged E component / E_new plane
-        dym[q] = sy[q] == 0 ? 0 : TT_HZ;                     // y-1 neighbour (self at y = 0)
-        dzm[q] = sz[q] == 0 ? 0 : 1;                         // z-1 neighbour (self at z = 0)
-    }
-    // UPML: regions meeting the CTA's box, then the (y, z) part of each cell's mask
-    uint32_t cand = 0, yzm[3] = {0u, 0u, 0u};
+    // TFSF faces meeting the tile's columns (halo column included)
+    bool tf_tile = false;
+    if (TF)
+        for (uint32_t f = 0; f < g.tf.n; ++f) tf_tile |= g.tf.z[f] >= z0 && g.tf.z[f] <= z0 + TT_Z;
+    // UPML: regions meeting the CTA's box, and those of them that not every plane meets
+    uint32_t cand = 0, xvar = 0;
     if (PML) {
         const uint32_t lo[3] = {xs, y0, z0};
         const uint32_t hb[3] = {xe, y0 + TT_Y, z0 + TT_Z};
         cand = region_mask(ps, lo, hb);
-        if (cand)
-#pragma unroll
-            for (int q = 0; q < 3; ++q) yzm[q] = axis_mask(ps, cand, 1, sy[q]) & axis_mask(ps, cand, 2, sz[q]);
+        if (cand) xvar = cand & ~(axis_mask(ps, cand, 0, xs) & axis_mask(ps, cand, 0, xl));
     }
 
-    bool tf_tile = false;
-    if (TF)
-        for (uint32_t f = 0; f < g.tf.n; ++f) tf_tile |= g.tf.z[f] >= z0 && g.tf.z[f] <= z0 + TT_Z;
-    const uint32_t dbytes = tf_tile ? g.tf.n * 2u * TF_DY * 4u : 0u;
-    int tfq[3] = {-1, -1, -1};
-    if (tf_tile)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) tfq[q] = sin[q] ? tf_face(g.tf, sz[q]) : -1;
+    if (warp == TT_Y + 1) {
+        // ---- halo column: Ex and Ey of the cell (y0 + lane, z0 + TT_Z); stores
+        const uint32_t y = y0 + lane, z = z0 + TT_Z;         // z >= TT_Z: never index 0
+        const bool has = lane < TT_Y, in = has && y < Ny && z < Nz;
+        const int hi = (lane + 1) * TT_HZ + TT_Z + 4, ei = lane * TT_EZ + TT_Z, hy_ = hi - (y == 0 ? 0 : TT_HZ);
+        const size_t off = (size_t)y * Pz + z;
+        const uint32_t yz = cand && has ? axis_mask(ps, cand, 1, y) & axis_mask(ps, cand, 2, z) : 0u;
+        const int tf = tf_tile && has ? tf_face(g.tf, z) : -1;
+        float hp = in ? __ldg(g.H0 + (size_t)(xs > 0 ? xs - 1 : 0) * NyNz + 2 * N + off) : 0.f;   // Hz(x-1)
+        float kc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};        // dense coefficients, loaded a plane ahead
+        if (!IDX && in) coeffs_f<false>(g, (size_t)xs * NyNz + off, 0u, 0, kc);
+        bool out = false;
+        for (int k = 0; k < nk; ++k) {
+            if (k > 0 && lane == 0) {                        // planes of the interval before: E(x-1), H(x-2)
+                tma_store_4d(tm.E1, S.En[rg.b ^ 1u], (int)z0, (int)y0, (int)(xs + k) - 1, 0);
+                if (k > 1) tma_store_4d(tm.H1, S.Hn[rg.b ^ 1u], (int)z0, (int)y0, (int)(xs + k) - 2, 0);
+                tma_store_commit();
+            }
+            __syncwarp();
+            const bool ok = mbar_wait_bounded(smem_u32(&S.full[rg.s]), rg.ph, g.wait_ns);
+            if (ok && has) {
+                const TmaStage& st = S.st[rg.s];
+                const float* Hs = &st.H[0][0][0];
+                const float* Es = &st.E[0][0][0];
+                if (IDX) coeffs_f<true>(g, 0, (&st.M[0][0])[ei], 0, kc);
+                const float hz = Hs[2 * HPL + hi], ex0 = Es[ei], ey0 = Es[EPL + ei];
+                float ex = upd(ex0, kc[0], kc[3], curl4(hz, Hs[2 * HPL + hy_], Hs[HPL + hi], Hs[HPL + hi - 1]));
+                float ey = upd(ey0, kc[1], kc[4], curl4(Hs[hi], Hs[hi - 1], hz, hp));
+                if (PML && yz && (yz & (~xvar | axis_mask(ps, xvar, 0, xs + k)))) { ex = ex0; ey = ey0; }
+                if (tf >= 0) { ex = __fadd_rn(ex, st.D[tf][0][lane]); ey = __fadd_rn(ey, st.D[tf][1][lane]); }
+                S.En[rg.b][TT_ECOL + lane] = ex;
+                S.En[rg.b][TT_ECOL + TT_EC + lane] = ey;
+                hp = hz;
+                if (!IDX && in && k + 1 < nk) coeffs_f<false>(g, (size_t)(xs + k + 1) * NyNz + off, 0u, 0, kc);
+            }
+            if (lane == 0) tma_store_wait_read();            // the buffers written in the next interval are free
+            __syncwarp();
+            out = __syncthreads_or(!ok) != 0;
+            if (out) break;
+            if (++rg.s == TT_S) { rg.s = 0; rg.ph ^= 1u; }
+            rg.b ^= 1u;
+        }
+        if (!out && lane == 0) {                             // the last plane (E only if owned) and H before it
+            if (xl < xe) tma_store_4d(tm.E1, S.En[rg.b ^ 1u], (int)z0, (int)y0, (int)xl, 0);
+            if (nk > 1) tma_store_4d(tm.H1, S.Hn[rg.b ^ 1u], (int)z0, (int)y0, (int)xl - 1, 0);
+            tma_store_commit();
+        }
+        __syncwarp();
+        return !out;
+    }
+
+    // ---- this thread's pair (row `warp`; the halo row for warp TT_Y)
+    const bool own = warp < TT_Y;
+    const uint32_t y = y0 + warp, z = z0 + 2 * lane;
+    const bool in = y < Ny && z < Nz;                        // the pair's first cell is inside the grid
+    const bool edge = y + 1 >= Ny || z + 2 >= Nz;            // some H of the pair has no update
+    const int hi = (warp + 1) * TT_HZ + 2 * lane + 4;        // index in a staged H component
+    const int ei = warp * TT_EZ + 2 * lane;                  // index in a staged E component
+    const int hy_ = hi - (y == 0 ? 0 : TT_HZ);               // y-1 neighbour (self at y = 0)
+    const int hz_ = hi - (z == 0 ? 0 : 1);                   // z-1 neighbour of the first cell (self at z = 0)
+    const int si = own ? warp * TT_Z + 2 * lane : TT_EROW + 2 * lane;   // index in an E_new / H_new plane
+    const int sy_ = warp == TT_Y - 1 ? TT_EROW + 2 * lane : si + TT_Z;  // its y+1 neighbour
+    const int sz_ = lane == 31 ? TT_ECOL + warp : si + 2;    // z+1 neighbour of the second cell
+    uint32_t yz0 = 0, yz1 = 0, up = 0;                       // regions of each cell's (y, z); UPML cells of the pair
+    if (PML && cand) {
+        const uint32_t ym = axis_mask(ps, cand, 1, y);
+        yz0 = ym & axis_mask(ps, cand, 2, z);
+        yz1 = ym & axis_mask(ps, cand, 2, z + 1);
+        up = (yz0 & ~xvar ? 1u : 0u) | (yz1 & ~xvar ? 2u : 0u);
+    }
+    int tf0 = -1, tf1 = -1;
+    if (tf_tile) {
+        tf0 = tf_face(g.tf, z);
+        tf1 = tf_face(g.tf, z + 1);
+    }
 
     // ---- first planes into the pipeline
-    int issued = 0;                                          // planes issued (thread 0's count)
-    if (threadIdx.x == 0)
+    const uint32_t dbytes = tf_tile ? g.tf.n * 2u * TF_DY * 4u : 0u;
+    const bool loader = threadIdx.x == 32 * TT_Y;
+    int issued = 0;                                          // planes issued (the loader's count)
+    if (loader)
         for (; issued < TT_S && issued < nk; ++issued)
             if (xs + issued != g.skip_plane)
-                tt_issue<IDX>(S, (int)((K + issued) % TT_S), tmH, tmE, tmM, tmD, dbytes, (int)(xs + issued), (int)y0, (int)z0);
+                tt_issue<IDX>(S, (rg.s + issued) % TT_S, tm, dbytes, (int)(xs + issued), (int)y0, (int)z0);
 
-    // H_old(xs-1) of the E cells (y, z components); at xs = 0 the x-1 neighbour is plane 0 itself
-    float hp[3][3];
-    {
-        const float* H = g.H0 + (size_t)(xs > 0 ? xs - 1 : 0) * NyNz;
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            hp[q][0] = 0.f;
-            hp[q][1] = sin[q] ? __ldg(H + (off[q] + N)) : 0.f;
-            hp[q][2] = sin[q] ? __ldg(H + (off[q] + 2 * N)) : 0.f;
-        }
+    // H_old(xs-1) of the pair; at xs = 0 the x-1 neighbour is plane 0 itself
+    const size_t off = (size_t)y * Pz + z;                   // offset inside a plane
+    size_t cell = (size_t)xs * NyNz + off;
+    f32x2 hp[3] = {0ull, 0ull, 0ull}, ep[3] = {0ull, 0ull, 0ull};   // H_old(x-1), E_new(x-1) of the pair
+    if (in) {
+        const float* H = g.H0 + (size_t)(xs > 0 ? xs - 1 : 0) * NyNz + off;
+        hp[1] = ldg2(H + N);
+        hp[2] = ldg2(H + 2 * N);
     }
-    float ep[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};      // E_new(x-1) of the owned cells
-    uint32_t mp[2] = {0u, 0u};                                // material of the owned cells at x-1
-    uint32_t xmask_p = 0;
+    const f32x2 nz = g.nz;
+    PairCoef ke, kh;                                         // E coefficients of plane x, H coefficients of plane x-1
+    uint2 mp = make_uint2(0u, 0u);                           // material of the pair at x-1
+    bool chg = false;                                        // it changed from plane x-2 to x-1
+    if (!IDX) ke = pair_dense(g.vv, g.vi, N, cell, in);
     bool timed_out = false;
     int k = 0;
 
     for (; k < nk; ++k) {
-        const uint32_t x = xs + k, kq = K + k;               // plane index within the tile / within the CTA
-        const int s = kq % TT_S;
-        const bool ok = mbar_wait_bounded(smem_u32(&S.full[s]), (kq / TT_S) & 1u, WAIT_NS);
-        const uint32_t xmask = cand ? axis_mask(ps, cand, 0, x) : 0u;
-        const float* Hs = &S.st[s].H[0][0][0];
-        const float* Es = &S.st[s].E[0][0][0];
-        const uint32_t* Ms = &S.st[s].M[0][0];
-        float* En = &S.En[kq % 3][0][0][0];
-        const uint32_t px = x * NyNz;
-        float en[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-        float hc[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-        uint32_t mc[3] = {0u, 0u, 0u};
+        if (IDX && chg) kh = pair_rows<6>(g.table, mp);      // H(x-1): known before the plane arrives
+        const bool ok = mbar_wait_bounded(smem_u32(&S.full[rg.s]), rg.ph, g.wait_ns);
         if (ok) {
-            // ---- E_new(x): gather every operand of the thread's cells, then update, then store
-            float hv[3][7], eo[3][3], kk[3][6];
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                if (q == 2 && !has2) continue;
-                const int h = hi[q], e = ei[q];
-                hv[q][0] = Hs[h]; hv[q][1] = Hs[HPL + h]; hv[q][2] = Hs[2 * HPL + h];
-                hv[q][3] = Hs[2 * HPL + h - dym[q]];         // hz(y-1)
-                hv[q][4] = Hs[HPL + h - dzm[q]];             // hy(z-1)
-                hv[q][5] = Hs[h - dzm[q]];                   // hx(z-1)
-                hv[q][6] = Hs[h - dym[q]];                   // hx(y-1)
-                eo[q][0] = Es[e]; eo[q][1] = Es[EPL + e]; eo[q][2] = Es[2 * EPL + e];
-                mc[q] = IDX ? Ms[e] : 0u;
+            const TmaStage& st = S.st[rg.s];
+            const float* Hs = &st.H[0][0][0];
+            const float* Es = &st.E[0][0][0];
+            float* En = S.En[rg.b];
+            const float* Ep = S.En[rg.b ^ 1u];
+            f32x2 hc[3], en[3];
+            // ---- E_new(x) of the pair
+            if (IDX) {
+                const uint2 mc = *reinterpret_cast<const uint2*>(&st.M[0][0] + ei);
+                chg = k == 0 || mc.x != mp.x || mc.y != mp.y;
+                if (chg) { ke = pair_rows<0>(g.table, mc); mp = mc; }
             }
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                if (q == 2 && !has2) continue;
-                if (IDX) coeffs_f<true>(g, 0, mc[q], 0, kk[q]);
-                else if (sin[q]) coeffs_f<false>(g, (size_t)px + off[q], 0u, 0, kk[q]);
-                else kk[q][0] = kk[q][1] = kk[q][2] = kk[q][3] = kk[q][4] = kk[q][5] = 0.f;
+            hc[0] = ld2(Hs + hi); hc[1] = ld2(Hs + HPL + hi); hc[2] = ld2(Hs + 2 * HPL + hi);
+            const f32x2 hzy = ld2(Hs + 2 * HPL + hy_), hxy = ld2(Hs + hy_);
+            const f32x2 hyz = pk2(Hs[HPL + hz_], lo2(hc[1])), hxz = pk2(Hs[hz_], lo2(hc[0]));
+            const f32x2 eo0 = ld2(Es + ei), eo1 = ld2(Es + EPL + ei), eo2 = ld2(Es + 2 * EPL + ei);
+            en[0] = upd_2(eo0, ke.v[0], ke.i[0], curl4_2(hc[2], hzy, hc[1], hyz), nz);
+            en[1] = upd_2(eo1, ke.v[1], ke.i[1], curl4_2(hc[0], hxz, hc[2], hp[2]), nz);
+            en[2] = upd_2(eo2, ke.v[2], ke.i[2], curl4_2(hc[1], hp[1], hc[0], hxy), nz);
+            if (PML && cand) {           // a UPML cell's E_new was computed by k_pml_e and staged in place of E_old
+                if (xvar) {
+                    const uint32_t xm = ~xvar | axis_mask(ps, xvar, 0, xs + k);
+                    up = (yz0 & xm ? 1u : 0u) | (yz1 & xm ? 2u : 0u);
+                }
+                if (up) { en[0] = pick2(en[0], eo0, up); en[1] = pick2(en[1], eo1, up); en[2] = pick2(en[2], eo2, up); }
             }
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                if (q == 2 && !has2) continue;
-                const float hx = hv[q][0], hy = hv[q][1], hz = hv[q][2];
-                const float cx = curl4(hz, hv[q][3], hy, hv[q][4]);
-                const float cy = curl4(hx, hv[q][5], hz, hp[q][2]);
-                const float cz = curl4(hy, hp[q][1], hx, hv[q][6]);
-                hc[q][0] = hx; hc[q][1] = hy; hc[q][2] = hz;
-                // a UPML cell's E_new was computed by k_pml_e and staged in place of E_old
-                const bool upml = PML && (yzm[q] & xmask);
-                en[q][0] = upml ? eo[q][0] : upd(eo[q][0], kk[q][0], kk[q][3], cx);
-                en[q][1] = upml ? eo[q][1] : upd(eo[q][1], kk[q][1], kk[q][4], cy);
-                en[q][2] = upml ? eo[q][2] : upd(eo[q][2], kk[q][2], kk[q][5], cz);
-                if (tf_tile && tfq[q] >= 0) {               // the TFSF point pass's add, here
-                    const float* D = &S.st[s].D[tfq[q]][0][0];
-                    en[q][0] = __fadd_rn(en[q][0], D[sr[q]]);
-                    en[q][1] = __fadd_rn(en[q][1], D[TF_DY + sr[q]]);
+            if (tf_tile) {               // the TFSF point pass's add, here
+                if (tf0 >= 0) {
+                    en[0] = pk2(__fadd_rn(lo2(en[0]), st.D[tf0][0][warp]), hi2(en[0]));
+                    en[1] = pk2(__fadd_rn(lo2(en[1]), st.D[tf0][1][warp]), hi2(en[1]));
+                }
+                if (tf1 >= 0) {
+                    en[0] = pk2(lo2(en[0]), __fadd_rn(hi2(en[0]), st.D[tf1][0][warp]));
+                    en[1] = pk2(lo2(en[1]), __fadd_rn(hi2(en[1]), st.D[tf1][1][warp]));
                 }
             }
-            float* V1 = g.V1 + px;
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                if (q == 2 && !has2) continue;
-                const int e = ei[q];
-                En[e] = en[q][0]; En[EPL + e] = en[q][1]; En[2 * EPL + e] = en[q][2];
-                if (own && q < 2 && sin[q] && x < xe) {
-                    V1[off[q]] = en[q][0];
-                    V1[off[q] + N] = en[q][1];
-                    V1[off[q] + 2 * N] = en[q][2];
+            st2(En + si, en[0]); st2(En + TT_EC + si, en[1]); st2(En + 2 * TT_EC + si, en[2]);
+            if (own) {
+                // ---- H_new(x-1) of the pair
+                if (k > 0) {
+                    const f32x2 ezy = ld2(Ep + 2 * TT_EC + sy_), exy = ld2(Ep + sy_);
+                    const f32x2 eyz = pk2(hi2(ep[1]), Ep[TT_EC + sz_]), exz = pk2(hi2(ep[0]), Ep[sz_]);
+                    f32x2 hn[3];
+                    hn[0] = upd_2(hp[0], kh.v[0], kh.i[0], curl4_2(ep[2], ezy, ep[1], eyz), nz);
+                    hn[1] = upd_2(hp[1], kh.v[1], kh.i[1], curl4_2(ep[0], exz, ep[2], en[2]), nz);
+                    hn[2] = upd_2(hp[2], kh.v[2], kh.i[2], curl4_2(ep[1], en[1], ep[0], exy), nz);
+                    if (edge) {                              // H beyond the last line: pass-through
+                        const uint32_t m = y + 1 >= Ny ? 3u : (z + 1 >= Nz ? 1u : 0u) | (z + 2 >= Nz ? 2u : 0u);
+                        hn[0] = pick2(hn[0], hp[0], m); hn[1] = pick2(hn[1], hp[1], m); hn[2] = pick2(hn[2], hp[2], m);
+                    }
+                    float* Hn = S.Hn[rg.b];                  // UPML cells among them are rewritten by k_pml_h
+                    st2(Hn + si, hn[0]); st2(Hn + TT_EC + si, hn[1]); st2(Hn + 2 * TT_EC + si, hn[2]);
                 }
+            } else if (loader && k > 0 && issued < nk) {
+                if (xs + issued != g.skip_plane)             // plane k-1+TT_S into the stage of plane k-1
+                    tt_issue<IDX>(S, (rg.s + TT_S - 1) % TT_S, tm, dbytes, (int)(xs + issued), (int)y0, (int)z0);
+                ++issued;
             }
+            if (!IDX) {                  // the next plane's E coefficients and this plane's H coefficients
+                if (k + 1 < nk) ke = pair_dense(g.vv, g.vi, N, cell + NyNz, in);
+                if (own) kh = pair_dense(g.ii, g.iv, N, cell, in);
+                cell += NyNz;
+            }
+#pragma unroll
+            for (int n = 0; n < 3; ++n) { hp[n] = hc[n]; ep[n] = en[n]; }
         }
-        // every read of stage s and every write of En[k % 3] done; agree on a timeout
+        // every read of the stage and of E_new(x-1) and every write of the plane buffers done; agree on a timeout
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the plane buffers' writes before their TMA stores
         timed_out = __syncthreads_or(!ok) != 0;
         if (timed_out) break;
-        if (threadIdx.x == 0 && issued < nk) {
-            if (xs + issued != g.skip_plane)   // stage of plane k+TT_S
-                tt_issue<IDX>(S, s, tmH, tmE, tmM, tmD, dbytes, (int)(xs + issued), (int)y0, (int)z0);
-            ++issued;
-        }
-        // ---- H_new(x-1) of the owned cells
-        if (k > 0 && own) {
-            const float* Ep = &S.En[(kq + 2) % 3][0][0][0];
-            float nb[2][4], kh[2][6];
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int e = ei[q];
-                nb[q][0] = Ep[2 * EPL + e + TT_EZ];          // ez(y+1)
-                nb[q][1] = Ep[EPL + e + 1];                  // ey(z+1)
-                nb[q][2] = Ep[e + 1];                        // ex(z+1)
-                nb[q][3] = Ep[e + TT_EZ];                    // ex(y+1)
-                if (IDX) coeffs_f<true>(g, 0, mp[q], 6, kh[q]);
-                else if (sin[q]) coeffs_f<false>(g, (size_t)(px - NyNz) + off[q], 0u, 6, kh[q]);
-                else kh[q][0] = kh[q][1] = kh[q][2] = kh[q][3] = kh[q][4] = kh[q][5] = 0.f;
-            }
-            float* H1 = g.H1 + (px - NyNz);
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const float ex = ep[q][0], ey = ep[q][1], ez = ep[q][2];
-                const float cx = curl4(ez, nb[q][0], ey, nb[q][1]);
-                const float cy = curl4(ex, nb[q][2], ez, en[q][2]);
-                const float cz = curl4(ey, en[q][1], ex, nb[q][3]);
-                float hn[3];
-                hn[0] = core[q] ? upd(hp[q][0], kh[q][0], kh[q][3], cx) : hp[q][0];
-                hn[1] = core[q] ? upd(hp[q][1], kh[q][1], kh[q][4], cy) : hp[q][1];
-                hn[2] = core[q] ? upd(hp[q][2], kh[q][2], kh[q][5], cz) : hp[q][2];
-                if (sin[q] && !(PML && (yzm[q] & xmask_p))) {     // UPML cells: k_pml_h
-                    H1[off[q]] = hn[0];
-                    H1[off[q] + N] = hn[1];
-                    H1[off[q] + 2 * N] = hn[2];
-                }
-            }
-        }
-        // ---- rotate
-#pragma unroll
-        for (int q = 0; q < 3; ++q) { hp[q][0] = hc[q][0]; hp[q][1] = hc[q][1]; hp[q][2] = hc[q][2]; }
-#pragma unroll
-        for (int q = 0; q < 2; ++q) { ep[q][0] = en[q][0]; ep[q][1] = en[q][1]; ep[q][2] = en[q][2]; mp[q] = mc[q]; }
-        xmask_p = xmask;
+        if (++rg.s == TT_S) { rg.s = 0; rg.ph ^= 1u; }
+        rg.b ^= 1u;
     }
-
     if (timed_out) {
-        if (threadIdx.x == 0) {
+        if (loader) {
             atomicOr(g.status, 1u);
-            for (int j = k; j < issued; ++j)                       // drain the loads still in flight
+            for (int j = k; j < issued; ++j) {                       // drain the loads still in flight
+                const uint32_t q = rg.s + (uint32_t)(j - k);         // plane k is in stage rg.s
                 if (xs + j != g.skip_plane)
-                    (void)mbar_wait_bounded(smem_u32(&S.full[(K + j) % TT_S]), ((K + j) / TT_S) & 1u, WAIT_NS);
+                    (void)mbar_wait_bounded(smem_u32(&S.full[q % TT_S]), rg.ph ^ (q / TT_S), g.wait_ns);
+            }
         }
         return false;
     }
     // ---- H of the last plane x = Nx-1: no core update (pass-through; UPML cells: k_pml_h)
-    if (xe == g.Nx && own) {
-        float* H1 = g.H1 + (size_t)(g.Nx - 1) * NyNz;
+    if (xe == g.Nx && own && in) {
+        float* H1 = g.H1 + (size_t)(g.Nx - 1) * NyNz + off;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            if (!sin[q] || (PML && (yzm[q] & xmask_p))) continue;
-#pragma unroll
-            for (int n = 0; n < 3; ++n) H1[off[q] + n * N] = hp[q][n];
+        for (int n = 0; n < 3; ++n) {
+            H1[n * N] = lo2(hp[n]);
+            if (z + 1 < Nz) H1[n * N + 1] = hi2(hp[n]);
         }
     }
-    K += nk;
     return true;
+}
+// The CTA's last stores have left shared memory (called once, after its last tile).
+__device__ __forceinline__ void tt_done() {
+    if (threadIdx.x == 32 * (TT_Y + 1)) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 // A TFSF face corrected in the core update meets the tile's columns (halo column included).
 template <bool IDX, bool PML>
-__device__ __forceinline__ bool tma_tile(TmaSmem& S, const CUtensorMap* tmH, const CUtensorMap* tmE, const CUtensorMap* tmM,
-                                         const CUtensorMap* tmD, const FusedGrid& g, const PmlSet& ps, uint32_t xs,
-                                         uint32_t y0, uint32_t z0, uint32_t& K) {
+__device__ __forceinline__ bool tma_tile(TmaSmem& S, const TmaMaps& tm, const FusedGrid& g, const PmlSet& ps, uint32_t xs,
+                                         uint32_t y0, uint32_t z0, TmaRing& rg) {
     bool tf = false;
     for (uint32_t f = 0; f < g.tf.n; ++f) tf |= g.tf.z[f] >= z0 && g.tf.z[f] <= z0 + TT_Z;
-    return tf ? tma_tile_body<IDX, PML, true>(S, tmH, tmE, tmM, tmD, g, ps, xs, y0, z0, K)
-              : tma_tile_body<IDX, PML, false>(S, tmH, tmE, tmM, tmD, g, ps, xs, y0, z0, K);
+    return tf ? tma_tile_body<IDX, PML, true>(S, tm, g, ps, xs, y0, z0, rg)
+              : tma_tile_body<IDX, PML, false>(S, tm, g, ps, xs, y0, z0, rg);
 }
 
+// Bound by DRAM on large grids (512^3: 1.114 ms a launch at 24 planes per CTA
+// for 7.0 GB, 0.96 of the measured copy rate; 1.29 ms with one cell per lane,
+// scalar accesses and stores from registers, which issued 225 warp
+// instructions per 32 cells).  Small or ragged grids are bound by a plane's
+// chain of wait, update and barrier, about 1.2 us with two CTAs per SM
+// (64 stub filters' sizes, 32 of them: 533 us a batched step at 0.83 of the
+// copy rate, 726 us before).  Tried and not kept: 7 owned rows in 8 warps (fewer warps, 128
+// registers: same time at 512^3, 4% slower at 256^3), loops unrolled 2 or 4
+// planes deep (slower: instruction fetch), TMA boxes without halo columns
+// (no change).
 template <bool IDX, bool PML>
 __global__ void __launch_bounds__(TT_THREADS, 2)
 k_fused_tma(const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmE,
-            const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmD, const FusedGrid g,
+            const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmD,
+            const __grid_constant__ CUtensorMap tmE1, const __grid_constant__ CUtensorMap tmH1, const FusedGrid g,
             const PmlSet ps) {
     const uint32_t xs = blockIdx.z * g.xchunk;
     if (xs >= g.Nx) return;                                  // uniform per CTA
     TmaSmem& S = tt_smem();
     tt_init(S);
-    uint32_t K = 0;
-    (void)tma_tile<IDX, PML>(S, &tmH, &tmE, &tmM, &tmD, g, ps, xs, blockIdx.y * TT_Y, blockIdx.x * TT_Z, K);
+    TmaRing rg;
+    (void)tma_tile<IDX, PML>(S, TmaMaps{&tmH, &tmE, &tmM, &tmD, &tmE1, &tmH1}, g, ps, xs, blockIdx.y * TT_Y, blockIdx.x * TT_Z, rg);
+    tt_done();
 }
 
 // ---------------------------------------------------------------------------
