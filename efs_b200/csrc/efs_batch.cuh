@@ -167,7 +167,9 @@ struct efs_batch {
     std::vector<efs_engine*> mem;
     std::vector<cudaEvent_t> ev_in;            // member stream -> batch stream
     cudaEvent_t ev_done = nullptr;             // batch stream -> member streams
-    uint32_t xchunk = 32, ctas_per_sm = 2, sms = 148;
+    uint32_t xchunk = 0;                       // plane depth asked for (0: chosen by the plan)
+    uint32_t xc = 0;                           // and the one in use
+    uint32_t ctas_per_sm = 2, sms = 148;
 
     // plan, per step phase s (member e at batch step k uses parity cur0[e] ^ s, s = (phase + k) & 1)
     bool planned = false;
@@ -230,12 +232,27 @@ struct efs_batch {
         }
     }
 
+    // Plane depth of the work tiles: a tile of d planes costs about d + 3 (the
+    // plane it shares with its neighbour and filling its pipeline), and the
+    // last tiles leave half a tile of idle time.  At most 24, as plane_depth.
+    uint32_t pick_depth() const {
+        double best = 1e300;
+        uint32_t pick = 1;
+        for (uint32_t d = 1; d <= TT_DEPTH; ++d) {
+            double planes = 0;
+            for (const efs_engine* e : mem)
+                planes += (double)blocks(e->Ny, TT_Y) * blocks(e->Nz, TT_Z) * (e->Nx + 3.0 * blocks(e->Nx, d));
+            const double c = planes / (ctas_per_sm * sms) + 0.5 * (d + 3);
+            if (c < best) { best = c; pick = d; }
+        }
+        return pick;
+    }
     // Tile list of a work tile: bit 0: material-index member; bit 1: the tile
     // meets a UPML region or a TFSF face of the core update (the tests of tma_tile).
     int tile_class(const efs_engine* e, uint32_t xs, uint32_t y0, uint32_t z0) const {
         bool some = false;
         for (uint32_t f = 0; f < e->tf.n; ++f) some |= e->tf.z[f] >= z0 && e->tf.z[f] <= z0 + TT_Z;
-        const uint32_t lo[3] = {xs, y0, z0}, hi[3] = {xs + xchunk, y0 + TT_Y, z0 + TT_Z};
+        const uint32_t lo[3] = {xs, y0, z0}, hi[3] = {xs + xc, y0 + TT_Y, z0 + TT_Z};
         for (auto& R : e->pml) {
             bool hit = true;
             for (int d = 0; d < 3; ++d) hit = hit && hi[d] >= R->s[d] && lo[d] < R->s[d] + R->n[d];
@@ -254,6 +271,7 @@ struct efs_batch {
         check_members();
         drop_graphs();
         const size_t E = mem.size();
+        xc = xchunk ? xchunk : pick_depth();
         cur0.resize(E);
         for (size_t i = 0; i < E; ++i) { mem[i]->build_plan(); cur0[i] = mem[i]->cur; }
         phase = 0;
@@ -293,7 +311,7 @@ struct efs_batch {
                 M.tmE1 = e->tensor_map(fg.V1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs);
                 M.tmH1 = e->tensor_map(fg.H1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs);
                 M.g = fg;
-                M.g.xchunk = xchunk;
+                M.g.xchunk = xc;
                 M.ps = ps;
                 float* V = e->vbuf(p);
                 float* V1 = e->vbuf(q);
@@ -381,7 +399,7 @@ struct efs_batch {
         std::vector<BatchTile> tl[4];
         for (size_t i : order) {
             const efs_engine* e = mem[i];
-            for (uint32_t xs = 0; xs < e->Nx; xs += xchunk)
+            for (uint32_t xs = 0; xs < e->Nx; xs += xc)
                 for (uint32_t y0 = 0; y0 < e->Ny; y0 += TT_Y)
                     for (uint32_t z0 = 0; z0 < e->Nz; z0 += TT_Z) tl[tile_class(e, xs, y0, z0)].push_back(BatchTile{(uint32_t)i, xs, y0, z0});
         }

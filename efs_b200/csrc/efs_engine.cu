@@ -144,7 +144,8 @@ struct efs_engine {
     DevBuf volt, curr;          // fields (parity 0)
     DevBuf volt_b, curr_b;      // second buffers (parity 1): a step reads one parity and writes the other
     int cur = 0;                // parity holding the current fields
-    uint32_t xchunk = 32;       // x-planes per CTA of the fused kernel (efs_set_plane_depth)
+    uint32_t xchunk = 0;        // x-planes per CTA of the fused kernel (efs_set_plane_depth; 0: plane_depth)
+    uint32_t sms = 148;
     uint64_t wait_ns = 1000000000ull;   // limit of the fused kernel's bounded waits
     uint32_t skip_plane = ~0u;          // diagnostics (efs_debug_set_wait): a plane whose loads are never issued
     DevBuf defer_cells;
@@ -370,9 +371,28 @@ struct efs_engine {
             if (p[i] >= 3 * N) fail(EFS_ERR_INVALID, std::string(what) + ": index out of range");
     }
 
+    // x-planes per CTA of the fused kernel: the depth whose waves of two CTAs
+    // per SM take the fewest plane times, a CTA of d planes taking about d + 3
+    // (the plane it shares with its neighbour and filling its pipeline).
+    // 81^3: 8 planes 12.6 us, 32 planes 26.8 us a launch; 200x200x100: 12
+    // planes 63 us, 32 planes 80 us; 256^3: 16 planes 151 us, 6 planes 173 us.
+    // Depths above 24 lose on large grids (512^3: 24 planes 1.114 ms, 32
+    // planes 1.131 ms, 64 planes 1.31 ms): neighbouring tiles drift apart and
+    // their shared halos leave L2.
+    uint32_t plane_depth() const {
+        if (xchunk) return xchunk;
+        const uint64_t tiles = (uint64_t)blocks(Nz, TT_Z) * blocks(Ny, TT_Y), slots = 2ull * sms;
+        uint64_t best = ~0ull;
+        uint32_t pick = 1;
+        for (uint32_t d = 1; d <= TT_DEPTH && d <= Nx; ++d) {
+            const uint64_t waves = (tiles * blocks(Nx, d) + slots - 1) / slots, c = waves * (d + 3);
+            if (c < best) { best = c; pick = d; }
+        }
+        return pick;
+    }
     FusedGrid fused_grid(int p) const {
         FusedGrid g;
-        g.Nx = Nx; g.Ny = Ny; g.Nz = Nz; g.xchunk = xchunk; g.Pz = Pz;
+        g.Nx = Nx; g.Ny = Ny; g.Nz = Nz; g.xchunk = plane_depth(); g.Pz = Pz;
         g.N = Nd; g.NyNz = (size_t)Ny * Pz;
         g.V0 = vbuf(p); g.H0 = cbuf(p); g.V1 = vbuf(1 - p); g.H1 = cbuf(1 - p);
         g.mat = mat.as<uint32_t>(); g.table = table.as<float>();
@@ -1022,6 +1042,9 @@ efs_status efs_create(efs_engine** out, int device) {
     try {
         ck(cudaSetDevice(device), "cudaSetDevice");
         ck(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking), "cudaStreamCreate");
+        int sms = 0;
+        ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "SM count");
+        e->sms = (uint32_t)sms;
         e->slot = host_slot_get();
         e->en_host = e->slot->energy;
         e->h_status = &e->slot->status;

@@ -48,6 +48,7 @@ constexpr int TT_HZ = TT_Z + 8;          // H box: z0-4 .. z0+TT_Z+3 (x coordina
 constexpr int TT_HY = TT_Y + 2;          // H box: y0-1 .. y0+TT_Y
 constexpr int TT_EZ = TT_Z + 4;          // E_old / material box: z0 .. z0+TT_Z+3
 constexpr int TT_EY = TT_Y + 1;          // E_old / material box: y0 .. y0+TT_Y
+constexpr uint32_t TT_DEPTH = 24;        // deepest x-chunk chosen without efs_set_plane_depth / efs_batch_set_shape
 constexpr int TT_THREADS = 32 * (TT_Y + 2);   // warps 0..TT_Y-1: owned rows; TT_Y: halo row, loads; TT_Y+1: halo column, stores
 constexpr uint32_t TT_H_BYTES = 3u * TT_HY * TT_HZ * 4u;
 constexpr uint32_t TT_E_BYTES = 3u * TT_EY * TT_EZ * 4u;

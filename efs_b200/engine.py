@@ -487,7 +487,7 @@ class CudaEngine:
 
     def setPlaneDepth(self, xchunk):
         """Tuning (efs_set_plane_depth): x-planes per CTA of the fused kernel
-        (default 32); results are bit-identical under every depth."""
+        (default: chosen from the grid); results are bit-identical under every depth."""
         self._ck(self._lib.efs_set_plane_depth(self._h, int(xchunk)))
 
     def timeCore(self, reps=10):
