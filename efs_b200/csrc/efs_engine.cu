@@ -30,6 +30,7 @@
 #include "efs_kernels.cuh"
 #include "efs_fused.cuh"
 #include "efs_tma.cuh"
+#include "efs_sweep.cuh"
 #include "efs_host.h"
 
 #include <cuda_runtime.h>
@@ -51,6 +52,8 @@
 using namespace efs;
 
 namespace {
+
+constexpr size_t SWEEP_BYTES = (size_t)92 << 20;   // fields and material index of the largest grid that runs as sweeps
 
 thread_local std::string g_create_error = "no error";
 
@@ -175,6 +178,7 @@ struct efs_engine {
     };
     std::vector<std::unique_ptr<Region>> pml;
     DevBuf vflux_ptrs[2], cflux_ptrs[2];
+    DevBuf pml_axis;                 // regions by x, y and z (PmlSet::xm, ym, zm, each padded)
 
     float* vbuf(int p) const { return p ? volt_b.as<float>() : volt.as<float>(); }
     float* cbuf(int p) const { return p ? curr_b.as<float>() : curr.as<float>(); }
@@ -404,11 +408,14 @@ struct efs_engine {
         g.tf = tf;
         return g;
     }
+    // entries of one axis in pml_axis: the axis, its padding, an even count (zm is read in pairs)
+    static size_t axis_room(uint32_t n) { return ((size_t)n + PML_AXIS_PAD + 1) & ~(size_t)1; }
     // UPML set whose flux pointers are the parity-p buffers
     PmlSet pml_set(int p = 0) const {
         PmlSet s;
         memset(&s, 0, sizeof(s));
         s.count = (int)pml.size();
+        s.xm = pml_axis.as<uint32_t>(); s.ym = s.xm + axis_room(Nx); s.zm = s.ym + axis_room(Ny);
         for (size_t r = 0; r < pml.size(); ++r) {
             const Region& R = *pml[r];
             for (int d = 0; d < 3; ++d) { s.r[r].s[d] = R.s[d]; s.r[r].n[d] = R.n[d]; }
@@ -546,10 +553,10 @@ struct efs_engine {
     std::vector<efs_tfsf_point> h_tfsf_v;      // the caller's voltage-side TFSF points
     TfsfFace tf{0, {0, 0}};
     uint32_t tf_n = 0, tf_ly = 0;
-    DevBuf tf_face, tf_dst, tf_delay, tf_frac, tf_amp;
+    DevBuf tf_face, tf_dst, tf_target, tf_delay, tf_frac, tf_amp;
     void plan_tfsf_faces();
     TfsfFaceDev tf_dev() const {
-        return TfsfFaceDev{tf_n, tf_dst.as<uint32_t>(), tf_delay.as<uint32_t>(), tf_frac.as<float>(), tf_amp.as<float>(),
+        return TfsfFaceDev{tf_n, tf_dst.as<uint32_t>(), tf_target.as<uint32_t>(), tf_delay.as<uint32_t>(), tf_frac.as<float>(), tf_amp.as<float>(),
                            tfsf_signal.as<float>(), tfsf_len, tfsf_period, tf_face.as<float>()};
     }
     // tensor map of the face array: dims y (pitch tf_ly), x, component, face; box TF_DY x 1 x 2 x faces
@@ -672,7 +679,7 @@ struct efs_engine {
         const uint32_t T = 256;
         const float* const* vfl = vflux_ptrs[p].as<const float*>();
         const float* const* cfl = cflux_ptrs[p].as<const float*>();
-        const bool split = pml_split();
+        const bool sweep = use_sweep(), split = pml_split() && !sweep;
 
         // --- pre-voltage ---
         if (ss_on)     // reads the fields before the UPML pre-update
@@ -697,11 +704,13 @@ struct efs_engine {
         // ADE(curr) reads H and the current flux, which the E side never
         // touches: it runs before the fused kernel overwrites the flux.
         if (ade_c.live()) k_ade<<<blocks(ade_c.n, ADE_BLOCK), ADE_T, 0, stream>>>(C, ade_dev(ade_c, cfl));
-        if (tf_n) k_tfsf_face<<<blocks(tf_n, T), T, 0, stream>>>(st, k, tf_dev());   // TFSF face values of this step
+        if (tf_n && !sweep) k_tfsf_face<<<blocks(tf_n, T), T, 0, stream>>>(st, k, tf_dev());   // TFSF face values of this step
         mark(2);
-        launch_fused_tma(p);
+        if (sweep) launch_sweep(p, true);
+        else launch_fused_tma(p);
         mark(3);
         // --- post-voltage / apply (on the updated E) ---
+        if (tf_n && sweep) k_tfsf_face_points<<<blocks(tf_n, T), T, 0, stream>>>(V1, st, k, tf_dev());
         if (tfsf_on && tfsf_v.groups) k_point_sources<1><<<blocks(tfsf_v.groups, T), T, 0, stream>>>(V1, st, k, point_dev(tfsf_v, tfsf_signal, tfsf_len, tfsf_period));
         if (pbc_on) for (auto& a : pbc_axes) launch_pbc(a, true, V1);
         if (mur_on) k_mur_post<<<blocks(mur_n, T), T, 0, stream>>>(V1, md);
@@ -715,7 +724,9 @@ struct efs_engine {
         if (ade_apply && ade_v.live()) launch_ade_apply(ade_v, V1);
         mark(4);
         // --- H of the UPML cells and of the cells next to those E writes ---
-        if (split && defer_n) {
+        if (sweep) {
+            launch_sweep(p, false);
+        } else if (split && defer_n) {
             const uint32_t na = blocks(pml_items(), T), nb = blocks(defer_n, T);
             if (indexed) pair(pml_h_pass<true>(p), na, deferred_pass<true>(p), nb);
             else pair(pml_h_pass<false>(p), na, deferred_pass<false>(p), nb);
@@ -851,6 +862,28 @@ struct efs_engine {
         const bool hp = !pml.empty();
         if (indexed) { if (hp) launch_fused_tma_k<true, true>(g, t, fg, ps); else launch_fused_tma_k<true, false>(g, t, fg, ps); }
         else { if (hp) launch_fused_tma_k<false, true>(g, t, fg, ps); else launch_fused_tma_k<false, false>(g, t, fg, ps); }
+    }
+    // E and H sweeps (efs_sweep.cuh) instead of the fused kernel and the passes
+    // around it: while both parities of the fields and the material index stay
+    // in L2 (us per timestep, fused / sweeps: 64^3 10.2 / 8.5, 112^3 19.0 /
+    // 18.8, 128^3 25.1 / 28.5; with UPML on all faces 64^3 17.1 / 12.2, 120^3
+    // 50 / 47, 128^3 58 / 60), and at every size with dense coefficients, which
+    // the plane pipeline reads with plain loads (120^3 44 / 30, 200^3 191 / 143).
+    // An explicit plane depth or a diagnostic plane is a property of the fused
+    // kernel and selects it.
+    bool use_sweep() const { return !xchunk && skip_plane == ~0u && (!indexed || Nd * 52 <= SWEEP_BYTES); }
+    template <bool IDX, bool PML>
+    void launch_sweep_k(int p, bool volt) {
+        const FusedGrid fg = fused_grid(p);
+        const PmlSet ps = pml_set(p), pn = pml_set(1 - p);
+        const uint32_t nb = Nx * sweep_plane_blocks(Ny, Pz);
+        if (volt) k_sweep_e<IDX, PML><<<nb, SW_T, 0, stream>>>(fg, ps, pn);
+        else k_sweep_h<IDX, PML><<<nb, SW_T, 0, stream>>>(fg, ps, pn);
+    }
+    void launch_sweep(int p, bool volt) {
+        const bool hp = !pml.empty();
+        if (indexed) { if (hp) launch_sweep_k<true, true>(p, volt); else launch_sweep_k<true, false>(p, volt); }
+        else { if (hp) launch_sweep_k<false, true>(p, volt); else launch_sweep_k<false, false>(p, volt); }
     }
     // UPML cells are updated by k_pml_e / k_pml_h around the fused kernel
     bool pml_split() const { return !pml.empty(); }
@@ -1315,6 +1348,14 @@ efs_status efs_configure_pml(efs_engine* e, uint32_t count, const efs_pml_region
         uint64_t cells = 0;   // the UPML passes of the TMA path index region cells with 32 bits
         for (auto& R : out) cells += (uint64_t)R->n[0] * R->n[1] * R->n[2];
         if (cells >= (1ull << 32)) fail(EFS_ERR_RANGE, "UPML regions hold 2^32 cells or more");
+        std::vector<uint32_t> axis(efs_engine::axis_room(nl[0]) + efs_engine::axis_room(nl[1]) + efs_engine::axis_room(nl[2]), 0);
+        size_t at = 0;
+        for (int d = 0; d < 3; ++d) {
+            for (uint32_t r = 0; r < count; ++r)
+                for (uint32_t c = out[r]->s[d]; c < out[r]->s[d] + out[r]->n[d]; ++c) axis[at + c] |= 1u << r;
+            at += efs_engine::axis_room(nl[d]);
+        }
+        e->upload(e->pml_axis, axis);
         e->pml = std::move(out);
         e->dirty();
     });
@@ -1377,7 +1418,7 @@ static void build_points(efs_engine* e, efs_engine::PointSet& ps, const efs_tfsf
 void efs_engine::plan_tfsf_faces() {
     tf = TfsfFace{0, {0, 0}};
     tf_n = 0;
-    tf_face.reset(); tf_dst.reset(); tf_delay.reset(); tf_frac.reset(); tf_amp.reset();
+    tf_face.reset(); tf_dst.reset(); tf_target.reset(); tf_delay.reset(); tf_frac.reset(); tf_amp.reset();
     if (!tfsf_on) return;
     const size_t nv = h_tfsf_v.size();
     std::vector<uint32_t> tg(nv);
@@ -1414,7 +1455,7 @@ void efs_engine::plan_tfsf_faces() {
         }
     const uint32_t ly = (Ny + 3) & ~3u;
     std::vector<uint8_t> on_face(nv, 0);
-    std::vector<uint32_t> dst, delay;
+    std::vector<uint32_t> dst, target, delay;
     std::vector<float> frac, amp;
     for (size_t i = 0; i < nv; ++i) {
         int f = -1;
@@ -1425,6 +1466,7 @@ void efs_engine::plan_tfsf_faces() {
         const uint32_t n = tg[i] / (uint32_t)Nd, c = tg[i] % (uint32_t)Nd;
         const uint32_t x = c / (Ny * Pz), y = (c / Pz) % Ny;
         dst.push_back(((uint32_t)(f * 2 + n) * Nx + x) * ly + y);
+        target.push_back(tg[i]);
         delay.push_back(h_tfsf_v[i].delay_int); frac.push_back(h_tfsf_v[i].delay_frac); amp.push_back(h_tfsf_v[i].amp);
     }
     // the point pass keeps the other entries, grouped by target in target
@@ -1452,7 +1494,7 @@ void efs_engine::plan_tfsf_faces() {
     alloc(tf_face, nface * 4, false);
     k_fill<<<(unsigned)std::min<size_t>(blocks(nface, 256), 4096), 256, 0, stream>>>(tf_face.as<float>(), nface, -0.0f);
     ck(cudaGetLastError(), "face fill");
-    upload(tf_dst, dst); upload(tf_delay, delay); upload(tf_frac, frac); upload(tf_amp, amp);
+    upload(tf_dst, dst); upload(tf_target, target); upload(tf_delay, delay); upload(tf_frac, frac); upload(tf_amp, amp);
     tf.n = (uint32_t)faces.size();
     for (size_t q = 0; q < faces.size(); ++q) tf.z[q] = faces[q];
     tf_n = (uint32_t)dst.size();
@@ -2168,8 +2210,12 @@ efs_status efs_time_core(efs_engine* e, uint32_t reps, float* ms) {
             return t / reps;
         };
         const int p = e->cur;
-        const float a = timed([&] { e->launch_fused_tma(p); });
-        const float b = e->pml_split() ? timed([&] { e->launch_pml_e(p); }) + timed([&] { e->launch_pml_h(p); }) : 0.f;
+        const bool sweep = e->use_sweep();
+        const float a = timed([&] {
+            if (sweep) { e->launch_sweep(p, true); e->launch_sweep(p, false); }
+            else e->launch_fused_tma(p);
+        });
+        const float b = e->pml_split() && !sweep ? timed([&] { e->launch_pml_e(p); }) + timed([&] { e->launch_pml_h(p); }) : 0.f;
         ck(cudaGetLastError(), "fused launch");
         for (auto& x : ev) cudaEventDestroy(x);
         e->sync("fused timing");
@@ -2193,12 +2239,14 @@ efs_status efs_kernels_per_step(efs_engine* e, uint32_t* out) {
         if (!out) fail(EFS_ERR_INVALID, "out must be non-null");
         e->build_plan();
         // fused kernel, UPML E pass, UPML H pass and deferred H (one paired launch when both)
-        uint32_t k = 1 + e->pml_split() + ((e->defer_n > 0) || e->pml_split());
+        const bool sweep = e->use_sweep(), split = e->pml_split() && !sweep;
+        // E and H sweeps, the TFSF faces added after the first
+        uint32_t k = sweep ? 2 + (e->tf_n > 0) : 1 + split + ((e->defer_n > 0) || split);
         k += e->ss_on + e->ade_v.live() + e->ade_c.live() + 3 * e->mur_on + 2 * e->rlc_on;
         if (e->ade_apply) k += e->ade_v.live() + e->ade_c.live();
         k += (e->tfsf_on && e->tfsf_v.groups) + (e->tfsf_on && e->tfsf_c.groups) + (e->exc_on && e->exc_groups > 0);
         k += e->pbc_on ? 2 * (uint32_t)e->pbc_axes.size() : 0;
-        k += (e->nf_on && !(e->nf_pair && e->pml_split())) + e->ring_on;   // paired samples ride on the UPML E pass
+        k += (e->nf_on && !(e->nf_pair && split)) + e->ring_on;   // paired samples ride on the UPML E pass
         *out = k;
     });
 }

@@ -84,12 +84,11 @@ __device__ __forceinline__ float pml_chain_pp(const PmlSet& ps, const PmlSet& pn
 
 // Regions (bit mask) whose extent along `axis` contains coordinate c.
 __device__ __forceinline__ uint32_t axis_mask(const PmlSet& ps, uint32_t cand, int axis, uint32_t c) {
-    uint32_t m = 0;
-    for (uint32_t b = cand; b; b &= b - 1) {
-        const int r = __ffs(b) - 1;
-        if (c - ps.r[r].s[axis] < ps.r[r].n[axis]) m |= 1u << r;
-    }
-    return m;
+    return cand & __ldg((axis == 0 ? ps.xm : axis == 1 ? ps.ym : ps.zm) + c);
+}
+// Regions that hold the cell.
+__device__ __forceinline__ uint32_t cell_mask(const PmlSet& ps, uint32_t x, uint32_t y, uint32_t z) {
+    return __ldg(ps.xm + x) & __ldg(ps.ym + y) & __ldg(ps.zm + z);
 }
 
 template <bool IDX>

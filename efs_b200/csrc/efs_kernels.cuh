@@ -29,8 +29,14 @@ struct PmlRegion {
     // six float4 {vv, vvfo, vvfn, ii, iifo, iifn} x 3 components (+ pad).
     const uint16_t* cidx; const float4* ctab;
 };
+// Regions by coordinate: bit r of xm[x] says that region r's x range holds x,
+// and so for y and z (zero beyond the grid), so the regions of a cell are three
+// loads that issue with its field loads.  (Walking the regions' bounds took
+// longer than the loads they gate: 86 x 87 x 71 with UPML on all faces.)
+constexpr uint32_t PML_AXIS_PAD = 80;   // zeros behind each axis: tiles overhang the grid
 struct PmlSet {
     int count;
+    const uint32_t* xm; const uint32_t* ym; const uint32_t* zm;
     PmlRegion r[MAX_PML];
 };
 
@@ -461,12 +467,12 @@ constexpr int TF_DY = 12;           // staged rows of a face array per plane (>=
 struct TfsfFaceDev {
     uint32_t n;                     // entries
     const uint32_t* dst;            // index into the face array
+    const uint32_t* target;         // field index
     const uint32_t* delay; const float* frac; const float* amp;
     const float* signal; uint32_t len, period;
     float* face;                    // [face][2][Nx][ly]
 };
-__device__ __forceinline__ void tfsf_face_body(const StepState* st, uint32_t k, const TfsfFaceDev& t, uint32_t i) {
-    if (i >= t.n) return;
+__device__ __forceinline__ float tfsf_face_value(const StepState* st, uint32_t k, const TfsfFaceDev& t, uint32_t i) {
     const int64_t ts = (int64_t)st->numTS + k;
     float v = -0.0f;                // the identity when the entry adds nothing this step
     int64_t d = ts - (int64_t)t.delay[i];
@@ -478,7 +484,18 @@ __device__ __forceinline__ void tfsf_face_body(const StepState* st, uint32_t k, 
             v = __fmul_rn(t.amp[i], sig);
         }
     }
-    t.face[t.dst[i]] = v;
+    return v;
+}
+__device__ __forceinline__ void tfsf_face_body(const StepState* st, uint32_t k, const TfsfFaceDev& t, uint32_t i) {
+    if (i < t.n) t.face[t.dst[i]] = tfsf_face_value(st, k, t, i);
+}
+// The same corrections added to E after a core update that did not apply them.
+__device__ __forceinline__ void tfsf_face_points_body(float* __restrict__ F, const StepState* st, uint32_t k, const TfsfFaceDev& t,
+                                                      uint32_t i) {
+    if (i < t.n) F[t.target[i]] = __fadd_rn(F[t.target[i]], tfsf_face_value(st, k, t, i));
+}
+__global__ void k_tfsf_face_points(float* __restrict__ F, const StepState* st, uint32_t k, const TfsfFaceDev t) {
+    tfsf_face_points_body(F, st, k, t, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void k_tfsf_face(const StepState* st, uint32_t k, const TfsfFaceDev t) {
     tfsf_face_body(st, k, t, blockIdx.x * blockDim.x + threadIdx.x);

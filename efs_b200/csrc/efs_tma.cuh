@@ -583,12 +583,8 @@ __device__ __forceinline__ bool pml_item(const PmlSet& ps, uint32_t i, int& r, u
 
 // Every region containing (x, y, z) when region r is the first that does, else 0.
 __device__ __forceinline__ uint32_t pml_owner_mask(const PmlSet& ps, int r, uint32_t x, uint32_t y, uint32_t z) {
-    for (int q = 0; q < r; ++q)
-        if (in_region(ps.r[q], x, y, z)) return 0u;
-    uint32_t m = 1u << r;
-    for (int q = r + 1; q < ps.count; ++q)
-        if (in_region(ps.r[q], x, y, z)) m |= 1u << q;
-    return m;
+    const uint32_t m = cell_mask(ps, x, y, z);
+    return m & ((1u << r) - 1u) ? 0u : m;
 }
 
 // Region coefficients and old flux of one single-region cell (3 components).

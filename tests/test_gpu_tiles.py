@@ -1,5 +1,9 @@
 """The core update at the edges of its tiles, bit for bit against the f32 oracle.
 
+With an explicit plane depth a grid runs the plane pipeline; without one a
+grid that stays in L2 (or has dense coefficients) runs the E and H sweeps, one
+thread per pair of z-adjacent cells in blocks of 256 pairs of an x-plane.
+
 A tile is 64 (z) x 8 (y) cells over a chunk of x-planes; a thread owns two
 z-adjacent cells and keeps their coefficients while their material repeats
 along x.  Grids end one cell before, on and after a tile or a pair; materials
@@ -44,6 +48,22 @@ def test_tile_edges(cuda_engine_cls, N, depth, coef):
         g.iterate(steps)
         o.iterate(steps)
         compare_fields(g, o, "%s depth %s %s +%d" % (N, depth, coef, steps))
+
+
+@pytest.mark.parametrize("N", [(3, 16, 32), (2, 8, 63), (4, 13, 40), (3, 129, 4), (120, 120, 120), (121, 122, 120)])
+def test_sweep_blocks_and_largest_grid(cuda_engine_cls, N):
+    """Planes of exactly one block, one pair more, many rows; the largest grid that runs as sweeps and one above it."""
+    g, o = engines(cuda_engine_cls, N, materials(N, 9, 3), None)
+    regs = [pml_region((0, 0, 0), (N[0], 4, N[2]), 11), pml_region((1, 4, 0), (1, N[1] - 4, 3), 12)]
+    for e in (g, o):
+        e.configurePML(regs)
+    seed_fields(g, o, N, 10)
+    g.iterate(3)
+    o.iterate(3)
+    compare_fields(g, o, "sweep %s" % (N,))
+    for r in range(2):
+        assert np.array_equal(g.debugRead("pml_volt_flux", r), o.read("pml_volt_flux", r))
+        assert np.array_equal(g.debugRead("pml_curr_flux", r), o.read("pml_curr_flux", r))
 
 
 @pytest.mark.parametrize("depth", [None, 1, 4])
