@@ -5,7 +5,7 @@
 // the batch is the engines' phase order with every phase issued once for all
 // members:
 //   * the core update is one persistent launch of k_fused_tma_batch per kind of
-//     tile present (material index or dense, with or without UPML / TFSF): every
+//     tile present (material index or dense, with or without a TFSF face): every
 //     CTA walks a work-tile list spanning all members (tile = member, 64x8
 //     tile origin, x-chunk) and runs each tile through the same TMA plane
 //     pipeline as the single engine, reading the member's grid, UPML set and
@@ -29,16 +29,14 @@ namespace efs {
 struct BatchMember {            // one member at one step parity (tensor maps first: 64-byte aligned)
     CUtensorMap tmH, tmE, tmM, tmD, tmE1, tmH1;
     FusedGrid g;
-    PmlSet ps;
 };
 struct BatchTile { uint32_t m, xs, y0, z0; };
 
 // Persistent: CTA b runs tiles b, b + gridDim.x, ... of a list whose members
-// all use material-index (IDX) or all dense coefficients and, if !SOME, whose
-// tiles meet neither a UPML region nor a TFSF face corrected in the update.
-// Tiles with and without that code are separate launches: with both bodies in
-// one kernel it spilled (32 stub filters: 620 us against 535 us a step).
-template <bool IDX, bool SOME>
+// all use material-index (IDX) or all dense coefficients and, if !TF, whose
+// tiles meet no TFSF face corrected in the update (with both bodies in one
+// kernel it spilled registers).
+template <bool IDX, bool TF>
 __global__ void __launch_bounds__(TT_THREADS, 2)
 k_fused_tma_batch(const BatchMember* __restrict__ mem, const BatchTile* __restrict__ tiles, uint32_t ntiles) {
     TmaSmem& S = tt_smem();
@@ -47,8 +45,7 @@ k_fused_tma_batch(const BatchMember* __restrict__ mem, const BatchTile* __restri
     for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const BatchTile w = tiles[t];
         const BatchMember& M = mem[w.m];
-        if (!tma_tile_body<IDX, SOME, SOME>(S, TmaMaps{&M.tmH, &M.tmE, &M.tmM, &M.tmD, &M.tmE1, &M.tmH1}, M.g, M.ps, w.xs, w.y0,
-                                            w.z0, rg))
+        if (!tma_tile_body<IDX, TF>(S, TmaMaps{&M.tmH, &M.tmE, &M.tmM, &M.tmD, &M.tmE1, &M.tmH1}, M.g, w.xs, w.y0, w.z0, rg))
             break;
     }
     tt_done();
@@ -66,6 +63,11 @@ __global__ void __launch_bounds__(256) k_seg(const Op* __restrict__ ops, SegMap 
     ops[s].run(blockIdx.x - sm.first[s], k, a, b);
 }
 
+template <bool IDX>
+struct OpMurAdopt {
+    FusedGrid g; float* V; MurAdoptDev d;
+    __device__ void run(uint32_t blk, uint32_t, uint32_t, uint32_t) const { mur_adopt_body<IDX>(g, V, d, blk * blockDim.x + threadIdx.x); }
+};
 struct OpMurPre {
     const float* V; MurDev m;
     __device__ void run(uint32_t blk, uint32_t, uint32_t, uint32_t) const { mur_pre_body(V, m, blk * blockDim.x + threadIdx.x); }
@@ -174,10 +176,11 @@ struct efs_batch {
     // plan, per step phase s (member e at batch step k uses parity cur0[e] ^ s, s = (phase + k) & 1)
     bool planned = false;
     std::vector<int> cur0;
+    std::vector<uint64_t> gen;                 // the members' plans this plan was made from
     uint32_t phase = 0;
     DevBuf members[2], tiles[4];               // tile lists by tile_class
     uint32_t ntiles[4] = {0, 0, 0, 0};
-    SegLaunch mur_pre[2], mur_post[2], mur_apply[2], exc[2], tfsf_v[2], tfsf_c[2], ade_v[2], ade_c[2], ade_apply_v[2], ade_apply_c[2],
+    SegLaunch mur_adopt_i[2], mur_adopt_d[2], mur_pre[2], mur_post[2], mur_apply[2], exc[2], tfsf_v[2], tfsf_c[2], ade_v[2], ade_c[2], ade_apply_v[2], ade_apply_c[2],
         ring[2], nf_sample[2], nf_flush[2],
         deferred_i[2], deferred_d[2], pml_e_i[2], pml_e_d[2], pml_h_i[2], pml_h_d[2], tfsf_face[2], advance;   // _i / _d: index / dense members
     bool any_nf = false;
@@ -248,22 +251,16 @@ struct efs_batch {
         return pick;
     }
     // Tile list of a work tile: bit 0: material-index member; bit 1: the tile
-    // meets a UPML region or a TFSF face of the core update (the tests of tma_tile).
-    int tile_class(const efs_engine* e, uint32_t xs, uint32_t y0, uint32_t z0) const {
-        bool some = false;
-        for (uint32_t f = 0; f < e->tf.n; ++f) some |= e->tf.z[f] >= z0 && e->tf.z[f] <= z0 + TT_Z;
-        const uint32_t lo[3] = {xs, y0, z0}, hi[3] = {xs + xc, y0 + TT_Y, z0 + TT_Z};
-        for (auto& R : e->pml) {
-            bool hit = true;
-            for (int d = 0; d < 3; ++d) hit = hit && hi[d] >= R->s[d] && lo[d] < R->s[d] + R->n[d];
-            some |= hit;
-        }
-        return (e->indexed ? 1 : 0) + (some ? 2 : 0);
+    // meets a TFSF face of the core update (the test of tma_tile).
+    int tile_class(const efs_engine* e, uint32_t z0) const {
+        bool tf = false;
+        for (uint32_t f = 0; f < e->tf.n; ++f) tf |= e->tf.z[f] >= z0 && e->tf.z[f] <= z0 + TT_Z;
+        return (e->indexed ? 1 : 0) + (tf ? 2 : 0);
     }
-    template <bool IDX, bool SOME>
+    template <bool IDX, bool TF>
     void launch_tiles(int t, const BatchMember* bm) {
         if (ntiles[t])
-            k_fused_tma_batch<IDX, SOME><<<std::min<uint32_t>(ntiles[t], ctas_per_sm * sms), TT_THREADS, TT_SMEM_BYTES, stream>>>(
+            k_fused_tma_batch<IDX, TF><<<std::min<uint32_t>(ntiles[t], ctas_per_sm * sms), TT_THREADS, TT_SMEM_BYTES, stream>>>(
                 bm, tiles[t].as<BatchTile>(), ntiles[t]);
     }
 
@@ -273,11 +270,14 @@ struct efs_batch {
         const size_t E = mem.size();
         xc = xchunk ? xchunk : pick_depth();
         cur0.resize(E);
-        for (size_t i = 0; i < E; ++i) { mem[i]->build_plan(); cur0[i] = mem[i]->cur; }
+        gen.resize(E);
+        for (size_t i = 0; i < E; ++i) { mem[i]->build_plan(); cur0[i] = mem[i]->cur; gen[i] = mem[i]->plan_gen; }
         phase = 0;
         any_nf = false;
         for (int s = 0; s < 2; ++s) {
             std::vector<BatchMember> bm(E);
+            std::vector<std::pair<uint32_t, OpMurAdopt<true>>> vmi;
+            std::vector<std::pair<uint32_t, OpMurAdopt<false>>> vmd;
             std::vector<std::pair<uint32_t, OpMurPre>> mpre;
             std::vector<std::pair<uint32_t, OpMurPost>> mpost;
             std::vector<std::pair<uint32_t, OpMurApply>> mapply;
@@ -306,21 +306,25 @@ struct efs_batch {
                 const uint32_t bh[4] = {TT_HZ, TT_HY, 1, 3}, be[4] = {TT_EZ, TT_EY, 1, 3}, bs[4] = {TT_Z, TT_Y, 1, 3};
                 M.tmH = e->tensor_map(fg.H0, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bh);
                 M.tmE = e->tensor_map(fg.V0, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, be);
-                M.tmM = e->indexed ? e->tensor_map(fg.mat, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, be) : M.tmE;
+                M.tmM = fg.mat ? e->tensor_map(fg.mat, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, be) : M.tmE;
                 M.tmD = e->tf.n ? e->tf_map() : M.tmE;
                 M.tmE1 = e->tensor_map(fg.V1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs);
                 M.tmH1 = e->tensor_map(fg.H1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs);
                 M.g = fg;
                 M.g.xchunk = xc;
-                M.ps = ps;
                 float* V = e->vbuf(p);
                 float* V1 = e->vbuf(q);
                 float* C1 = e->cbuf(q);
                 StepState* st = e->state.as<StepState>();
                 const MurDev md = e->mur_dev(e->vflux_ptrs[p].as<const float*>());
-                if (e->mur_on) {
-                    mpre.push_back({e->mur_n, OpMurPre{V, md}});
-                    mpost.push_back({e->mur_n, OpMurPost{V1, md}});
+                if (e->mur_fast) {
+                    const uint32_t cnt = e->mur_threads();
+                    if (e->indexed) vmi.push_back({cnt, OpMurAdopt<true>{fg, V, e->mur_adopt_dev()}});
+                    else vmd.push_back({cnt, OpMurAdopt<false>{fg, V, e->mur_adopt_dev()}});
+                }
+                if (e->mur_gen) {
+                    mpre.push_back({e->mur_gen, OpMurPre{V, md}});
+                    mpost.push_back({e->mur_gen, OpMurPost{V1, md}});
                     mapply.push_back({e->mur_napply, OpMurApply{V1, md}});
                 }
                 if (e->exc_on && e->exc_groups) {
@@ -368,6 +372,8 @@ struct efs_batch {
                 }
             }
             upload_raw(members[s], bm.data(), bm.size() * sizeof(BatchMember));
+            build_seg(mur_adopt_i[s], vmi);
+            build_seg(mur_adopt_d[s], vmd);
             build_seg(mur_pre[s], mpre);
             build_seg(mur_post[s], mpost);
             build_seg(mur_apply[s], mapply);
@@ -401,7 +407,7 @@ struct efs_batch {
             const efs_engine* e = mem[i];
             for (uint32_t xs = 0; xs < e->Nx; xs += xc)
                 for (uint32_t y0 = 0; y0 < e->Ny; y0 += TT_Y)
-                    for (uint32_t z0 = 0; z0 < e->Nz; z0 += TT_Z) tl[tile_class(e, xs, y0, z0)].push_back(BatchTile{(uint32_t)i, xs, y0, z0});
+                    for (uint32_t z0 = 0; z0 < e->Nz; z0 += TT_Z) tl[tile_class(e, z0)].push_back(BatchTile{(uint32_t)i, xs, y0, z0});
         }
         // a batch of few tiles runs them all in one launch: two short ones leave two half-empty
         // last waves (16 members of 40-96 lines, 1,100 tiles: 101 us in two, 89 us in one)
@@ -427,6 +433,8 @@ struct efs_batch {
         launch_seg<OpPmlE<false>>(pml_e_d[s], k); // to the old flux, which this pass does not write)
         mark(1);
         launch_seg<OpAde>(ade_v[s], k);          // pre-voltage, as the single engine: ADE(volt), Mur pre
+        launch_seg<OpMurAdopt<true>>(mur_adopt_i[s], k);
+        launch_seg<OpMurAdopt<false>>(mur_adopt_d[s], k);
         launch_seg<OpMurPre>(mur_pre[s], k);
         launch_seg<OpAde>(ade_c[s], k);          // ADE(curr) before the core update rewrites H and the flux
         launch_seg<OpTfsfFace>(tfsf_face[s], k); // TFSF face values the core update adds
@@ -523,7 +531,7 @@ struct efs_batch {
     bool stale() const {
         if (!planned) return true;
         for (size_t i = 0; i < mem.size(); ++i)
-            if (mem[i]->plan_dirty || mem[i]->cur != (cur0[i] ^ (int)phase)) return true;
+            if (mem[i]->plan_dirty || mem[i]->plan_gen != gen[i] || mem[i]->cur != (cur0[i] ^ (int)phase)) return true;
         return false;
     }
 

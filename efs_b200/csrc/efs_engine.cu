@@ -153,7 +153,7 @@ struct efs_engine {
     uint32_t skip_plane = ~0u;          // diagnostics (efs_debug_set_wait): a plane whose loads are never issued
     DevBuf defer_cells;
     uint32_t defer_n = 0;
-    std::vector<uint32_t> h_exc_targets, h_tfsf_v_targets, h_mur_apply, h_rlc_series;
+    std::vector<uint32_t> h_exc_targets, h_tfsf_v_targets, h_rlc_series;
     bool indexed = false;
     DevBuf mat, table, vv, vi, ii, iv;
     uint32_t ntable = 0;
@@ -246,6 +246,18 @@ struct efs_engine {
     std::vector<uint32_t> h_mur_normal, h_mur_shifted;
     DevBuf mur_coeff, mur_pre_normal, mur_pre_shifted, mur_shifted, mur_apply_target, mur_apply_src, mur_saved;
     uint32_t mur_n = 0, mur_napply = 0;
+    // the plan's split: entries the core update adopts (k_mur_adopt; mur_fast: any) and entries of the three passes
+    bool mur_fast = false;
+    uint32_t mur_gen = 0, mur_nslots = 0;
+    std::vector<uint32_t> h_mur_gen_apply;   // targets the apply pass writes after the core update
+    DevBuf mur_ids, mur_kind, mur_target, mur_slot;
+    void plan_mur();
+    MurAdoptDev mur_adopt_dev() const {
+        return MurAdoptDev{mur_n, mur_first(), mur_nslots, mur_target.as<uint32_t>(), mur_shifted.as<uint32_t>(), mur_coeff.as<float>(),
+                           mur_kind.as<uint8_t>(), mur_slot.as<uint32_t>(), mur_saved.as<float>()};
+    }
+    uint32_t mur_first() const { return (mur_n + 31) & ~31u; }
+    uint32_t mur_threads() const { return mur_nslots ? mur_first() + mur_nslots : mur_n; }   // of k_mur_adopt
 
     // TFSF
     bool tfsf_on = false;
@@ -323,6 +335,7 @@ struct efs_engine {
 
     // graphs
     bool plan_dirty = true;
+    uint64_t plan_gen = 0;           // plans built (a batch holds pointers of one)
     std::map<uint32_t, cudaGraphExec_t> graphs;
 
     ~efs_engine() {
@@ -461,15 +474,9 @@ struct efs_engine {
             upload(cflux_ptrs[p], cp);
         }
         plan_tfsf_faces();
+        plan_mur();
         build_deferred();
-        if (mur_on) {
-            std::vector<ReadLoc> rn(mur_n), rs(mur_n);
-            parallel_chunks(mur_n, host_threads(mur_n), [&](unsigned, size_t lo, size_t hi) {
-                for (size_t i = lo; i < hi; ++i) { rn[i] = redirect(h_mur_normal[i]); rs[i] = redirect(h_mur_shifted[i]); }
-            });
-            upload(mur_pre_normal, rn);
-            upload(mur_pre_shifted, rs);
-        }
+        mark_adopted();
         for (AdeSide* s : {&ade_v, &ade_c}) {
             if (!s->n) continue;
             std::vector<AdeRun> runs;
@@ -498,6 +505,7 @@ struct efs_engine {
             if (ade_apply) build_ade_apply(*s);
         }
         plan_dirty = false;
+        ++plan_gen;
     }
 
     // Apply-step plan of one ADE side: runs over consecutive field locations
@@ -573,7 +581,7 @@ struct efs_engine {
         auto add = [&](const std::vector<uint32_t>& v) { mod.insert(mod.end(), v.begin(), v.end()); };
         if (tfsf_on) add(h_tfsf_v_targets);
         if (exc_on) add(h_exc_targets);
-        if (mur_on) add(h_mur_apply);
+        if (mur_gen) add(h_mur_gen_apply);
         if (rlc_on) add(h_rlc_series);
         if (ade_apply && ade_v.live()) add(ade_v.h_field);
         const uint32_t nl[3] = {Nx, Ny, Nz};
@@ -698,7 +706,8 @@ struct efs_engine {
         mark(1);
         if (ade_v.live()) k_ade<<<blocks(ade_v.n, ADE_BLOCK), ADE_T, 0, stream>>>(V, ade_dev(ade_v, vfl));
         MurDev md = mur_dev(vfl);
-        if (mur_on) k_mur_pre<<<blocks(mur_n, T), T, 0, stream>>>(V, md);
+        if (mur_fast) launch_mur_adopt(p);
+        if (mur_gen) k_mur_pre<<<blocks(mur_gen, T), T, 0, stream>>>(V, md);
         RlcDev rd = rlc_dev();
         if (rlc_on) k_rlc_pre<<<blocks(rlc_n, T), T, 0, stream>>>(rd);
         // ADE(curr) reads H and the current flux, which the E side never
@@ -713,13 +722,13 @@ struct efs_engine {
         if (tf_n && sweep) k_tfsf_face_points<<<blocks(tf_n, T), T, 0, stream>>>(V1, st, k, tf_dev());
         if (tfsf_on && tfsf_v.groups) k_point_sources<1><<<blocks(tfsf_v.groups, T), T, 0, stream>>>(V1, st, k, point_dev(tfsf_v, tfsf_signal, tfsf_len, tfsf_period));
         if (pbc_on) for (auto& a : pbc_axes) launch_pbc(a, true, V1);
-        if (mur_on) k_mur_post<<<blocks(mur_n, T), T, 0, stream>>>(V1, md);
+        if (mur_gen) k_mur_post<<<blocks(mur_gen, T), T, 0, stream>>>(V1, md);
         if (exc_on && exc_groups) {
             PointSources s{exc_groups, exc_target.as<uint32_t>(), exc_off.as<uint32_t>(), exc_delay.as<uint32_t>(),
                            exc_amp.as<float>(), nullptr, exc_signal.as<float>(), exc_len, exc_period};
             k_point_sources<0><<<blocks(exc_groups, T), T, 0, stream>>>(V1, st, k, s);
         }
-        if (mur_on) k_mur_apply<<<blocks(mur_napply, T), T, 0, stream>>>(V1, md);
+        if (mur_gen) k_mur_apply<<<blocks(mur_napply, T), T, 0, stream>>>(V1, md);
         if (rlc_on) k_rlc_apply<<<blocks(rlc_groups, T), T, 0, stream>>>(V1, rd);
         if (ade_apply && ade_v.live()) launch_ade_apply(ade_v, V1);
         mark(4);
@@ -769,6 +778,29 @@ struct efs_engine {
     template <class A, class B>
     void pair(const A& a, uint32_t na, const B& b, uint32_t nb) {
         if (na + nb) k_pair<A, B><<<na + nb, 256, 0, stream>>>(a, na, b, nb);
+    }
+    void launch_mur_adopt(int p) {
+        const uint32_t T = 256, nb = blocks(mur_threads(), T);
+        if (indexed) k_mur_adopt<true><<<nb, T, 0, stream>>>(fused_grid(p), vbuf(p), mur_adopt_dev());
+        else k_mur_adopt<false><<<nb, T, 0, stream>>>(fused_grid(p), vbuf(p), mur_adopt_dev());
+    }
+    // The adopt bits of the material index: UPML cells and the Mur targets of
+    // k_mur_adopt.  A dense engine gets an array for them when it has any.
+    void mark_adopted() {
+        if (!mat.p) {
+            if (pml.empty() && !mur_fast) return;
+            alloc(mat, Nd * 4);
+        } else {
+            k_mat_clear<<<(unsigned)std::min<size_t>(blocks(Nd, 256), 148 * 16), 256, 0, stream>>>(mat.as<uint32_t>(), Nd);
+        }
+        for (auto& R : pml) {
+            const uint32_t cells = (uint32_t)(R->total / 3);   // < 2^32 (efs_configure_pml)
+            if (cells)
+                k_mat_box<<<blocks(cells, 256), 256, 0, stream>>>(mat.as<uint32_t>(), Ny, Pz, R->s[0], R->s[1], R->s[2], R->n[1],
+                                                                  R->n[2], cells);
+        }
+        if (mur_fast) k_mat_mur<<<blocks(mur_n, 256), 256, 0, stream>>>(mat.as<uint32_t>(), (uint32_t)Nd, mur_adopt_dev());
+        ck(cudaGetLastError(), "adopt bits");
     }
     void launch_deferred(int p) {
         const uint32_t T = 256;
@@ -838,30 +870,28 @@ struct efs_engine {
         if (r != CUDA_SUCCESS) fail(EFS_ERR_CUDA, "cuTensorMapEncodeTiled failed (code " + std::to_string((int)r) + ")");
         return m;
     }
-    template <bool IDX, bool PML>
-    void launch_fused_tma_k(dim3 g, const CUtensorMap (&t)[6], const FusedGrid& fg, const PmlSet& ps) {
+    template <bool IDX>
+    void launch_fused_tma_k(dim3 g, const CUtensorMap (&t)[6], const FusedGrid& fg) {
         static bool attr_set = false;   // per instantiation; the attribute is per kernel, all devices alike
         if (!attr_set) {
-            ck(cudaFuncSetAttribute(k_fused_tma<IDX, PML>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT_SMEM_BYTES),
+            ck(cudaFuncSetAttribute(k_fused_tma<IDX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT_SMEM_BYTES),
                "smem attr");
             attr_set = true;
         }
-        k_fused_tma<IDX, PML><<<g, TT_THREADS, TT_SMEM_BYTES, stream>>>(t[0], t[1], t[2], t[3], t[4], t[5], fg, ps);
+        k_fused_tma<IDX><<<g, TT_THREADS, TT_SMEM_BYTES, stream>>>(t[0], t[1], t[2], t[3], t[4], t[5], fg);
     }
     void launch_fused_tma(int p) {
         const FusedGrid fg = fused_grid(p);
-        const PmlSet ps = pml_set(p);
         const uint32_t bh[4] = {TT_HZ, TT_HY, 1, 3}, be[4] = {TT_EZ, TT_EY, 1, 3}, bs[4] = {TT_Z, TT_Y, 1, 3};
         const CUtensorMap tE = tensor_map(fg.V0, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, be);
         const CUtensorMap t[6] = {tensor_map(fg.H0, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bh), tE,
-                                  indexed ? tensor_map(fg.mat, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, be) : tE,
+                                  fg.mat ? tensor_map(fg.mat, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, be) : tE,
                                   tf.n ? tf_map() : tE,      // unused without TFSF faces
                                   tensor_map(fg.V1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs),
                                   tensor_map(fg.H1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs)};
         dim3 g(blocks(Nz, TT_Z), blocks(Ny, TT_Y), blocks(Nx, fg.xchunk));
-        const bool hp = !pml.empty();
-        if (indexed) { if (hp) launch_fused_tma_k<true, true>(g, t, fg, ps); else launch_fused_tma_k<true, false>(g, t, fg, ps); }
-        else { if (hp) launch_fused_tma_k<false, true>(g, t, fg, ps); else launch_fused_tma_k<false, false>(g, t, fg, ps); }
+        if (indexed) launch_fused_tma_k<true>(g, t, fg);
+        else launch_fused_tma_k<false>(g, t, fg);
     }
     // E and H sweeps (efs_sweep.cuh) instead of the fused kernel and the passes
     // around it: while both parities of the fields and the material index stay
@@ -916,7 +946,7 @@ struct efs_engine {
                       s.lor.as<float>(), flux};
     }
     MurDev mur_dev(const float* const* vfl) const {
-        return MurDev{mur_n, mur_napply, mur_coeff.as<float>(), mur_pre_normal.as<ReadLoc>(), mur_pre_shifted.as<ReadLoc>(),
+        return MurDev{mur_gen, mur_napply, mur_ids.as<uint32_t>(), mur_coeff.as<float>(), mur_pre_normal.as<ReadLoc>(), mur_pre_shifted.as<ReadLoc>(),
                       mur_shifted.as<uint32_t>(), mur_apply_target.as<uint32_t>(), mur_apply_src.as<uint32_t>(),
                       mur_saved.as<float>(), vfl};
     }
@@ -1028,7 +1058,7 @@ void alloc_fields(efs_engine* e, const uint32_t dims[3]) {
     e->ade_apply = false;
     e->gd_n = 0;
     e->Nx = dims[0]; e->Ny = dims[1]; e->Nz = dims[2]; e->N = N; e->Pz = Pz; e->Nd = Nd;
-    e->h_exc_targets.clear(); e->h_tfsf_v_targets.clear(); e->h_mur_apply.clear(); e->h_rlc_series.clear();
+    e->h_exc_targets.clear(); e->h_tfsf_v_targets.clear(); e->h_rlc_series.clear();
     e->h_tfsf_v.clear();
     e->tf = TfsfFace{0, {0, 0}};
     e->tf_n = 0;
@@ -1153,13 +1183,13 @@ efs_status efs_init_indexed(efs_engine* e, const uint32_t dims[3], const uint32_
         alloc_fields(e, dims);
         // indices are checked on the device after the upload (pad cells hold 0)
         e->upload_padded(e->mat, mat, 1);
+        uint32_t hmax = 0;
         {
             DevBuf mx;
             e->alloc(mx, 4);
             k_max_u32<<<std::min<uint32_t>(blocks(e->Nd, 256), 148 * 8), 256, 0, e->stream>>>(e->mat.as<uint32_t>(), e->Nd,
                                                                                                mx.as<uint32_t>());
             ck(cudaGetLastError(), "material index check");
-            uint32_t hmax = 0;
             ck(cudaMemcpyAsync(&hmax, mx.p, 4, cudaMemcpyDeviceToHost, e->stream), "material index check");
             e->sync("material index check");
             if (hmax >= ntable) {
@@ -1167,9 +1197,20 @@ efs_status efs_init_indexed(efs_engine* e, const uint32_t dims[3], const uint32_
                 fail(EFS_ERR_INVALID, "material index out of range");
             }
         }
-        e->indexed = true;
-        e->ntable = ntable;
-        e->upload(e->table, table, (size_t)ntable * 12);
+        e->indexed = hmax <= MAT_MASK;
+        if (e->indexed) {
+            e->ntable = ntable;
+            e->upload(e->table, table, (size_t)ntable * 12);
+        } else {                   // indices that reach the adopt bits (tables above 25 GB): as dense arrays
+            e->mat.reset();
+            std::vector<float> a(3 * e->N);
+            DevBuf* dst[4] = {&e->vv, &e->vi, &e->ii, &e->iv};
+            for (int k = 0; k < 4; ++k) {
+                for (int n = 0; n < 3; ++n)
+                    for (size_t c = 0; c < e->N; ++c) a[n * e->N + c] = table[(size_t)mat[c] * 12 + 3 * k + n];
+                e->upload_padded(*dst[k], a.data(), 3);
+            }
+        }
         e->sync_state_to_device();
         e->inited = true;
         e->dirty();
@@ -1378,20 +1419,15 @@ efs_status efs_configure_mur(efs_engine* e, const float* coeff, const uint32_t* 
         std::vector<uint32_t> ss(n);
         std::vector<float> sc(n);
         for (uint32_t k = 0; k < n; ++k) { ss[k] = e->dev_index(shifted[perm[k]]); sc[k] = coeff[perm[k]]; }
-        // apply: per distinct normal (ascending) its last writer in the caller's
-        // order, which is the last entry of its run in the sorted order
-        std::vector<uint32_t> at, as;
-        for (uint32_t k = 0; k < n; ++k)
-            if (k + 1 == n || sn[k + 1] != sn[k]) { at.push_back(sn[k]); as.push_back(k); }
+        // apply: per distinct normal its last writer in the caller's order, which
+        // is the last entry of its run in the sorted order (plan_mur)
         e->h_mur_normal = sn;
         e->h_mur_shifted = ss;
         e->upload(e->mur_coeff, sc);
-        e->upload(e->mur_shifted, ss);
-        e->upload(e->mur_apply_target, at); e->upload(e->mur_apply_src, as);
+        e->upload(e->mur_target, sn); e->upload(e->mur_shifted, ss);
         e->mur_perm = perm;
-        e->h_mur_apply = at;
         e->alloc(e->mur_saved, (size_t)n * 4);
-        e->mur_n = n; e->mur_napply = (uint32_t)at.size();
+        e->mur_n = n;
         e->mur_on = n > 0;
         e->dirty();
     });
@@ -1499,6 +1535,105 @@ void efs_engine::plan_tfsf_faces() {
     for (size_t q = 0; q < faces.size(); ++q) tf.z[q] = faces[q];
     tf_n = (uint32_t)dst.size();
     tf_ly = ly;
+}
+
+// Mur entries: which ones k_mur_adopt computes before the core update.  An
+// entry qualifies when nothing but the core update comes between E_old and what
+// the reference's post step reads at its shifted cell, and nothing after its
+// apply step's place in the reference changes what the core update then adopts
+// at its target: neither cell in a UPML region or rewritten by TFSF, no
+// excitation on the target, no periodic axis.  Entries that share cells (grid
+// edges) qualify together, in groups whose lanes sit in one warp.
+void efs_engine::plan_mur() {
+    mur_fast = false;
+    mur_gen = mur_nslots = mur_napply = 0;
+    h_mur_gen_apply.clear();
+    if (!mur_on) return;
+    const size_t n = mur_n;
+    const std::vector<uint32_t>&t = h_mur_normal, &sh = h_mur_shifted;      // t ascends
+    // one bit per field location: Mur targets, and targets of TFSF and excitation
+    const size_t words = (3 * Nd + 31) / 32;
+    auto bitmap = [&] { return std::unique_ptr<uint32_t, decltype(&free)>((uint32_t*)calloc(words, 4), &free); };
+    auto T = bitmap(), F = bitmap();
+    if (!T || !F) fail(EFS_ERR_OOM, "Mur plan: out of host memory");
+    auto set = [](uint32_t* b, uint32_t i) { __atomic_fetch_or(&b[i >> 5], 1u << (i & 31), __ATOMIC_RELAXED); };
+    auto has = [](const uint32_t* b, uint32_t i) { return (b[i >> 5] >> (i & 31)) & 1u; };
+    const unsigned W = host_threads(n);
+    parallel_chunks(n, W, [&](unsigned, size_t lo, size_t hi) { for (size_t i = lo; i < hi; ++i) set(T.get(), t[i]); });
+    if (tfsf_on)
+        parallel_chunks(h_tfsf_v.size(), host_threads(h_tfsf_v.size()), [&](unsigned, size_t lo, size_t hi) {
+            for (size_t i = lo; i < hi; ++i) set(F.get(), dev_index(h_tfsf_v[i].field_idx));
+        });
+    std::vector<uint32_t> exc;
+    if (exc_on) { exc = h_exc_targets; std::sort(exc.begin(), exc.end()); }
+    std::vector<uint8_t> kind(n, 0), ok(n, 0), shared(n, 0);
+    constexpr uint8_t WRITES = 1, READS = 2, GROUPED = 4;     // shared: target shared; shifted cell is a target; in a group
+    parallel_chunks(n, W, [&](unsigned, size_t lo, size_t hi) {
+        for (size_t i = lo; i < hi; ++i) {
+            ok[i] = !pbc_on && !has(F.get(), t[i]) && !has(F.get(), sh[i]) && redirect(t[i]).sel == 0 && redirect(sh[i]).sel == 0 &&
+                    !std::binary_search(exc.begin(), exc.end(), t[i]);
+            if (i + 1 == n || t[i + 1] != t[i]) kind[i] = MUR_LAST;
+            shared[i] = ((i > 0 && t[i - 1] == t[i]) || (i + 1 < n && t[i + 1] == t[i]) ? WRITES : 0) | (has(T.get(), sh[i]) ? READS : 0);
+        }
+    });
+    std::vector<uint32_t> read;                               // targets that some entry reads at its shifted cell
+    for (size_t i = 0; i < n; ++i)
+        if (shared[i] & READS) read.push_back(sh[i]);
+    std::sort(read.begin(), read.end());
+    read.erase(std::unique(read.begin(), read.end()), read.end());
+    parallel_chunks(n, W, [&](unsigned, size_t lo, size_t hi) {
+        for (size_t i = lo; i < hi; ++i) if (std::binary_search(read.begin(), read.end(), t[i])) shared[i] |= WRITES;
+    });
+    // entries that share cells: connected through their targets
+    std::vector<uint32_t> ents, slot;
+    for (size_t i = 0; i < n; ++i)
+        if (shared[i]) ents.push_back((uint32_t)i);
+    std::unordered_map<uint32_t, uint32_t> node;              // target -> node
+    std::vector<uint32_t> up;
+    auto find = [&](uint32_t a) { while (up[a] != a) a = up[a] = up[up[a]]; return a; };
+    auto of = [&](uint32_t target) {
+        auto r = node.emplace(target, (uint32_t)up.size());
+        if (r.second) up.push_back((uint32_t)up.size());
+        return r.first->second;
+    };
+    for (uint32_t i : ents) {
+        const uint32_t a = of(t[i]);
+        if (shared[i] & READS) { const uint32_t b = of(sh[i]); up[find(a)] = find(b); }
+    }
+    std::vector<std::vector<uint32_t>> group(up.size());
+    for (uint32_t i : ents) group[find(of(t[i]))].push_back(i);
+    for (auto& g : group) {
+        if (g.empty() || g.size() > MUR_GROUP) continue;
+        bool all = true;
+        for (uint32_t i : g) all = all && ok[i];
+        if (!all) continue;
+        if (slot.size() % 32 + g.size() > 32) slot.resize((slot.size() + 31) & ~(size_t)31, ~0u);
+        for (uint32_t i : g) { slot.push_back(i); shared[i] = GROUPED; }
+    }
+    std::vector<uint32_t> ids, at, as;
+    size_t singles = 0;
+    for (size_t i = 0; i < n; ++i) {
+        if (shared[i] == GROUPED) continue;
+        if (!shared[i] && ok[i]) { kind[i] |= MUR_SINGLE; ++singles; continue; }
+        ids.push_back((uint32_t)i);
+        if (kind[i] & MUR_LAST) { at.push_back(t[i]); as.push_back((uint32_t)i); }
+        kind[i] = 0;
+    }
+    mur_nslots = (uint32_t)slot.size();
+    mur_fast = singles > 0 || mur_nslots > 0;
+    mur_gen = (uint32_t)ids.size();
+    mur_napply = (uint32_t)at.size();
+    h_mur_gen_apply = at;
+    upload(mur_kind, kind);
+    if (mur_nslots) upload(mur_slot, slot);
+    if (mur_gen) {
+        upload(mur_ids, ids);
+        upload(mur_apply_target, at); upload(mur_apply_src, as);
+        std::vector<ReadLoc> rn(n), rs(n);
+        for (uint32_t i : ids) { rn[i] = redirect(t[i]); rs[i] = redirect(sh[i]); }
+        upload(mur_pre_normal, rn);
+        upload(mur_pre_shifted, rs);
+    }
 }
 
 efs_status efs_configure_tfsf(efs_engine* e, const float* signal, uint32_t L, uint32_t period, const efs_tfsf_point* vp,
@@ -2242,7 +2377,7 @@ efs_status efs_kernels_per_step(efs_engine* e, uint32_t* out) {
         const bool sweep = e->use_sweep(), split = e->pml_split() && !sweep;
         // E and H sweeps, the TFSF faces added after the first
         uint32_t k = sweep ? 2 + (e->tf_n > 0) : 1 + split + ((e->defer_n > 0) || split);
-        k += e->ss_on + e->ade_v.live() + e->ade_c.live() + 3 * e->mur_on + 2 * e->rlc_on;
+        k += e->ss_on + e->ade_v.live() + e->ade_c.live() + e->mur_fast + 3 * (e->mur_gen > 0) + 2 * e->rlc_on;
         if (e->ade_apply) k += e->ade_v.live() + e->ade_c.live();
         k += (e->tfsf_on && e->tfsf_v.groups) + (e->tfsf_on && e->tfsf_c.groups) + (e->exc_on && e->exc_groups > 0);
         k += e->pbc_on ? 2 * (uint32_t)e->pbc_axes.size() : 0;

@@ -26,13 +26,20 @@ namespace efs {
 
 constexpr int PML_MAX_OVERLAP = 4;
 
+// The material index of a cell carries, in its top three bits, the E components
+// (bit 29 + n) whose E_new is known before the core update and stands in place
+// of E_old in the step's old-E buffer: the core update adopts it as is.  These
+// are all components of UPML cells (k_pml_e) and the Mur targets that
+// k_mur_adopt computes.  With dense coefficients the array holds these bits alone.
+constexpr uint32_t MAT_BITS = 29, MAT_MASK = (1u << MAT_BITS) - 1u;
+
 struct FusedGrid {
     uint32_t Nx, Ny, Nz, xchunk;
     uint32_t Pz;                        // z pitch of the device layout (Nz rounded up to a multiple of 4)
     size_t N, NyNz;                     // device component stride Nx*Ny*Pz and plane stride Ny*Pz
     const float* V0; const float* H0;   // fields at the start of the step
     float* V1; float* H1;               // fields after the step
-    const uint32_t* mat; const float* table;
+    const uint32_t* mat; const float* table;   // mat: null with dense coefficients and no adopted cell
     const float* vv; const float* vi; const float* ii; const float* iv;
     uint32_t* status;                   // device status word (bit 0: a bounded wait ran out)
     uint64_t wait_ns;                   // limit of every bounded mbarrier wait (about 1 s)
@@ -95,7 +102,7 @@ template <bool IDX>
 __device__ __forceinline__ void coeffs_f(const FusedGrid& g, size_t c, uint32_t m, int base, float out[6]) {
     if (IDX) {
         // a 48-byte row is three float4: [vv0 vv1 vv2 vi0][vi1 vi2 ii0 ii1][ii2 iv0 iv1 iv2]
-        const float4* t = reinterpret_cast<const float4*>(g.table) + (size_t)m * 3;
+        const float4* t = reinterpret_cast<const float4*>(g.table) + (size_t)(m & MAT_MASK) * 3;
         if (base == 0) {
             const float4 a = __ldg(t), b = __ldg(t + 1);
             out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w; out[4] = b.x; out[5] = b.y;
@@ -109,6 +116,88 @@ __device__ __forceinline__ void coeffs_f(const FusedGrid& g, size_t c, uint32_t 
         out[0] = __ldg(a + c); out[1] = __ldg(a + g.N + c); out[2] = __ldg(a + 2 * g.N + c);
         out[3] = __ldg(b + c); out[4] = __ldg(b + g.N + c); out[5] = __ldg(b + 2 * g.N + c);
     }
+}
+
+// Adopt bits of the material index (one launch per UPML region; Mur targets).
+__global__ void k_mat_clear(uint32_t* mat, size_t n) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) mat[i] &= MAT_MASK;
+}
+__global__ void k_mat_box(uint32_t* mat, uint32_t Ny, uint32_t Pz, uint32_t sx, uint32_t sy, uint32_t sz, uint32_t ny, uint32_t nz,
+                          uint32_t cells) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= cells) return;
+    const uint32_t z = i % nz, r = i / nz, y = r % ny, x = r / ny;
+    atomicOr(mat + ((size_t)(sx + x) * Ny + sy + y) * Pz + sz + z, 7u << MAT_BITS);
+}
+
+// Mur ABC ahead of the core update (src/webgpu-fdtd.mjs:992-1023).  An entry's
+// pre, post and apply steps need E_old at its two cells and E_new at the
+// shifted one, which follows from the old fields, so one kernel before the core
+// update computes the entry's value, writes it over E_old at the target (dead
+// after the step) and the core update adopts it there: one pass over the
+// entries instead of three, and no H next to a Mur face is computed twice.
+//
+// Entries whose target no other entry reads or writes run one per thread; the
+// others in groups of lanes of one warp, which all read before any writes.
+// The plan keeps entries out that anything else comes between (UPML cells,
+// TFSF, periodic copies, an excitation on the target): k_mur_pre/post/apply.
+//
+// Bound by the sectors and latency of scattered points.  32 stub filters
+// batched (4.7 M entries): 104 us a step, where the three passes took 161 us
+// and the H cells next to the faces, updated again, another 122 us; 81^3 with
+// six faces: 17.1 -> 13.6 us a step.
+constexpr uint32_t MUR_SINGLE = 1u, MUR_LAST = 2u;   // one per thread; writes its target (the last entry that does)
+constexpr uint32_t MUR_GROUP = 8u;                   // most entries of a group
+struct MurAdoptDev {
+    uint32_t n, first, nslots;                       // entries; first group slot (n rounded up to a warp); group slots
+    const uint32_t* target; const uint32_t* shifted; const float* coeff;   // per entry, by target
+    const uint8_t* kind;                             // MUR_SINGLE, MUR_LAST
+    const uint32_t* slot;                            // entry of a group slot (~0: none); a group's slots lie in one warp
+    float* saved;
+};
+template <bool IDX>
+__device__ __forceinline__ float mur_value(const FusedGrid& g, const float* V, const MurAdoptDev& d, uint32_t i) {
+    const uint32_t N = (uint32_t)g.N, NyNz = (uint32_t)g.NyNz, Pz = g.Pz;
+    const uint32_t t = d.target[i], s = d.shifted[i];
+    const float c = d.coeff[i], vt = V[t], vs = V[s];
+    const uint32_t n = s / N, cell = s - n * N, x = cell / NyNz, r = cell - x * NyNz, y = r / Pz, z = r - y * Pz;
+    const uint32_t p = n == 2 ? 0u : n + 1u, q = p == 2 ? 0u : p + 1u;       // E_n: H_q along p, H_p along q
+    const uint32_t dp = p == 0 ? (x ? NyNz : 0u) : p == 1 ? (y ? Pz : 0u) : (z ? 1u : 0u);   // self at index 0
+    const uint32_t dq = q == 0 ? (x ? NyNz : 0u) : q == 1 ? (y ? Pz : 0u) : (z ? 1u : 0u);
+    const float *Hq = g.H0 + q * N + cell, *Hp = g.H0 + p * N + cell;
+    const float curl = curl4(Hq[0], *(Hq - dp), Hp[0], *(Hp - dq));
+    float cv, ci;
+    if (IDX) {
+        const float* row = g.table + (size_t)(g.mat[cell] & MAT_MASK) * 12;
+        cv = __ldg(row + n);
+        ci = __ldg(row + 3 + n);
+    } else {
+        cv = __ldg(g.vv + s);
+        ci = __ldg(g.vi + s);
+    }
+    return __fadd_rn(__fsub_rn(vs, __fmul_rn(c, vt)), __fmul_rn(c, upd(vs, cv, ci, curl)));
+}
+template <bool IDX>
+__device__ __forceinline__ void mur_adopt_body(const FusedGrid& g, float* V, const MurAdoptDev& d, uint32_t i) {
+    const bool grouped = i >= d.first;               // uniform in a warp
+    uint32_t e = i;
+    if (grouped) e = i - d.first < d.nslots ? d.slot[i - d.first] : ~0u;
+    const bool live = e < d.n;
+    const uint32_t kind = live ? d.kind[e] : 0u;
+    float v = 0.f;
+    if (live) v = mur_value<IDX>(g, V, d, e);        // also of entries left to the three passes: their loads are in flight with `kind`
+    if (grouped) __syncwarp();
+    if (!live || !(grouped || kind & MUR_SINGLE)) return;
+    d.saved[e] = v;
+    if (kind & MUR_LAST) V[d.target[e]] = v;
+}
+template <bool IDX>
+__global__ void __launch_bounds__(256) k_mur_adopt(const FusedGrid g, float* V, const MurAdoptDev d) {
+    mur_adopt_body<IDX>(g, V, d, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void k_mat_mur(uint32_t* mat, uint32_t N, const MurAdoptDev d) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < d.n && d.kind[i] & MUR_LAST) atomicOr(mat + d.target[i] % N, 1u << (MAT_BITS + d.target[i] / N));
 }
 
 // H update of the deferred cells, after the E-side sparse operations: reads

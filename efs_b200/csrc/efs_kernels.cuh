@@ -136,6 +136,7 @@ __device__ __forceinline__ float read_loc(const float* F, const float* const* fl
 // Mur ABC (src/webgpu-fdtd.mjs:992-1023)
 struct MurDev {
     uint32_t n, napply;
+    const uint32_t* ids;           // the entries of these passes
     const float* coeff;
     const ReadLoc* pre_normal;     // reads after the UPML pre swap
     const ReadLoc* pre_shifted;
@@ -147,12 +148,14 @@ struct MurDev {
 };
 __device__ __forceinline__ void mur_pre_body(const float* __restrict__ V, const MurDev& m, uint32_t i) {
     if (i >= m.n) return;
+    i = m.ids[i];
     float s = read_loc(V, m.vflux, m.pre_shifted[i]);
     float nv = read_loc(V, m.vflux, m.pre_normal[i]);
     m.saved[i] = __fsub_rn(s, __fmul_rn(m.coeff[i], nv));
 }
 __device__ __forceinline__ void mur_post_body(const float* __restrict__ V, const MurDev& m, uint32_t i) {
     if (i >= m.n) return;
+    i = m.ids[i];
     m.saved[i] = __fadd_rn(m.saved[i], __fmul_rn(m.coeff[i], V[m.shifted[i]]));
 }
 __device__ __forceinline__ void mur_apply_body(float* __restrict__ V, const MurDev& m, uint32_t i) {

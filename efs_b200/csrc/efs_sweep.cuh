@@ -97,7 +97,7 @@ __device__ __forceinline__ void sweep_e_body(const FusedGrid& g, const PmlSet& p
     const uint32_t dx = q.x > 0 ? NyNz : 0u, dy = q.y > 0 ? Pz : 0u, dz = q.z > 0 ? 1u : 0u;   // self at index 0
     const float *H = g.H0, *V = g.V0;
     uint2 m = make_uint2(0u, 0u);
-    if (IDX) m = __ldg(reinterpret_cast<const uint2*>(g.mat + c));
+    if (IDX || g.mat) m = __ldg(reinterpret_cast<const uint2*>(g.mat + c));
     const f32x2 hx = ldg2(H + c), hy = ldg2(H + N + c), hz = ldg2(H + 2 * N + c);
     const f32x2 hzy = ldg2(H + 2 * N + c - dy), hxy = ldg2(H + c - dy);
     const f32x2 hzx = ldg2(H + 2 * N + c - dx), hyx = ldg2(H + N + c - dx);
@@ -113,6 +113,13 @@ __device__ __forceinline__ void sweep_e_body(const FusedGrid& g, const PmlSet& p
     f32x2 en[3];
 #pragma unroll
     for (int n = 0; n < 3; ++n) en[n] = upd_2(eo[n], k.v[n], k.i[n], curl[n], g.nz);
+    if ((m.x | m.y) >> MAT_BITS) {                        // Mur targets (UPML cells are updated here)
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+            const f32x2 ad = adopt_mask(m, n);
+            en[n] = (en[n] & ~ad) | (eo[n] & ad);
+        }
+    }
     if (PML && (m0 | m1)) sweep_pair_upml<true>(ps, pn, q, m0, m1, true, true, k, curl, eo, en);
     sweep_store(g.V1, N, c, q.both, en);
 }

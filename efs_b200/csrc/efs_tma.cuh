@@ -20,9 +20,10 @@
 // E_new(x-1), which the interval before left in the other of two plane
 // buffers, and the thread's own E_new(x).
 //
-// UPML cells are updated by k_pml_e (E, before this kernel: its E_new is
-// staged here in place of E_old and adopted as is) and k_pml_h (H, after it);
-// this kernel only needs to know which cells they are.
+// E values known before this kernel (UPML cells by k_pml_e, Mur targets by
+// k_mur_adopt) are staged in place of E_old and adopted as is where the
+// material index says so.  H of UPML cells is provisional here and rewritten
+// by k_pml_h.
 //
 // Boundaries follow the reference's index-0 self reference: the x-1, y-1 and
 // z-1 neighbours of index 0 are the cell itself (the TMA zero fill outside
@@ -140,15 +141,14 @@ struct TmaMaps { const CUtensorMap *H, *E, *M, *D, *E1, *H1; };
 
 // Issue the loads of plane x into stage s (one thread); dbytes > 0: also the
 // plane's TFSF face corrections (rows y0 .. y0+TF_DY-1 of every face).
-template <bool IDX>
-__device__ __forceinline__ void tt_issue(TmaSmem& S, uint32_t s, const TmaMaps& tm, uint32_t dbytes, int x, int y0, int z0) {
+__device__ __forceinline__ void tt_issue(TmaSmem& S, uint32_t s, const TmaMaps& tm, bool mats, uint32_t dbytes, int x, int y0, int z0) {
     const uint32_t bar = smem_u32(&S.full[s]);
-    const uint32_t bytes = TT_H_BYTES + TT_E_BYTES + (IDX ? TT_M_BYTES : 0u) + dbytes;
+    const uint32_t bytes = TT_H_BYTES + TT_E_BYTES + (mats ? TT_M_BYTES : 0u) + dbytes;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // earlier generic reads of the stage before the refill
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
     tma_load_4d(&S.st[s].H[0][0][0], tm.H, z0 - 4, y0 - 1, x, 0, bar);
     tma_load_4d(&S.st[s].E[0][0][0], tm.E, z0, y0, x, 0, bar);
-    if (IDX) tma_load_3d(&S.st[s].M[0][0], tm.M, z0, y0, x, bar);
+    if (mats) tma_load_3d(&S.st[s].M[0][0], tm.M, z0, y0, x, bar);
     if (dbytes) tma_load_4d(&S.st[s].D[0][0][0], tm.D, y0, x, 0, 0, bar);
 }
 
@@ -224,8 +224,8 @@ __device__ __forceinline__ f32x2 pick2(f32x2 a, f32x2 b, uint32_t m) {
 struct PairCoef { f32x2 v[3], i[3]; };
 template <int BASE>
 __device__ __forceinline__ PairCoef pair_rows(const float* table, uint2 m) {
-    const float4* t0 = reinterpret_cast<const float4*>(table) + (size_t)m.x * 3 + (BASE ? 1 : 0);
-    const float4* t1 = reinterpret_cast<const float4*>(table) + (size_t)m.y * 3 + (BASE ? 1 : 0);
+    const float4* t0 = reinterpret_cast<const float4*>(table) + (size_t)(m.x & MAT_MASK) * 3 + (BASE ? 1 : 0);
+    const float4* t1 = reinterpret_cast<const float4*>(table) + (size_t)(m.y & MAT_MASK) * 3 + (BASE ? 1 : 0);
     const float4 a0 = __ldg(t0), b0 = __ldg(t0 + 1), a1 = __ldg(t1), b1 = __ldg(t1 + 1);
     PairCoef k;
     if (BASE == 0) {
@@ -236,6 +236,11 @@ __device__ __forceinline__ PairCoef pair_rows(const float* table, uint2 m) {
         k.i[0] = pk2(b0.y, b1.y); k.i[1] = pk2(b0.z, b1.z); k.i[2] = pk2(b0.w, b1.w);
     }
     return k;
+}
+// All ones in the halves of a pair (material indices m) whose component n is adopted.
+__device__ __forceinline__ f32x2 adopt_mask(uint2 m, int n) {
+    const uint32_t lo = 0u - (m.x >> (MAT_BITS + n) & 1u), hi = 0u - (m.y >> (MAT_BITS + n) & 1u);
+    return (f32x2)hi << 32 | lo;
 }
 // Dense coefficients of the pair at cell c (component stride N); zero for a
 // pair outside the grid.  Pad cells of a padded row hold zeros.
@@ -255,8 +260,8 @@ __device__ __forceinline__ PairCoef pair_dense(const float* v, const float* i, s
 // before it returns; its last stores may still be reading shared memory (the
 // next plane's barrier, or tt_done, waits for them).  Returns false after a
 // wait ran out.
-// PML, TF: the tile may meet a UPML region, a TFSF face corrected here; the
-// single engine tests the second per tile (tma_tile), the batch sorts its tiles.
+// TF: the tile may meet a TFSF face corrected here (the single engine tests it
+// per tile, tma_tile; the batch sorts its tiles).
 //
 // Warp r < TT_Y owns tile row r, lane l the cells z0+2l and z0+2l+1.  Two more
 // warps compute the E_new that their H needs beyond the tile and run the
@@ -270,8 +275,8 @@ __device__ __forceinline__ PairCoef pair_dense(const float* v, const float* i, s
 // A pair's coefficients stay in registers while its material does not change
 // along x.
 //
-template <bool IDX, bool PML, bool TF>
-__device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, const FusedGrid& g, const PmlSet& ps, uint32_t xs,
+template <bool IDX, bool TF>
+__device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, const FusedGrid& g, uint32_t xs,
                                               uint32_t y0, uint32_t z0, TmaRing& rg) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t xe = min(xs + g.xchunk, g.Nx);
@@ -286,14 +291,7 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
     bool tf_tile = false;
     if (TF)
         for (uint32_t f = 0; f < g.tf.n; ++f) tf_tile |= g.tf.z[f] >= z0 && g.tf.z[f] <= z0 + TT_Z;
-    // UPML: regions meeting the CTA's box, and those of them that not every plane meets
-    uint32_t cand = 0, xvar = 0;
-    if (PML) {
-        const uint32_t lo[3] = {xs, y0, z0};
-        const uint32_t hb[3] = {xe, y0 + TT_Y, z0 + TT_Z};
-        cand = region_mask(ps, lo, hb);
-        if (cand) xvar = cand & ~(axis_mask(ps, cand, 0, xs) & axis_mask(ps, cand, 0, xl));
-    }
+    const bool mats = IDX || g.mat;                          // the material index is staged
 
     if (warp == TT_Y + 1) {
         // ---- halo column: Ex and Ey of the cell (y0 + lane, z0 + TT_Z); stores
@@ -301,7 +299,6 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
         const bool has = lane < TT_Y, in = has && y < Ny && z < Nz;
         const int hi = (lane + 1) * TT_HZ + TT_Z + 4, ei = lane * TT_EZ + TT_Z, hy_ = hi - (y == 0 ? 0 : TT_HZ);
         const size_t off = (size_t)y * Pz + z;
-        const uint32_t yz = cand && has ? axis_mask(ps, cand, 1, y) & axis_mask(ps, cand, 2, z) : 0u;
         const int tf = tf_tile && has ? tf_face(g.tf, z) : -1;
         float hp = in ? __ldg(g.H0 + (size_t)(xs > 0 ? xs - 1 : 0) * NyNz + 2 * N + off) : 0.f;   // Hz(x-1)
         float kc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};        // dense coefficients, loaded a plane ahead
@@ -319,11 +316,13 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
                 const TmaStage& st = S.st[rg.s];
                 const float* Hs = &st.H[0][0][0];
                 const float* Es = &st.E[0][0][0];
-                if (IDX) coeffs_f<true>(g, 0, (&st.M[0][0])[ei], 0, kc);
+                const uint32_t m = mats ? (&st.M[0][0])[ei] : 0u;
+                if (IDX) coeffs_f<true>(g, 0, m, 0, kc);
                 const float hz = Hs[2 * HPL + hi], ex0 = Es[ei], ey0 = Es[EPL + ei];
                 float ex = upd(ex0, kc[0], kc[3], curl4(hz, Hs[2 * HPL + hy_], Hs[HPL + hi], Hs[HPL + hi - 1]));
                 float ey = upd(ey0, kc[1], kc[4], curl4(Hs[hi], Hs[hi - 1], hz, hp));
-                if (PML && yz && (yz & (~xvar | axis_mask(ps, xvar, 0, xs + k)))) { ex = ex0; ey = ey0; }
+                if (m >> MAT_BITS & 1u) ex = ex0;            // adopted
+                if (m >> MAT_BITS & 2u) ey = ey0;
                 if (tf >= 0) { ex = __fadd_rn(ex, st.D[tf][0][lane]); ey = __fadd_rn(ey, st.D[tf][1][lane]); }
                 S.En[rg.b][TT_ECOL + lane] = ex;
                 S.En[rg.b][TT_ECOL + TT_EC + lane] = ey;
@@ -358,13 +357,6 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
     const int si = own ? warp * TT_Z + 2 * lane : TT_EROW + 2 * lane;   // index in an E_new / H_new plane
     const int sy_ = warp == TT_Y - 1 ? TT_EROW + 2 * lane : si + TT_Z;  // its y+1 neighbour
     const int sz_ = lane == 31 ? TT_ECOL + warp : si + 2;    // z+1 neighbour of the second cell
-    uint32_t yz0 = 0, yz1 = 0, up = 0;                       // regions of each cell's (y, z); UPML cells of the pair
-    if (PML && cand) {
-        const uint32_t ym = axis_mask(ps, cand, 1, y);
-        yz0 = ym & axis_mask(ps, cand, 2, z);
-        yz1 = ym & axis_mask(ps, cand, 2, z + 1);
-        up = (yz0 & ~xvar ? 1u : 0u) | (yz1 & ~xvar ? 2u : 0u);
-    }
     int tf0 = -1, tf1 = -1;
     if (tf_tile) {
         tf0 = tf_face(g.tf, z);
@@ -378,7 +370,7 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
     if (loader)
         for (; issued < TT_S && issued < nk; ++issued)
             if (xs + issued != g.skip_plane)
-                tt_issue<IDX>(S, (rg.s + issued) % TT_S, tm, dbytes, (int)(xs + issued), (int)y0, (int)z0);
+                tt_issue(S, (rg.s + issued) % TT_S, tm, mats, dbytes, (int)(xs + issued), (int)y0, (int)z0);
 
     // H_old(xs-1) of the pair; at xs = 0 the x-1 neighbour is plane 0 itself
     const size_t off = (size_t)y * Pz + z;                   // offset inside a plane
@@ -393,6 +385,7 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
     PairCoef ke, kh;                                         // E coefficients of plane x, H coefficients of plane x-1
     uint2 mp = make_uint2(0u, 0u);                           // material of the pair at x-1
     bool chg = false;                                        // it changed from plane x-2 to x-1
+    f32x2 ad[3] = {0ull, 0ull, 0ull};                        // the pair's adopted components, as bit masks
     if (!IDX) ke = pair_dense(g.vv, g.vi, N, cell, in);
     bool timed_out = false;
     int k = 0;
@@ -408,25 +401,25 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
             const float* Ep = S.En[rg.b ^ 1u];
             f32x2 hc[3], en[3];
             // ---- E_new(x) of the pair
-            if (IDX) {
+            if (mats) {
                 const uint2 mc = *reinterpret_cast<const uint2*>(&st.M[0][0] + ei);
                 chg = k == 0 || mc.x != mp.x || mc.y != mp.y;
-                if (chg) { ke = pair_rows<0>(g.table, mc); mp = mc; }
+                if (chg) {
+                    if (IDX) ke = pair_rows<0>(g.table, mc);
+#pragma unroll
+                    for (int n = 0; n < 3; ++n) ad[n] = adopt_mask(mc, n);
+                    mp = mc;
+                }
             }
             hc[0] = ld2(Hs + hi); hc[1] = ld2(Hs + HPL + hi); hc[2] = ld2(Hs + 2 * HPL + hi);
             const f32x2 hzy = ld2(Hs + 2 * HPL + hy_), hxy = ld2(Hs + hy_);
             const f32x2 hyz = pk2(Hs[HPL + hz_], lo2(hc[1])), hxz = pk2(Hs[hz_], lo2(hc[0]));
-            const f32x2 eo0 = ld2(Es + ei), eo1 = ld2(Es + EPL + ei), eo2 = ld2(Es + 2 * EPL + ei);
-            en[0] = upd_2(eo0, ke.v[0], ke.i[0], curl4_2(hc[2], hzy, hc[1], hyz), nz);
-            en[1] = upd_2(eo1, ke.v[1], ke.i[1], curl4_2(hc[0], hxz, hc[2], hp[2]), nz);
-            en[2] = upd_2(eo2, ke.v[2], ke.i[2], curl4_2(hc[1], hp[1], hc[0], hxy), nz);
-            if (PML && cand) {           // a UPML cell's E_new was computed by k_pml_e and staged in place of E_old
-                if (xvar) {
-                    const uint32_t xm = ~xvar | axis_mask(ps, xvar, 0, xs + k);
-                    up = (yz0 & xm ? 1u : 0u) | (yz1 & xm ? 2u : 0u);
-                }
-                if (up) { en[0] = pick2(en[0], eo0, up); en[1] = pick2(en[1], eo1, up); en[2] = pick2(en[2], eo2, up); }
-            }
+            const f32x2 eo[3] = {ld2(Es + ei), ld2(Es + EPL + ei), ld2(Es + 2 * EPL + ei)};
+            en[0] = upd_2(eo[0], ke.v[0], ke.i[0], curl4_2(hc[2], hzy, hc[1], hyz), nz);
+            en[1] = upd_2(eo[1], ke.v[1], ke.i[1], curl4_2(hc[0], hxz, hc[2], hp[2]), nz);
+            en[2] = upd_2(eo[2], ke.v[2], ke.i[2], curl4_2(hc[1], hp[1], hc[0], hxy), nz);
+#pragma unroll
+            for (int n = 0; n < 3; ++n) en[n] = (en[n] & ~ad[n]) | (eo[n] & ad[n]);
             if (tf_tile) {               // the TFSF point pass's add, here
                 if (tf0 >= 0) {
                     en[0] = pk2(__fadd_rn(lo2(en[0]), st.D[tf0][0][warp]), hi2(en[0]));
@@ -456,7 +449,7 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
                 }
             } else if (loader && k > 0 && issued < nk) {
                 if (xs + issued != g.skip_plane)             // plane k-1+TT_S into the stage of plane k-1
-                    tt_issue<IDX>(S, (rg.s + TT_S - 1) % TT_S, tm, dbytes, (int)(xs + issued), (int)y0, (int)z0);
+                    tt_issue(S, (rg.s + TT_S - 1) % TT_S, tm, mats, dbytes, (int)(xs + issued), (int)y0, (int)z0);
                 ++issued;
             }
             if (!IDX) {                  // the next plane's E coefficients and this plane's H coefficients
@@ -501,13 +494,12 @@ __device__ __forceinline__ void tt_done() {
     if (threadIdx.x == 32 * (TT_Y + 1)) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 // A TFSF face corrected in the core update meets the tile's columns (halo column included).
-template <bool IDX, bool PML>
-__device__ __forceinline__ bool tma_tile(TmaSmem& S, const TmaMaps& tm, const FusedGrid& g, const PmlSet& ps, uint32_t xs,
-                                         uint32_t y0, uint32_t z0, TmaRing& rg) {
+template <bool IDX>
+__device__ __forceinline__ bool tma_tile(TmaSmem& S, const TmaMaps& tm, const FusedGrid& g, uint32_t xs, uint32_t y0, uint32_t z0,
+                                         TmaRing& rg) {
     bool tf = false;
     for (uint32_t f = 0; f < g.tf.n; ++f) tf |= g.tf.z[f] >= z0 && g.tf.z[f] <= z0 + TT_Z;
-    return tf ? tma_tile_body<IDX, PML, true>(S, tm, g, ps, xs, y0, z0, rg)
-              : tma_tile_body<IDX, PML, false>(S, tm, g, ps, xs, y0, z0, rg);
+    return tf ? tma_tile_body<IDX, true>(S, tm, g, xs, y0, z0, rg) : tma_tile_body<IDX, false>(S, tm, g, xs, y0, z0, rg);
 }
 
 // Bound by DRAM on large grids (512^3: 1.114 ms a launch at 24 planes per CTA
@@ -520,18 +512,17 @@ __device__ __forceinline__ bool tma_tile(TmaSmem& S, const TmaMaps& tm, const Fu
 // registers: same time at 512^3, 4% slower at 256^3), loops unrolled 2 or 4
 // planes deep (slower: instruction fetch), TMA boxes without halo columns
 // (no change).
-template <bool IDX, bool PML>
+template <bool IDX>
 __global__ void __launch_bounds__(TT_THREADS, 2)
 k_fused_tma(const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmE,
             const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmD,
-            const __grid_constant__ CUtensorMap tmE1, const __grid_constant__ CUtensorMap tmH1, const FusedGrid g,
-            const PmlSet ps) {
+            const __grid_constant__ CUtensorMap tmE1, const __grid_constant__ CUtensorMap tmH1, const FusedGrid g) {
     const uint32_t xs = blockIdx.z * g.xchunk;
     if (xs >= g.Nx) return;                                  // uniform per CTA
     TmaSmem& S = tt_smem();
     tt_init(S);
     TmaRing rg;
-    (void)tma_tile<IDX, PML>(S, TmaMaps{&tmH, &tmE, &tmM, &tmD, &tmE1, &tmH1}, g, ps, xs, blockIdx.y * TT_Y, blockIdx.x * TT_Z, rg);
+    (void)tma_tile<IDX>(S, TmaMaps{&tmH, &tmE, &tmM, &tmD, &tmE1, &tmH1}, g, xs, blockIdx.y * TT_Y, blockIdx.x * TT_Z, rg);
     tt_done();
 }
 
