@@ -53,6 +53,9 @@ using namespace efs;
 
 namespace {
 
+// Far field: a launch's angles, its blocks (148 SMs x 2 x 6 waves), the workspace an engine keeps between calls.
+constexpr uint32_t FF_SLAB = 1u << 18, FF_BLOCKS = 1776;
+constexpr size_t FF_KEEP = (size_t)64 << 20;
 constexpr size_t SWEEP_BYTES = (size_t)92 << 20;   // fields and material index of the largest grid that runs as sweeps
 
 thread_local std::string g_create_error = "no error";
@@ -320,6 +323,8 @@ struct efs_engine {
     DevBuf nf_pts, nf_el, nf_E, nf_H, nf_samp;
     Nf2ffDev nf{};
     float ff_ms[2] = {0.f, 0.f};     // device time of the last far-field call: point records, angle sums
+    DevBuf ff_ws;                    // far-field workspace, kept up to FF_KEEP bytes
+    cudaEvent_t ff_event[3] = {nullptr, nullptr, nullptr};
 
     // energy (lagged, double-buffered like computeEnergy :2974-3021)
     DevBuf en_partial, en_result;
@@ -341,6 +346,7 @@ struct efs_engine {
     ~efs_engine() {
         drop_graphs();
         for (auto& ev : en_event) if (ev) cudaEventDestroy(ev);
+        for (auto& ev : ff_event) if (ev) cudaEventDestroy(ev);
         host_slot_put(slot);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -1974,52 +1980,79 @@ efs_status efs_far_field(efs_engine* e, uint32_t fi, const float* meta, const fl
         const uint64_t A64 = (uint64_t)nth * nph;
         if (A64 >= (1ull << 31)) fail(EFS_ERR_RANGE, "too many far-field angles");
         const uint32_t A = (uint32_t)A64;
-        // points grouped by the normal axis of their face (counting sort, stable)
-        std::vector<uint32_t> perm(np);
+        // points grouped by the normal axis of their face (counting sort, stable);
+        // a caller's list that is already in that order needs no permutation
+        std::vector<uint32_t> perm;
         FarFieldDev d;
         memset(&d, 0, sizeof(d));
         {
             uint32_t cnt[4] = {0, 0, 0, 0};
+            bool ordered = true;
+            float last = 0.f;
             for (uint32_t p = 0; p < np; ++p) {
                 const float nd = meta[8 * (size_t)p + 3];
                 if (!(nd == 0.f || nd == 1.f || nd == 2.f)) fail(EFS_ERR_INVALID, "pointMeta normal direction must be 0, 1 or 2");
                 ++cnt[(int)nd + 1];
+                ordered = ordered && nd >= last;
+                last = nd;
             }
             for (int n = 0; n < 3; ++n) cnt[n + 1] += cnt[n];
             for (int n = 0; n < 4; ++n) d.seg[n] = cnt[n];
-            for (uint32_t p = 0; p < np; ++p) perm[cnt[(int)meta[8 * (size_t)p + 3]]++] = p;
+            if (!ordered) {
+                perm.resize(np);
+                for (uint32_t p = 0; p < np; ++p) perm[cnt[(int)meta[8 * (size_t)p + 3]]++] = p;
+            }
         }
-        DevBuf dm, dperm, drec, dth, dph, dout;
-        e->upload(dm, meta, 8 * (size_t)np);
-        e->upload(dperm, perm);
-        e->upload(dth, theta, nth);
-        e->upload(dph, phi, nph);
-        e->alloc(drec, (size_t)np * sizeof(FfRecord), false);
-        e->alloc(dout, (size_t)A * 5 * 4, false);
+        // angles in slabs (bounds the scratch), records in chunks: about FF_BLOCKS blocks a launch
+        const uint32_t slab = std::min<uint32_t>(A, FF_SLAB), ab = blocks(slab, FF_ANG);
+        const uint64_t tiles = (uint64_t)blocks(np, FF_TILE) * ab;
+        d.chunk = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, (tiles + FF_BLOCKS - 1) / FF_BLOCKS), blocks(np, FF_TILE)) * FF_TILE;
+        d.nchunks = 0;
+        for (int n = 0; n < 3; ++n) d.nchunks += blocks(d.seg[n + 1] - d.seg[n], d.chunk);
+        // one workspace: meta, perm, theta, phi, records, partial sums, result
+        size_t at = 0;
+        auto room = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~(size_t)255; return o; };
+        const size_t om = room(32 * (size_t)np), op = room(4 * perm.size()), ot = room(4 * (size_t)nth), oph = room(4 * (size_t)nph),
+                     orec = room(np * sizeof(FfRecord)), opart = room((size_t)d.nchunks * 64 * slab), oout = room((size_t)A * 20);
+        DevBuf once, &ws = at <= FF_KEEP ? e->ff_ws : once;
+        if (ws.bytes < at) e->alloc(ws, at, false);
+        uint8_t* w = ws.as<uint8_t>();
+        auto put = [&](size_t o, const void* src, size_t bytes) {
+            if (bytes) ck(cudaMemcpyAsync(w + o, src, bytes, cudaMemcpyHostToDevice, e->stream), "far-field upload");
+        };
+        put(om, meta, 32 * (size_t)np);
+        put(op, perm.data(), 4 * perm.size());
+        put(ot, theta, 4 * (size_t)nth);
+        put(oph, phi, 4 * (size_t)nph);
         const double C0 = 299792458.0;
         const double k = 2 * M_PI * freq / C0;
         const double fmag = k / (4 * M_PI * radius), fph = -k * radius;   // (:2880-2884)
-        d.np = np; d.nth = nth; d.nph = nph;
-        d.rec = drec.as<FfRecord>();
-        d.theta = dth.as<float>(); d.phi = dph.as<float>();
+        d.nth = nth; d.nph = nph;
+        d.rec = reinterpret_cast<FfRecord*>(w + orec);
+        d.theta = reinterpret_cast<float*>(w + ot); d.phi = reinterpret_cast<float*>(w + oph);
+        d.part = reinterpret_cast<double*>(w + opart);
         d.fre = fmag * (-std::sin(fph)); d.fim = fmag * std::cos(fph);
-        d.out = dout.as<float>();
-        cudaEvent_t ev[3];
-        for (auto& x : ev) ck(cudaEventCreate(&x), "event");
-        ck(cudaEventRecord(ev[0], e->stream), "record");
-        k_ff_prep<<<blocks(np, 256), 256, 0, e->stream>>>(dm.as<float>(), e->nf_E.as<float>() + (size_t)fi * np * 6,
-                                                          e->nf_H.as<float>() + (size_t)fi * np * 6, dperm.as<uint32_t>(), np,
+        d.out = reinterpret_cast<float*>(w + oout);
+        for (auto& x : e->ff_event)
+            if (!x) ck(cudaEventCreate(&x), "event");
+        ck(cudaEventRecord(e->ff_event[0], e->stream), "record");
+        k_ff_prep<<<blocks(np, 256), 256, 0, e->stream>>>(reinterpret_cast<float*>(w + om), e->nf_E.as<float>() + (size_t)fi * np * 6,
+                                                          e->nf_H.as<float>() + (size_t)fi * np * 6,
+                                                          perm.empty() ? nullptr : reinterpret_cast<uint32_t*>(w + op), np,
                                                           (float)(k / (2 * M_PI)), (float)center[0], (float)center[1],
-                                                          (float)center[2], drec.as<FfRecord>());
-        ck(cudaEventRecord(ev[1], e->stream), "record");
-        k_ff_angles<<<blocks(A, FF_ANG), FF_THREADS, 0, e->stream>>>(d);
-        ck(cudaEventRecord(ev[2], e->stream), "record");
+                                                          (float)center[2], reinterpret_cast<FfRecord*>(w + orec));
+        ck(cudaEventRecord(e->ff_event[1], e->stream), "record");
+        for (uint32_t a0 = 0; a0 < A; a0 += slab) {
+            d.a0 = a0; d.na = std::min(slab, A - a0);
+            k_ff_angles<<<dim3(blocks(d.na, FF_ANG), d.nchunks), FF_THREADS, 0, e->stream>>>(d);
+            k_ff_final<<<blocks(d.na, 256), 256, 0, e->stream>>>(d);
+        }
+        ck(cudaEventRecord(e->ff_event[2], e->stream), "record");
         ck(cudaGetLastError(), "far field");
-        ck(cudaMemcpyAsync(out, dout.p, (size_t)A * 5 * 4, cudaMemcpyDeviceToHost, e->stream), "read far field");
+        ck(cudaMemcpyAsync(out, d.out, (size_t)A * 20, cudaMemcpyDeviceToHost, e->stream), "read far field");
         e->sync("sync");
-        cudaEventElapsedTime(&e->ff_ms[0], ev[0], ev[1]);
-        cudaEventElapsedTime(&e->ff_ms[1], ev[1], ev[2]);
-        for (auto& x : ev) cudaEventDestroy(x);
+        cudaEventElapsedTime(&e->ff_ms[0], e->ff_event[0], e->ff_event[1]);
+        cudaEventElapsedTime(&e->ff_ms[1], e->ff_event[1], e->ff_event[2]);
     });
 }
 
@@ -2395,7 +2428,7 @@ efs_status efs_device_bytes(const efs_engine* e, size_t* out) {
         const DevBuf* rb[] = {&r->vv, &r->vvfo, &r->vvfn, &r->ii, &r->iifo, &r->iifn, &r->vflux, &r->cflux, &r->vflux_b, &r->cflux_b};
         for (auto* b : rb) t += b->bytes;
     }
-    t += e->nf_E.bytes + e->nf_H.bytes + e->nf_samp.bytes + e->ring.bytes;
+    t += e->nf_E.bytes + e->nf_H.bytes + e->nf_samp.bytes + e->ring.bytes + e->ff_ws.bytes;
     *out = t;
     return EFS_OK;
 }

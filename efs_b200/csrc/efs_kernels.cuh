@@ -737,39 +737,73 @@ __global__ void __launch_bounds__(256) k_energy_ranges(const float* __restrict__
 // with the surface currents J = n x H, M = -n x E of each point's face, then
 // E_theta, E_phi and the radiated intensity from the theta/phi projections.
 //
-// k_ff_prep turns every point into a 48-byte record: its position times
-// k / 2 pi (the phase comes out in turns) and the two tangential components
-// of area*J and area*M (a face with normal axis n carries currents along
-// a = n+1 and b = n+2 only), with the points ordered by normal axis (the
-// host passes the permutation).  k_ff_angles: a block takes FF_ANG angles; a
-// warp holds FF_ANG/8 angles x FF_PL point lanes; the block stages tiles of
-// records in shared memory and each thread sums its angle over every
-// FF_PL-th point of the tile in f32 (only the two tangential accumulators of
-// the segment's normal axis are live), adding the tile's sum into f64
-// accumulators; the FF_PL point lanes of an angle are combined with warp
-// shuffles and one lane forms the result in f64.  The phase is reduced to
-// [-1/2, 1/2] turns before the hardware sine/cosine (error ~2^-21 there).
+// k_ff_prep turns every point into a record: its position times k / 2 pi (the
+// phase comes out in turns) and the two tangential components of area*J and
+// area*M (a face with normal axis n carries currents along a = n+1 and b = n+2
+// only), with the points ordered by normal axis (the host passes the
+// permutation when the caller's order is another).
+//
+// k_ff_angles: a block takes FF_ANG angles and one chunk of the records of one
+// normal axis; a warp holds 32/FF_PL angle slots x FF_PL point lanes.  A thread
+// carries FF_AT angles through the records, two at a time as packed f32x2
+// values (phase, sine and cosine, and the eight sums of both): a 128-bit
+// shared-memory load takes four wavefronts for 32 lanes whatever they read, so
+// with one angle per thread the records' loads alone took as long as the
+// arithmetic does now.  The f32 sums of FF_TILE/FF_PL records go into f64
+// sums; the FF_PL point lanes are combined with warp shuffles and a chunk's
+// sums written to scratch.  k_ff_final adds the chunks and forms the
+// result in f64.  The phase is reduced to [-1/2, 1/2] turns before the hardware
+// sine/cosine (error ~2^-21 there) by adding and subtracting 1.5 * 2^23, which
+// rounds to the nearest integer in the adder: the round instruction shares
+// the special-function pipe with sine and cosine.
+//
+// Splitting the records over blocks is what a pattern of few angles needs
+// (61 x 73 angles filled 70 blocks, each with all points in series).
+//
+// Bound by the FMA pipe (70% active; 24 of its slots per angle and point).
+// Measured on B200, device time: 65,341 angles x 334,176 points 30.9 -> 20.5
+// ms, 4,453 angles x 22,410 points 0.34 -> 0.14 ms.
 // ---------------------------------------------------------------------------
-constexpr int FF_THREADS = 256;
-constexpr int FF_PL = 4;                                  // point lanes per angle (a shuffle group)
-constexpr int FF_ANG = FF_THREADS / FF_PL;                // angles per block
-constexpr int FF_TILE = 512;                              // records per shared-memory tile
+constexpr int FF_THREADS = 128;
+constexpr int FF_PL = 4;                                  // point lanes per angle slot (a shuffle group)
+constexpr int FF_AT = 4;                                  // angles per thread
+constexpr int FF_SLOTS = FF_THREADS / FF_PL;
+constexpr int FF_ANG = FF_AT * FF_SLOTS;                  // angles per block
+constexpr uint32_t FF_TILE = 256;                         // records per shared-memory tile
 struct FfRecord { float4 pos; float4 j; float4 m; };     // pos: x,y,z in turns (w unused); j, m: a_re a_im b_re b_im
 struct FarFieldDev {
-    uint32_t np, nth, nph;
+    uint32_t nth, nph;
     uint32_t seg[4];                                      // records of normal axis n: [seg[n], seg[n+1])
+    uint32_t chunk;                                       // records per chunk, a multiple of FF_TILE
+    uint32_t nchunks;                                     // of all three axes
+    uint32_t a0, na;                                      // angles of this launch
     const FfRecord* rec;
     const float* theta; const float* phi;
+    double* part;                                         // [chunk][8][na]: N_a, N_b, L_a, L_b (re, im)
     double fre, fim;                                      // k/(4 pi r) e^{-j k r} factor (re, im)
     float* out;                                           // 5 per angle
 };
-// One record per point, in the order perm (points grouped by normal axis).
+// Chunk c -> its normal axis and records [p0, p1).
+__host__ __device__ inline int ff_chunk(const FarFieldDev& d, uint32_t c, uint32_t& p0, uint32_t& p1) {
+    for (int n = 0; n < 3; ++n) {
+        const uint32_t len = d.seg[n + 1] - d.seg[n], k = (len + d.chunk - 1) / d.chunk;
+        if (c < k) {
+            p0 = d.seg[n] + c * d.chunk;
+            p1 = p0 + d.chunk < d.seg[n + 1] ? p0 + d.chunk : d.seg[n + 1];
+            return n;
+        }
+        c -= k;
+    }
+    p0 = p1 = 0;
+    return 2;
+}
+// One record per point, in the order perm (points grouped by normal axis; null: the caller's order).
 __global__ void k_ff_prep(const float* __restrict__ meta, const float* __restrict__ accE, const float* __restrict__ accH,
                           const uint32_t* __restrict__ perm, uint32_t np, float kx, float cx, float cy, float cz,
                           FfRecord* __restrict__ rec) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
-    const uint32_t p = perm[i];
+    const uint32_t p = perm ? perm[i] : i;
     const float* m = meta + 8 * (size_t)p;
     const float* E = accE + 6 * (size_t)p;
     const float* H = accH + 6 * (size_t)p;
@@ -783,78 +817,140 @@ __global__ void k_ff_prep(const float* __restrict__ meta, const float* __restric
     r.m = make_float4(s * E[2 * cb], s * E[2 * cb + 1], -s * E[2 * ca], -s * E[2 * ca + 1]);
     rec[i] = r;
 }
-// One (angle, point) pair: the record's tangential currents times e^{j 2 pi phase}
-// added into a (N_a, N_b, L_a, L_b as re, im).
-__device__ __forceinline__ void ff_pair(const FfRecord& r, float ux, float uy, float uz, float (&a)[8]) {
-    float ph = r.pos.x * ux;
-    ph = fmaf(r.pos.y, uy, ph);
-    ph = fmaf(r.pos.z, uz, ph);
-    ph -= rintf(ph);                                       // turns in [-1/2, 1/2]
-    float sn, cs;
-    __sincosf(6.2831853071795864f * ph, &sn, &cs);
-    a[0] = fmaf(r.j.x, cs, fmaf(-r.j.y, sn, a[0])); a[1] = fmaf(r.j.y, cs, fmaf(r.j.x, sn, a[1]));
-    a[2] = fmaf(r.j.z, cs, fmaf(-r.j.w, sn, a[2])); a[3] = fmaf(r.j.w, cs, fmaf(r.j.z, sn, a[3]));
-    a[4] = fmaf(r.m.x, cs, fmaf(-r.m.y, sn, a[4])); a[5] = fmaf(r.m.y, cs, fmaf(r.m.x, sn, a[5]));
-    a[6] = fmaf(r.m.z, cs, fmaf(-r.m.w, sn, a[6])); a[7] = fmaf(r.m.w, cs, fmaf(r.m.z, sn, a[7]));
+
+typedef unsigned long long ff_pair;                       // two packed f32: the thread's two angles
+__device__ __forceinline__ ff_pair ff_pk(float a, float b) {
+    ff_pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
 }
-// Records [p0, p1) of normal axis ND for this thread's angle (direction u).
-template <int ND>
-__device__ __forceinline__ void ff_segment(const FarFieldDev& d, FfRecord* tile, uint32_t p0, uint32_t p1, float ux, float uy,
-                                           float uz, int q, bool live, double acc[12]) {
-    constexpr int CA = (ND + 1) % 3, CB = (ND + 2) % 3;
+__device__ __forceinline__ ff_pair ff_fma(ff_pair a, ff_pair b, ff_pair c) {
+    ff_pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ ff_pair ff_mul(ff_pair a, ff_pair b) {
+    ff_pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ ff_pair ff_add(ff_pair a, ff_pair b) {
+    ff_pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ ff_pair ff_sub(ff_pair a, ff_pair b) {
+    ff_pair r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float ff_lo(ff_pair v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float ff_hi(ff_pair v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+// One record into the eight sums of two angles.
+__device__ __forceinline__ void ff_record(const ff_pair (&v)[11], ff_pair ux, ff_pair uy, ff_pair uz, ff_pair big, ff_pair turn,
+                                          ff_pair (&s)[8]) {
+    ff_pair ph = ff_fma(v[2], uz, ff_fma(v[1], uy, ff_mul(v[0], ux)));
+    ph = ff_mul(ff_sub(ph, ff_sub(ff_add(ph, big), big)), turn);              // radians in [-pi, pi]
+    float s0, c0, s1, c1;
+    __sincosf(ff_lo(ph), &s0, &c0);
+    __sincosf(ff_hi(ph), &s1, &c1);
+    const ff_pair cs = ff_pk(c0, c1), sn = ff_pk(s0, s1), ns = ff_pk(-s0, -s1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {                         // N_a, N_b, L_a, L_b: (re + j im) e^{j ph}
+        s[2 * i] = ff_fma(v[3 + 2 * i], cs, ff_fma(v[4 + 2 * i], ns, s[2 * i]));
+        s[2 * i + 1] = ff_fma(v[4 + 2 * i], cs, ff_fma(v[3 + 2 * i], sn, s[2 * i + 1]));
+    }
+}
+__global__ void __launch_bounds__(FF_THREADS, 3) k_ff_angles(const FarFieldDev d) {
+    __shared__ FfRecord tile[FF_TILE];
+    const int q = threadIdx.x % FF_PL;
+    const uint32_t l0 = blockIdx.x * FF_ANG + threadIdx.x / FF_PL;     // the thread's first angle in this launch; step FF_SLOTS
+    uint32_t p0, p1;
+    ff_chunk(d, blockIdx.y, p0, p1);
+    ff_pair ux[FF_AT / 2], uy[FF_AT / 2], uz[FF_AT / 2];
+#pragma unroll
+    for (int h = 0; h < FF_AT; h += 2) {
+        float u[2][3] = {{0.f, 0.f, 1.f}, {0.f, 0.f, 1.f}};
+        for (int k = 0; k < 2; ++k) {
+            const uint32_t l = l0 + (h + k) * FF_SLOTS;
+            if (l >= d.na) continue;
+            float sT, cT, sP, cP;
+            sincosf(d.theta[(d.a0 + l) / d.nph], &sT, &cT);
+            sincosf(d.phi[(d.a0 + l) % d.nph], &sP, &cP);
+            u[k][0] = sT * cP; u[k][1] = sT * sP; u[k][2] = cT;
+        }
+        ux[h / 2] = ff_pk(u[0][0], u[1][0]); uy[h / 2] = ff_pk(u[0][1], u[1][1]); uz[h / 2] = ff_pk(u[0][2], u[1][2]);
+    }
+    const ff_pair big = ff_pk(12582912.f, 12582912.f), turn = ff_pk(6.2831853071795864f, 6.2831853071795864f);
+    double acc[FF_AT][8];
+#pragma unroll
+    for (int h = 0; h < FF_AT; ++h)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[h][i] = 0.0;
     for (uint32_t t0 = p0; t0 < p1; t0 += FF_TILE) {
-        const uint32_t nt = min((uint32_t)FF_TILE, p1 - t0);
+        const uint32_t nt = min(FF_TILE, p1 - t0);
         __syncthreads();
         for (uint32_t j = threadIdx.x; j < nt; j += FF_THREADS) tile[j] = d.rec[t0 + j];
         __syncthreads();
-        if (!live) continue;
-        // four points per iteration into two sets of sums: their phases and
-        // sines / cosines are independent, so several are in flight per thread
-        float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // N_a, N_b, L_a, L_b (re, im)
-        float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        uint32_t j = q;
-        for (; j + 3 * FF_PL < nt; j += 4 * FF_PL) {
-            ff_pair(tile[j], ux, uy, uz, s);
-            ff_pair(tile[j + FF_PL], ux, uy, uz, t);
-            ff_pair(tile[j + 2 * FF_PL], ux, uy, uz, s);
-            ff_pair(tile[j + 3 * FF_PL], ux, uy, uz, t);
-        }
-        for (; j < nt; j += FF_PL) ff_pair(tile[j], ux, uy, uz, s);
+        ff_pair s[FF_AT / 2][8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s[i] += t[i];
-        acc[2 * CA] += s[0]; acc[2 * CA + 1] += s[1];
-        acc[2 * CB] += s[2]; acc[2 * CB + 1] += s[3];
-        acc[6 + 2 * CA] += s[4]; acc[6 + 2 * CA + 1] += s[5];
-        acc[6 + 2 * CB] += s[6]; acc[6 + 2 * CB + 1] += s[7];
+        for (int h = 0; h < FF_AT / 2; ++h)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s[h][i] = 0ull;
+        for (uint32_t j = q; j < nt; j += FF_PL) {
+            const FfRecord r = tile[j];
+            const ff_pair v[11] = {ff_pk(r.pos.x, r.pos.x), ff_pk(r.pos.y, r.pos.y), ff_pk(r.pos.z, r.pos.z),
+                                   ff_pk(r.j.x, r.j.x), ff_pk(r.j.y, r.j.y), ff_pk(r.j.z, r.j.z), ff_pk(r.j.w, r.j.w),
+                                   ff_pk(r.m.x, r.m.x), ff_pk(r.m.y, r.m.y), ff_pk(r.m.z, r.m.z), ff_pk(r.m.w, r.m.w)};
+#pragma unroll
+            for (int h = 0; h < FF_AT / 2; ++h) ff_record(v, ux[h], uy[h], uz[h], big, turn, s[h]);
+        }
+#pragma unroll
+        for (int h = 0; h < FF_AT / 2; ++h)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { acc[2 * h][i] += ff_lo(s[h][i]); acc[2 * h + 1][i] += ff_hi(s[h][i]); }
+    }
+    // the FF_PL point lanes of an angle slot are adjacent lanes of one warp
+    double* w = d.part + (size_t)blockIdx.y * 8 * d.na;
+#pragma unroll
+    for (int h = 0; h < FF_AT; ++h) {
+        const uint32_t l = l0 + h * FF_SLOTS;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            double v = acc[h][i];
+#pragma unroll
+            for (int o = 1; o < FF_PL; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (i % FF_PL == q && l < d.na) w[(size_t)i * d.na + l] = v;      // point lane q writes sums q and q + 4
+        }
     }
 }
-__global__ void __launch_bounds__(FF_THREADS) k_ff_angles(const FarFieldDev d) {
-    __shared__ FfRecord tile[FF_TILE];
-    const int lane = threadIdx.x & 31, q = lane % FF_PL;
-    const uint32_t A = d.nth * d.nph;
-    const uint32_t a = blockIdx.x * FF_ANG + threadIdx.x / FF_PL;
-    const bool live = a < A;
-    float sT = 0.f, cT = 1.f, sP = 0.f, cP = 1.f;
-    if (live) {
-        sincosf(d.theta[a / d.nph], &sT, &cT);
-        sincosf(d.phi[a % d.nph], &sP, &cP);
-    }
-    const float ux = sT * cP, uy = sT * sP, uz = cT;
+__global__ void __launch_bounds__(256) k_ff_final(const FarFieldDev d) {
+    const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (l >= d.na) return;
     double acc[12];                                      // N_x, N_y, N_z, L_x, L_y, L_z (re, im)
 #pragma unroll
     for (int i = 0; i < 12; ++i) acc[i] = 0.0;
-    ff_segment<0>(d, tile, d.seg[0], d.seg[1], ux, uy, uz, q, live, acc);
-    ff_segment<1>(d, tile, d.seg[1], d.seg[2], ux, uy, uz, q, live, acc);
-    ff_segment<2>(d, tile, d.seg[2], d.seg[3], ux, uy, uz, q, live, acc);
-    // the FF_PL point lanes of this angle are adjacent lanes of one warp
+    uint32_t c = 0;
 #pragma unroll
-    for (int i = 0; i < 12; ++i)
-#pragma unroll
-        for (int o = 1; o < FF_PL; o <<= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-    if (!live || q != 0) return;
+    for (int n = 0; n < 3; ++n) {
+        const int a = 2 * ((n + 1) % 3), b = 2 * ((n + 2) % 3);
+        const uint32_t end = c + (d.seg[n + 1] - d.seg[n] + d.chunk - 1) / d.chunk;
+        for (; c < end; ++c) {
+            const double* w = d.part + (size_t)c * 8 * d.na + l;
+            acc[a] += w[0]; acc[a + 1] += w[(size_t)d.na];
+            acc[b] += w[2 * (size_t)d.na]; acc[b + 1] += w[3 * (size_t)d.na];
+            acc[6 + a] += w[4 * (size_t)d.na]; acc[6 + a + 1] += w[5 * (size_t)d.na];
+            acc[6 + b] += w[6 * (size_t)d.na]; acc[6 + b + 1] += w[7 * (size_t)d.na];
+        }
+    }
+    const uint32_t an = d.a0 + l;
+    float sT, cT, sP, cP;
+    sincosf(d.theta[an / d.nph], &sT, &cT);
+    sincosf(d.phi[an % d.nph], &sP, &cP);
     const double cTcP = (double)cT * cP, cTsP = (double)cT * sP;
-    auto proj_t = [&](int b, int c) { return acc[b + c] * cTcP + acc[b + 2 + c] * cTsP - acc[b + 4 + c] * (double)sT; };
-    auto proj_p = [&](int b, int c) { return acc[b + 2 + c] * (double)cP - acc[b + c] * (double)sP; };
+    auto proj_t = [&](int b, int k) { return acc[b + k] * cTcP + acc[b + 2 + k] * cTsP - acc[b + 4 + k] * (double)sT; };
+    auto proj_p = [&](int b, int k) { return acc[b + 2 + k] * (double)cP - acc[b + k] * (double)sP; };
     const double Ntr = proj_t(0, 0), Nti = proj_t(0, 1), Npr = proj_p(0, 0), Npi = proj_p(0, 1);
     const double Ltr = proj_t(6, 0), Lti = proj_t(6, 1), Lpr = proj_p(6, 0), Lpi = proj_p(6, 1);
     const double Z0 = 376.73031346177066;
@@ -862,7 +958,7 @@ __global__ void __launch_bounds__(FF_THREADS) k_ff_angles(const FarFieldDev d) {
     const double Etr = -(d.fre * ar - d.fim * ai), Eti = -(d.fre * ai + d.fim * ar);
     const double br = Ltr - Z0 * Npr, bi = Lti - Z0 * Npi;
     const double Epr = d.fre * br - d.fim * bi, Epi = d.fre * bi + d.fim * br;
-    float* o = d.out + 5 * (size_t)a;
+    float* o = d.out + 5 * (size_t)an;
     o[0] = (float)((Etr * Etr + Eti * Eti + Epr * Epr + Epi * Epi) / (2 * Z0));
     o[1] = (float)Etr; o[2] = (float)Eti; o[3] = (float)Epr; o[4] = (float)Epi;
 }
