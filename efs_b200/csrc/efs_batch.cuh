@@ -39,6 +39,7 @@ struct BatchTile { uint32_t m, xs, y0, z0; };
 template <bool IDX, bool TF>
 __global__ void __launch_bounds__(TT_THREADS, 2)
 k_fused_tma_batch(const BatchMember* __restrict__ mem, const BatchTile* __restrict__ tiles, uint32_t ntiles) {
+    step_begin();
     TmaSmem& S = tt_smem();
     tt_init(S);
     TmaRing rg;                                        // pipeline state across the CTA's tiles
@@ -59,6 +60,7 @@ struct SegMap { const uint32_t* seg; const uint32_t* first; };
 
 template <class Op>
 __global__ void __launch_bounds__(256) k_seg(const Op* __restrict__ ops, SegMap sm, uint32_t k, uint32_t a, uint32_t b) {
+    step_begin();
     const uint32_t s = sm.seg[blockIdx.x];
     ops[s].run(blockIdx.x - sm.first[s], k, a, b);
 }
@@ -222,7 +224,7 @@ struct efs_batch {
     }
     template <class Op>
     void launch_seg(const SegLaunch& L, uint32_t k, uint32_t a = 0, uint32_t b = 0) {
-        if (L.blocks) k_seg<Op><<<L.blocks, SEG_T, 0, stream>>>(L.ops.as<Op>(), L.map(), k, a, b);
+        if (L.blocks) launch_k(false, k_seg<Op>, L.blocks, SEG_T, 0, stream, L.ops.as<Op>(), L.map(), k, a, b);
     }
 
     void check_members() {
@@ -260,7 +262,7 @@ struct efs_batch {
     template <bool IDX, bool TF>
     void launch_tiles(int t, const BatchMember* bm) {
         if (ntiles[t])
-            k_fused_tma_batch<IDX, TF><<<std::min<uint32_t>(ntiles[t], ctas_per_sm * sms), TT_THREADS, TT_SMEM_BYTES, stream>>>(
+            launch_k(false, k_fused_tma_batch<IDX, TF>, std::min<uint32_t>(ntiles[t], ctas_per_sm * sms), TT_THREADS, TT_SMEM_BYTES, stream, 
                 bm, tiles[t].as<BatchTile>(), ntiles[t]);
     }
 

@@ -91,6 +91,24 @@ void ck(cudaError_t err, const char* what) {
     if (err != cudaSuccess) fail(err == cudaErrorMemoryAllocation ? EFS_ERR_OOM : EFS_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(err));
 }
 
+// Launch of a timestep's kernel.  early: it may be put on the device while the
+// kernel ahead of it in the stream is still running (step_begin waits for that
+// kernel); captured into a graph as the same kind of edge.
+template <class... P, class... A>
+void launch_k(bool early, void (*k)(P...), dim3 grid, dim3 threads, size_t smem, cudaStream_t stream, A&&... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = threads;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = early ? 1 : 0;
+    ck(cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...), "kernel launch");
+}
+
 inline uint32_t blocks(size_t n, uint32_t t) { return (uint32_t)((n + t - 1) / t); }
 
 using efs_host::host_threads;
@@ -553,8 +571,8 @@ struct efs_engine {
                            s.app_off.as<uint32_t>(), s.app_perm.as<uint32_t>(), s.state.as<float>()};
     }
     void launch_ade_apply(const AdeSide& s, float* F) {
-        if (s.app_runs) k_ade_apply_runs<<<blocks(s.app_n, ADE_BLOCK), ADE_T, 0, stream>>>(F, ade_apply_dev(s));
-        else k_ade_apply_grouped<<<blocks(s.app_n, 256), 256, 0, stream>>>(F, ade_apply_dev(s));
+        if (s.app_runs) launch_k(early, k_ade_apply_runs, blocks(s.app_n, ADE_BLOCK), ADE_T, 0, stream, F, ade_apply_dev(s));
+        else launch_k(early, k_ade_apply_grouped, blocks(s.app_n, 256), 256, 0, stream, F, ade_apply_dev(s));
     }
 
     // H cells whose curl reads an E value rewritten by a sparse post-update
@@ -694,48 +712,49 @@ struct efs_engine {
         const float* const* vfl = vflux_ptrs[p].as<const float*>();
         const float* const* cfl = cflux_ptrs[p].as<const float*>();
         const bool sweep = use_sweep(), split = pml_split() && !sweep;
+        early = sweep && pml.empty();
 
         // --- pre-voltage ---
         if (ss_on)     // reads the fields before the UPML pre-update
-            k_steady_state<<<blocks(ss_n, T), T, 0, stream>>>(V, st, k, ss_idx.as<uint32_t>(), ss_n, ss_period,
+            launch_k(early, k_steady_state, blocks(ss_n, T), T, 0, stream, V, st, k, ss_idx.as<uint32_t>(), ss_n, ss_period,
                                                               ss_e1.as<float>(), ss_e2.as<float>());
         if (nf_held.on) {            // samples of step k-1 (its fields are this step's inputs) beside the UPML E pass
             const PassNfSample a{V, C, nf_held.j, nf};
             const uint32_t na = blocks(nf.np, T), nb = blocks(pml_items(), T);
             if (indexed) pair(a, na, pml_e_pass<true>(p), nb);
             else pair(a, na, pml_e_pass<false>(p), nb);
-            if (nf_held.j == NF_K - 1) k_nf2ff_flush<<<blocks(nf.np, T), T, 0, stream>>>(st, k - 1 - nf_held.j, nf_held.j + 1, nf);
+            if (nf_held.j == NF_K - 1) launch_k(early, k_nf2ff_flush, blocks(nf.np, T), T, 0, stream, st, k - 1 - nf_held.j, nf_held.j + 1, nf);
             nf_held.on = false;
         } else if (split) {
             launch_pml_e(p);
         }
         mark(1);
-        if (ade_v.live()) k_ade<<<blocks(ade_v.n, ADE_BLOCK), ADE_T, 0, stream>>>(V, ade_dev(ade_v, vfl));
+        if (ade_v.live()) launch_k(early, k_ade, blocks(ade_v.n, ADE_BLOCK), ADE_T, 0, stream, V, ade_dev(ade_v, vfl));
         MurDev md = mur_dev(vfl);
         if (mur_fast) launch_mur_adopt(p);
-        if (mur_gen) k_mur_pre<<<blocks(mur_gen, T), T, 0, stream>>>(V, md);
+        if (mur_gen) launch_k(early, k_mur_pre, blocks(mur_gen, T), T, 0, stream, V, md);
         RlcDev rd = rlc_dev();
-        if (rlc_on) k_rlc_pre<<<blocks(rlc_n, T), T, 0, stream>>>(rd);
+        if (rlc_on) launch_k(early, k_rlc_pre, blocks(rlc_n, T), T, 0, stream, rd);
         // ADE(curr) reads H and the current flux, which the E side never
         // touches: it runs before the fused kernel overwrites the flux.
-        if (ade_c.live()) k_ade<<<blocks(ade_c.n, ADE_BLOCK), ADE_T, 0, stream>>>(C, ade_dev(ade_c, cfl));
-        if (tf_n && !sweep) k_tfsf_face<<<blocks(tf_n, T), T, 0, stream>>>(st, k, tf_dev());   // TFSF face values of this step
+        if (ade_c.live()) launch_k(early, k_ade, blocks(ade_c.n, ADE_BLOCK), ADE_T, 0, stream, C, ade_dev(ade_c, cfl));
+        if (tf_n && !sweep) launch_k(early, k_tfsf_face, blocks(tf_n, T), T, 0, stream, st, k, tf_dev());   // TFSF face values of this step
         mark(2);
         if (sweep) launch_sweep(p, true);
         else launch_fused_tma(p);
         mark(3);
         // --- post-voltage / apply (on the updated E) ---
-        if (tf_n && sweep) k_tfsf_face_points<<<blocks(tf_n, T), T, 0, stream>>>(V1, st, k, tf_dev());
-        if (tfsf_on && tfsf_v.groups) k_point_sources<1><<<blocks(tfsf_v.groups, T), T, 0, stream>>>(V1, st, k, point_dev(tfsf_v, tfsf_signal, tfsf_len, tfsf_period));
+        if (tf_n && sweep) launch_k(early, k_tfsf_face_points, blocks(tf_n, T), T, 0, stream, V1, st, k, tf_dev());
+        if (tfsf_on && tfsf_v.groups) launch_k(early, k_point_sources<1>, blocks(tfsf_v.groups, T), T, 0, stream, V1, st, k, point_dev(tfsf_v, tfsf_signal, tfsf_len, tfsf_period));
         if (pbc_on) for (auto& a : pbc_axes) launch_pbc(a, true, V1);
-        if (mur_gen) k_mur_post<<<blocks(mur_gen, T), T, 0, stream>>>(V1, md);
+        if (mur_gen) launch_k(early, k_mur_post, blocks(mur_gen, T), T, 0, stream, V1, md);
         if (exc_on && exc_groups) {
             PointSources s{exc_groups, exc_target.as<uint32_t>(), exc_off.as<uint32_t>(), exc_delay.as<uint32_t>(),
                            exc_amp.as<float>(), nullptr, exc_signal.as<float>(), exc_len, exc_period};
-            k_point_sources<0><<<blocks(exc_groups, T), T, 0, stream>>>(V1, st, k, s);
+            launch_k(early, k_point_sources<0>, blocks(exc_groups, T), T, 0, stream, V1, st, k, s);
         }
-        if (mur_gen) k_mur_apply<<<blocks(mur_napply, T), T, 0, stream>>>(V1, md);
-        if (rlc_on) k_rlc_apply<<<blocks(rlc_groups, T), T, 0, stream>>>(V1, rd);
+        if (mur_gen) launch_k(early, k_mur_apply, blocks(mur_napply, T), T, 0, stream, V1, md);
+        if (rlc_on) launch_k(early, k_rlc_apply, blocks(rlc_groups, T), T, 0, stream, V1, rd);
         if (ade_apply && ade_v.live()) launch_ade_apply(ade_v, V1);
         mark(4);
         // --- H of the UPML cells and of the cells next to those E writes ---
@@ -749,7 +768,7 @@ struct efs_engine {
         else if (defer_n) launch_deferred(p);
         mark(5);
         // --- post-current (on the updated H) ---
-        if (tfsf_on && tfsf_c.groups) k_point_sources<1><<<blocks(tfsf_c.groups, T), T, 0, stream>>>(C1, st, k, point_dev(tfsf_c, tfsf_signal, tfsf_len, tfsf_period));
+        if (tfsf_on && tfsf_c.groups) launch_k(early, k_point_sources<1>, blocks(tfsf_c.groups, T), T, 0, stream, C1, st, k, point_dev(tfsf_c, tfsf_signal, tfsf_len, tfsf_period));
         if (pbc_on) for (auto& a : pbc_axes) launch_pbc(a, false, C1);
         if (ade_apply && ade_c.live()) launch_ade_apply(ade_c, C1);
         mark(6);
@@ -761,11 +780,11 @@ struct efs_engine {
             if (nf_pair && split && !last) {
                 nf_held = NfHeld{true, j};           // sampled beside the next step's UPML E pass
             } else {
-                k_nf2ff_sample<<<blocks(nf.np, T), T, 0, stream>>>(V1, C1, j, nf);
-                if (j == NF_K - 1 || last) k_nf2ff_flush<<<blocks(nf.np, T), T, 0, stream>>>(st, k - j, j + 1, nf);
+                launch_k(early, k_nf2ff_sample, blocks(nf.np, T), T, 0, stream, V1, C1, j, nf);
+                if (j == NF_K - 1 || last) launch_k(early, k_nf2ff_flush, blocks(nf.np, T), T, 0, stream, st, k - j, j + 1, nf);
             }
         }
-        if (ring_on) k_gather_ring<<<blocks(ring_n, 64), 64, 0, stream>>>(V1, C1, st, k, ring_dev());
+        if (ring_on) launch_k(early, k_gather_ring, blocks(ring_n, 64), 64, 0, stream, V1, C1, st, k, ring_dev());
         mark(7);
     }
     struct NfHeld { bool on; uint32_t j; };
@@ -783,12 +802,12 @@ struct efs_engine {
     }
     template <class A, class B>
     void pair(const A& a, uint32_t na, const B& b, uint32_t nb) {
-        if (na + nb) k_pair<A, B><<<na + nb, 256, 0, stream>>>(a, na, b, nb);
+        if (na + nb) launch_k(early, k_pair<A, B>, na + nb, 256, 0, stream, a, na, b, nb);
     }
     void launch_mur_adopt(int p) {
         const uint32_t T = 256, nb = blocks(mur_threads(), T);
-        if (indexed) k_mur_adopt<true><<<nb, T, 0, stream>>>(fused_grid(p), vbuf(p), mur_adopt_dev());
-        else k_mur_adopt<false><<<nb, T, 0, stream>>>(fused_grid(p), vbuf(p), mur_adopt_dev());
+        if (indexed) launch_k(early, k_mur_adopt<true>, nb, T, 0, stream, fused_grid(p), vbuf(p), mur_adopt_dev());
+        else launch_k(early, k_mur_adopt<false>, nb, T, 0, stream, fused_grid(p), vbuf(p), mur_adopt_dev());
     }
     // The adopt bits of the material index: UPML cells and the Mur targets of
     // k_mur_adopt.  A dense engine gets an array for them when it has any.
@@ -810,8 +829,8 @@ struct efs_engine {
     }
     void launch_deferred(int p) {
         const uint32_t T = 256;
-        if (indexed) k_deferred_h<true><<<blocks(defer_n, T), T, 0, stream>>>(fused_grid(p), defer_cells.as<uint32_t>(), defer_n);
-        else k_deferred_h<false><<<blocks(defer_n, T), T, 0, stream>>>(fused_grid(p), defer_cells.as<uint32_t>(), defer_n);
+        if (indexed) launch_k(early, k_deferred_h<true>, blocks(defer_n, T), T, 0, stream, fused_grid(p), defer_cells.as<uint32_t>(), defer_n);
+        else launch_k(early, k_deferred_h<false>, blocks(defer_n, T), T, 0, stream, fused_grid(p), defer_cells.as<uint32_t>(), defer_n);
     }
     // `steps` timesteps (at most 64) launched one kernel at a time with the
     // phase marks; accumulates device ms per phase into ms[EFS_PHASES].  Same
@@ -828,7 +847,7 @@ struct efs_engine {
                 enqueue_step(k, q, k + 1 == steps, ev.data() + (size_t)k * (EFS_PHASES + 1));
                 q = pnext(q);
             }
-            k_advance<<<1, 1, 0, stream>>>(state.as<StepState>(), steps);
+            launch_k(early, k_advance, 1, 1, 0, stream, state.as<StepState>(), steps);
             ck(cudaGetLastError(), "phase run");
             sync("phase run");
             for (uint32_t k = 0; k < steps; ++k)
@@ -884,7 +903,7 @@ struct efs_engine {
                "smem attr");
             attr_set = true;
         }
-        k_fused_tma<IDX><<<g, TT_THREADS, TT_SMEM_BYTES, stream>>>(t[0], t[1], t[2], t[3], t[4], t[5], fg);
+        launch_k(early, k_fused_tma<IDX>, g, TT_THREADS, TT_SMEM_BYTES, stream, t[0], t[1], t[2], t[3], t[4], t[5], fg);
     }
     void launch_fused_tma(int p) {
         const FusedGrid fg = fused_grid(p);
@@ -907,14 +926,20 @@ struct efs_engine {
     // the plane pipeline reads with plain loads (120^3 44 / 30, 200^3 191 / 143).
     // An explicit plane depth or a diagnostic plane is a property of the fused
     // kernel and selects it.
+    // Steps of sweeps without UPML are short kernels in a row and launch early;
+    // elsewhere the waiting blocks take their places unevenly on the SMs as the
+    // kernel ahead drains (us per timestep, early / not: cavity 5.8 / 6.1, 81^3
+    // with Mur 12.9 / 14.9, dense 121x109x97 26.5 / 29.1; with UPML 86x87x71
+    // 20.0 / 19.7; 256^3 287 / 253, 16 members batched 205 / 149).
+    bool early = false;              // of the step being enqueued
     bool use_sweep() const { return !xchunk && skip_plane == ~0u && (!indexed || Nd * 52 <= SWEEP_BYTES); }
     template <bool IDX, bool PML>
     void launch_sweep_k(int p, bool volt) {
         const FusedGrid fg = fused_grid(p);
         const PmlSet ps = pml_set(p), pn = pml_set(1 - p);
         const uint32_t nb = Nx * sweep_plane_blocks(Ny, Pz);
-        if (volt) k_sweep_e<IDX, PML><<<nb, SW_T, 0, stream>>>(fg, ps, pn);
-        else k_sweep_h<IDX, PML><<<nb, SW_T, 0, stream>>>(fg, ps, pn);
+        if (volt) launch_k(early, k_sweep_e<IDX, PML>, nb, SW_T, 0, stream, fg, ps, pn);
+        else launch_k(early, k_sweep_h<IDX, PML>, nb, SW_T, 0, stream, fg, ps, pn);
     }
     void launch_sweep(int p, bool volt) {
         const bool hp = !pml.empty();
@@ -932,15 +957,15 @@ struct efs_engine {
         const FusedGrid fg = fused_grid(p);
         const PmlSet ps = pml_set(p), pn = pml_set(1 - p);
         const uint32_t t = pml_items(), T = 256;
-        if (indexed) k_pml_e<true><<<blocks(t, T), T, 0, stream>>>(fg, ps, pn, vbuf(p), t);
-        else k_pml_e<false><<<blocks(t, T), T, 0, stream>>>(fg, ps, pn, vbuf(p), t);
+        if (indexed) launch_k(early, k_pml_e<true>, blocks(t, T), T, 0, stream, fg, ps, pn, vbuf(p), t);
+        else launch_k(early, k_pml_e<false>, blocks(t, T), T, 0, stream, fg, ps, pn, vbuf(p), t);
     }
     void launch_pml_h(int p) {
         const FusedGrid fg = fused_grid(p);
         const PmlSet ps = pml_set(p), pn = pml_set(1 - p);
         const uint32_t t = pml_items(), T = 256;
-        if (indexed) k_pml_h<true><<<blocks(t, T), T, 0, stream>>>(fg, ps, pn, t);
-        else k_pml_h<false><<<blocks(t, T), T, 0, stream>>>(fg, ps, pn, t);
+        if (indexed) launch_k(early, k_pml_h<true>, blocks(t, T), T, 0, stream, fg, ps, pn, t);
+        else launch_k(early, k_pml_h<false>, blocks(t, T), T, 0, stream, fg, ps, pn, t);
     }
 
     PointSources point_dev(const PointSet& p, const DevBuf& sig, uint32_t len, uint32_t period) const {
@@ -971,7 +996,7 @@ struct efs_engine {
         p.Nx = Nx; p.Ny = Ny; p.Nz = Nz; p.Pz = Pz; p.cosP = a.c; p.sinP = a.s;
         p.imag = pbc_imag.as<float>() + a.imag_off;
         dim3 b(16, 16), gr(blocks(p.b0, 16), blocks(p.b1, 16));
-        if (p.b0 && p.b1) k_pbc<<<gr, b, 0, stream>>>(F, p);
+        if (p.b0 && p.b1) launch_k(early, k_pbc, gr, b, 0, stream, F, p);
     }
 
     void iterate(uint32_t n) {
@@ -1001,7 +1026,7 @@ struct efs_engine {
         try {
             int q = p;
             for (uint32_t k = 0; k < m; ++k) { enqueue_step(k, q, k + 1 == m); q = pnext(q); }
-            k_advance<<<1, 1, 0, stream>>>(state.as<StepState>(), m);
+            launch_k(early, k_advance, 1, 1, 0, stream, state.as<StepState>(), m);
         } catch (...) {
             cudaStreamEndCapture(stream, &graph);
             throw;

@@ -12,6 +12,17 @@
 namespace efs {
 
 constexpr int MAX_PML = 24;     // UPML regions handled by the fused update
+// Every kernel of a timestep begins with this.  Where it was launched early
+// (launch_k in efs_engine.cu), its successor may be put on the SMs from here on
+// and its own work starts once every kernel ahead has ended and its writes are
+// visible, so a launch's latency overlaps the kernel ahead.  Field, flux and
+// state loads of these kernels are plain loads: the non-coherent path (__ldg)
+// is for data no timestep writes.
+__device__ __forceinline__ void step_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 struct StepState {              // device-resident, read by every per-step kernel
     uint32_t numTS;
     uint32_t ss_recording;
@@ -93,7 +104,7 @@ struct PointSources {
 // Thread bodies below are shared by the single-engine kernels and the
 // segmented kernels that advance several engines at once (efs_batch.cuh).
 template <int KIND>
-__device__ __forceinline__ void point_sources_body(float* __restrict__ F, const StepState* st, uint32_t k, const PointSources& s,
+__device__ __forceinline__ void point_sources_body(float* F, const StepState* st, uint32_t k, const PointSources& s,
                                                    uint32_t gi) {
     if (gi >= s.ngroups) return;
     const int64_t ts = (int64_t)st->numTS + k;
@@ -120,7 +131,8 @@ __device__ __forceinline__ void point_sources_body(float* __restrict__ F, const 
     F[t] = v;
 }
 template <int KIND>
-__global__ void k_point_sources(float* __restrict__ F, const StepState* st, uint32_t k, const PointSources s) {
+__global__ void k_point_sources(float* F, const StepState* st, uint32_t k, const PointSources s) {
+    step_begin();
     point_sources_body<KIND>(F, st, k, s, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -146,25 +158,25 @@ struct MurDev {
     float* saved;
     const float* const* vflux;
 };
-__device__ __forceinline__ void mur_pre_body(const float* __restrict__ V, const MurDev& m, uint32_t i) {
+__device__ __forceinline__ void mur_pre_body(const float* V, const MurDev& m, uint32_t i) {
     if (i >= m.n) return;
     i = m.ids[i];
     float s = read_loc(V, m.vflux, m.pre_shifted[i]);
     float nv = read_loc(V, m.vflux, m.pre_normal[i]);
     m.saved[i] = __fsub_rn(s, __fmul_rn(m.coeff[i], nv));
 }
-__device__ __forceinline__ void mur_post_body(const float* __restrict__ V, const MurDev& m, uint32_t i) {
+__device__ __forceinline__ void mur_post_body(const float* V, const MurDev& m, uint32_t i) {
     if (i >= m.n) return;
     i = m.ids[i];
     m.saved[i] = __fadd_rn(m.saved[i], __fmul_rn(m.coeff[i], V[m.shifted[i]]));
 }
-__device__ __forceinline__ void mur_apply_body(float* __restrict__ V, const MurDev& m, uint32_t i) {
+__device__ __forceinline__ void mur_apply_body(float* V, const MurDev& m, uint32_t i) {
     if (i >= m.napply) return;
     V[m.apply_target[i]] = m.saved[m.apply_src[i]];
 }
-__global__ void k_mur_pre(const float* __restrict__ V, const MurDev m) { mur_pre_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
-__global__ void k_mur_post(const float* __restrict__ V, const MurDev m) { mur_post_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
-__global__ void k_mur_apply(float* __restrict__ V, const MurDev m) { mur_apply_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
+__global__ void k_mur_pre(const float* V, const MurDev m) { step_begin(); mur_pre_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
+__global__ void k_mur_post(const float* V, const MurDev m) { step_begin(); mur_post_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
+__global__ void k_mur_apply(float* V, const MurDev m) { step_begin(); mur_apply_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
 
 // Lorentz/Drude ADE state update (src/webgpu-fdtd.mjs:405-454), all orders
 // and directions of one field flattened into one list of entries.  The
@@ -199,7 +211,7 @@ __device__ __forceinline__ float ade_one(float v, float st, float& l, uint32_t c
     return __fadd_rn(__fmul_rn(c.x, st), __fmul_rn(c.y, v));
 }
 // Group q of one side (thread body shared with the batched form's segmented launch).
-__device__ __forceinline__ void ade_body(const float* __restrict__ F, const AdeDev& a, uint32_t q) {
+__device__ __forceinline__ void ade_body(const float* F, const AdeDev& a, uint32_t q) {
     constexpr uint32_t NQ = ADE_V / 4;
     const uint32_t i0 = q * ADE_V;
     if (i0 >= a.n) return;
@@ -250,7 +262,8 @@ __device__ __forceinline__ void ade_body(const float* __restrict__ F, const AdeD
         }
     }
 }
-__global__ void __launch_bounds__(ADE_T) k_ade(const float* __restrict__ F, const AdeDev a) {
+__global__ void __launch_bounds__(ADE_T) k_ade(const float* F, const AdeDev a) {
+    step_begin();
     ade_body(F, a, blockIdx.x * ADE_T + threadIdx.x);
 }
 
@@ -271,7 +284,7 @@ struct AdeApplyDev {
     const uint32_t* perm;
     const float* state;
 };
-__device__ __forceinline__ void ade_apply_runs_body(float* __restrict__ F, const AdeApplyDev& a, uint32_t q) {
+__device__ __forceinline__ void ade_apply_runs_body(float* F, const AdeApplyDev& a, uint32_t q) {
     const uint32_t i0 = q * ADE_V;
     if (i0 >= a.n) return;
     const uint32_t cnt = min(ADE_V, a.n - i0);
@@ -298,17 +311,19 @@ __device__ __forceinline__ void ade_apply_runs_body(float* __restrict__ F, const
         }
     }
 }
-__device__ __forceinline__ void ade_apply_grouped_body(float* __restrict__ F, const AdeApplyDev& a, uint32_t g) {
+__device__ __forceinline__ void ade_apply_grouped_body(float* F, const AdeApplyDev& a, uint32_t g) {
     if (g >= a.n) return;
     const uint32_t t = a.target[g];
     float v = F[t];
     for (uint32_t e = a.off[g]; e < a.off[g + 1]; ++e) v = __fsub_rn(v, a.state[a.perm[e]]);
     F[t] = v;
 }
-__global__ void __launch_bounds__(ADE_T) k_ade_apply_runs(float* __restrict__ F, const AdeApplyDev a) {
+__global__ void __launch_bounds__(ADE_T) k_ade_apply_runs(float* F, const AdeApplyDev a) {
+    step_begin();
     ade_apply_runs_body(F, a, blockIdx.x * ADE_T + threadIdx.x);
 }
-__global__ void __launch_bounds__(256) k_ade_apply_grouped(float* __restrict__ F, const AdeApplyDev a) {
+__global__ void __launch_bounds__(256) k_ade_apply_grouped(float* F, const AdeApplyDev a) {
+    step_begin();
     ade_apply_grouped_body(F, a, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -322,6 +337,7 @@ struct RlcDev {
     float* vdn; float* jn; float* vil;
 };
 __global__ void k_rlc_pre(const RlcDev r) {
+    step_begin();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= r.n) return;
     float* V = r.vdn + 3 * (size_t)i;
@@ -332,7 +348,8 @@ __global__ void k_rlc_pre(const RlcDev r) {
         r.vil[i] = __fadd_rn(r.vil[i], __fmul_rn(__fmul_rn(p[0], p[1]), V[1]));
     }
 }
-__global__ void k_rlc_apply(float* __restrict__ F, const RlcDev r) {
+__global__ void k_rlc_apply(float* F, const RlcDev r) {
+    step_begin();
     uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
     if (gi >= r.ngroups) return;
     const uint32_t g = r.gtarget[gi];
@@ -361,8 +378,9 @@ __global__ void k_rlc_apply(float* __restrict__ F, const RlcDev r) {
 
 // Steady-state energy accumulation (src/webgpu-fdtd.mjs:1054-1070); the
 // sample counter is derived from numTS so the kernel needs no atomics.
-__global__ void k_steady_state(const float* __restrict__ V, const StepState* st, uint32_t k, const uint32_t* idx,
+__global__ void k_steady_state(const float* V, const StepState* st, uint32_t k, const uint32_t* idx,
                                uint32_t n, uint32_t period, float* e1, float* e2) {
+    step_begin();
     if (!st->ss_recording) return;
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -380,7 +398,8 @@ struct PbcDev {
     float cosP, sinP;
     float* imag;       // Bloch imaginary parts of this axis, already offset
 };
-__global__ void k_pbc(float* __restrict__ F, const PbcDev p) {
+__global__ void k_pbc(float* F, const PbcDev p) {
+    step_begin();
     const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i1 = blockIdx.y * blockDim.y + threadIdx.y;
     if (i0 >= p.b0 || i1 >= p.b1) return;
@@ -416,7 +435,7 @@ struct RingDev {
     uint32_t G, interval, q0, maxS;
     float* ring;
 };
-__device__ __forceinline__ void gather_ring_body(const float* __restrict__ V, const float* __restrict__ C, const StepState* st,
+__device__ __forceinline__ void gather_ring_body(const float* V, const float* C, const StepState* st,
                                                  uint32_t k, const RingDev& r, uint32_t i) {
     const uint32_t ts1 = st->numTS + k + 1;
     if (ts1 % r.interval != 0) return;
@@ -433,18 +452,19 @@ __device__ __forceinline__ void gather_ring_body(const float* __restrict__ V, co
     row[2 * i] = V[t];
     row[2 * i + 1] = C[t];
 }
-__global__ void k_gather_ring(const float* __restrict__ V, const float* __restrict__ C, const StepState* st, uint32_t k,
+__global__ void k_gather_ring(const float* V, const float* C, const StepState* st, uint32_t k,
                               const RingDev r) {
+    step_begin();
     gather_ring_body(V, C, st, k, r, blockIdx.x * blockDim.x + threadIdx.x);
 }
-__global__ void k_gather(const float* __restrict__ V, const float* __restrict__ C, const uint32_t* idx, uint32_t G, float* out) {
+__global__ void k_gather(const float* V, const float* C, const uint32_t* idx, uint32_t G, float* out) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= G) return;
     out[2 * i] = V[idx[i]];
     out[2 * i + 1] = C[idx[i]];
 }
 
-__global__ void k_advance(StepState* st, uint32_t n) { st->numTS += n; }
+__global__ void k_advance(StepState* st, uint32_t n) { step_begin(); st->numTS += n; }
 
 // ---------------------------------------------------------------------------
 // NF2FF running DFT (src/webgpu-engine.mjs:675-799) for F frequencies.  The
@@ -493,14 +513,16 @@ __device__ __forceinline__ void tfsf_face_body(const StepState* st, uint32_t k, 
     if (i < t.n) t.face[t.dst[i]] = tfsf_face_value(st, k, t, i);
 }
 // The same corrections added to E after a core update that did not apply them.
-__device__ __forceinline__ void tfsf_face_points_body(float* __restrict__ F, const StepState* st, uint32_t k, const TfsfFaceDev& t,
+__device__ __forceinline__ void tfsf_face_points_body(float* F, const StepState* st, uint32_t k, const TfsfFaceDev& t,
                                                       uint32_t i) {
     if (i < t.n) F[t.target[i]] = __fadd_rn(F[t.target[i]], tfsf_face_value(st, k, t, i));
 }
-__global__ void k_tfsf_face_points(float* __restrict__ F, const StepState* st, uint32_t k, const TfsfFaceDev t) {
+__global__ void k_tfsf_face_points(float* F, const StepState* st, uint32_t k, const TfsfFaceDev t) {
+    step_begin();
     tfsf_face_points_body(F, st, k, t, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void k_tfsf_face(const StepState* st, uint32_t k, const TfsfFaceDev t) {
+    step_begin();
     tfsf_face_body(st, k, t, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void k_fill(float* p, size_t n, float v) {
@@ -527,7 +549,7 @@ struct Nf2ffDev {
     float dT32, wnorm;
 };
 // Cell-interpolated E and H at surface point pid (webgpu-engine.mjs:690-761).
-__device__ __forceinline__ void nf2ff_fields(const float* __restrict__ V, const float* __restrict__ C, const Nf2ffDev& d,
+__device__ __forceinline__ void nf2ff_fields(const float* V, const float* C, const Nf2ffDev& d,
                                              uint32_t pid, float E[3], float Hh[3]) {
     const uint32_t ix = d.pts[3 * pid], iy = d.pts[3 * pid + 1], iz = d.pts[3 * pid + 2];
     const size_t Ny = d.Ny, Pz = d.Pz, N = (size_t)d.Nx * Ny * Pz, NyNz = Ny * Pz;
@@ -563,7 +585,7 @@ __device__ __forceinline__ void nf2ff_fields(const float* __restrict__ V, const 
 
 // Every step: the interpolated surface fields of the step into sample slot
 // `slot` ([slot][6][np], E then H components).
-__device__ __forceinline__ void nf2ff_sample_body(const float* __restrict__ V, const float* __restrict__ C, uint32_t slot,
+__device__ __forceinline__ void nf2ff_sample_body(const float* V, const float* C, uint32_t slot,
                                                   const Nf2ffDev& d, uint32_t pid) {
     if (pid >= d.np) return;
     float E[3], Hh[3];
@@ -575,8 +597,9 @@ __device__ __forceinline__ void nf2ff_sample_body(const float* __restrict__ V, c
         s[(size_t)(3 + n) * d.np] = Hh[n];
     }
 }
-__global__ void __launch_bounds__(256) k_nf2ff_sample(const float* __restrict__ V, const float* __restrict__ C, uint32_t slot,
+__global__ void __launch_bounds__(256) k_nf2ff_sample(const float* V, const float* C, uint32_t slot,
                                                       const Nf2ffDev d) {
+    step_begin();
     nf2ff_sample_body(V, C, slot, d, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -651,6 +674,7 @@ __device__ __forceinline__ void nf2ff_flush_block(const StepState* st, uint32_t 
     }
 }
 __global__ void __launch_bounds__(256) k_nf2ff_flush(const StepState* st, uint32_t k0, uint32_t cnt, const Nf2ffDev d) {
+    step_begin();
     nf2ff_flush_block(st, k0, cnt, d, blockIdx.x);
 }
 

@@ -98,11 +98,11 @@ __device__ __forceinline__ void sweep_e_body(const FusedGrid& g, const PmlSet& p
     const float *H = g.H0, *V = g.V0;
     uint2 m = make_uint2(0u, 0u);
     if (IDX || g.mat) m = __ldg(reinterpret_cast<const uint2*>(g.mat + c));
-    const f32x2 hx = ldg2(H + c), hy = ldg2(H + N + c), hz = ldg2(H + 2 * N + c);
-    const f32x2 hzy = ldg2(H + 2 * N + c - dy), hxy = ldg2(H + c - dy);
-    const f32x2 hzx = ldg2(H + 2 * N + c - dx), hyx = ldg2(H + N + c - dx);
-    const float hyz = __ldg(H + N + c - dz), hxz = __ldg(H + c - dz);
-    const f32x2 eo[3] = {ldg2(V + c), ldg2(V + N + c), ldg2(V + 2 * N + c)};
+    const f32x2 hx = ld2(H + c), hy = ld2(H + N + c), hz = ld2(H + 2 * N + c);
+    const f32x2 hzy = ld2(H + 2 * N + c - dy), hxy = ld2(H + c - dy);
+    const f32x2 hzx = ld2(H + 2 * N + c - dx), hyx = ld2(H + N + c - dx);
+    const float hyz = H[N + c - dz], hxz = H[c - dz];
+    const f32x2 eo[3] = {ld2(V + c), ld2(V + N + c), ld2(V + 2 * N + c)};
     PairCoef k;
     if (IDX) k = pair_rows<0>(g.table, m);
     else k = pair_dense(g.vv, g.vi, N, c, true);
@@ -133,7 +133,7 @@ __device__ __forceinline__ void sweep_h_body(const FusedGrid& g, const PmlSet& p
     const uint32_t c = q.x * NyNz + q.y * Pz + q.z;
     const bool core = q.x + 1 < g.Nx && q.y + 1 < g.Ny && q.both, core1 = core && q.z + 2 < g.Nz;   // H beyond the last line: pass-through
     const float* V = g.V1;
-    const f32x2 ho[3] = {ldg2(g.H0 + c), ldg2(g.H0 + N + c), ldg2(g.H0 + 2 * N + c)};
+    const f32x2 ho[3] = {ld2(g.H0 + c), ld2(g.H0 + N + c), ld2(g.H0 + 2 * N + c)};
     PairCoef k;
 #pragma unroll
     for (int n = 0; n < 3; ++n) k.v[n] = k.i[n] = 0ull;
@@ -163,15 +163,14 @@ __device__ __forceinline__ void sweep_h_body(const FusedGrid& g, const PmlSet& p
     sweep_store(g.H1, N, c, q.both, hn);
 }
 
-#ifndef SWB_PML
-#define SWB_PML 4
-#endif
 template <bool IDX, bool PML>
-__global__ void __launch_bounds__(SW_T, PML ? SWB_PML : 4) k_sweep_e(const FusedGrid g, const PmlSet ps, const PmlSet pn) {
+__global__ void __launch_bounds__(SW_T, 4) k_sweep_e(const FusedGrid g, const PmlSet ps, const PmlSet pn) {
+    step_begin();
     sweep_e_body<IDX, PML>(g, ps, pn, blockIdx.x);
 }
 template <bool IDX, bool PML>
-__global__ void __launch_bounds__(SW_T, PML ? SWB_PML : 4) k_sweep_h(const FusedGrid g, const PmlSet ps, const PmlSet pn) {
+__global__ void __launch_bounds__(SW_T, 4) k_sweep_h(const FusedGrid g, const PmlSet ps, const PmlSet pn) {
+    step_begin();
     sweep_h_body<IDX, PML>(g, ps, pn, blockIdx.x);
 }
 

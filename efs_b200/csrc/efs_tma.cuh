@@ -208,7 +208,6 @@ __device__ __forceinline__ f32x2 upd_2(f32x2 vold, f32x2 cv, f32x2 ci, f32x2 cur
     return add2(mul2(vold, cv, nz), mul2(ci, curl, nz));
 }
 __device__ __forceinline__ f32x2 ld2(const float* p) { return *reinterpret_cast<const f32x2*>(p); }
-__device__ __forceinline__ f32x2 ldg2(const float* p) { return __ldg(reinterpret_cast<const f32x2*>(p)); }
 __device__ __forceinline__ f32x2 ldg2_once(const float* p) {   // read once: no L1 line
     f32x2 r;
     asm("ld.global.nc.L1::no_allocate.b64 %0, [%1];" : "=l"(r) : "l"(p));
@@ -300,7 +299,7 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
         const int hi = (lane + 1) * TT_HZ + TT_Z + 4, ei = lane * TT_EZ + TT_Z, hy_ = hi - (y == 0 ? 0 : TT_HZ);
         const size_t off = (size_t)y * Pz + z;
         const int tf = tf_tile && has ? tf_face(g.tf, z) : -1;
-        float hp = in ? __ldg(g.H0 + (size_t)(xs > 0 ? xs - 1 : 0) * NyNz + 2 * N + off) : 0.f;   // Hz(x-1)
+        float hp = in ? g.H0[(size_t)(xs > 0 ? xs - 1 : 0) * NyNz + 2 * N + off] : 0.f;   // Hz(x-1)
         float kc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};        // dense coefficients, loaded a plane ahead
         if (!IDX && in) coeffs_f<false>(g, (size_t)xs * NyNz + off, 0u, 0, kc);
         bool out = false;
@@ -378,8 +377,8 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
     f32x2 hp[3] = {0ull, 0ull, 0ull}, ep[3] = {0ull, 0ull, 0ull};   // H_old(x-1), E_new(x-1) of the pair
     if (in) {
         const float* H = g.H0 + (size_t)(xs > 0 ? xs - 1 : 0) * NyNz + off;
-        hp[1] = ldg2(H + N);
-        hp[2] = ldg2(H + 2 * N);
+        hp[1] = ld2(H + N);
+        hp[2] = ld2(H + 2 * N);
     }
     const f32x2 nz = g.nz;
     PairCoef ke, kh;                                         // E coefficients of plane x, H coefficients of plane x-1
@@ -517,6 +516,7 @@ __global__ void __launch_bounds__(TT_THREADS, 2)
 k_fused_tma(const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmE,
             const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmD,
             const __grid_constant__ CUtensorMap tmE1, const __grid_constant__ CUtensorMap tmH1, const FusedGrid g) {
+    step_begin();
     const uint32_t xs = blockIdx.z * g.xchunk;
     if (xs >= g.Nx) return;                                  // uniform per CTA
     TmaSmem& S = tt_smem();
@@ -586,7 +586,7 @@ __device__ __forceinline__ void pml_fetch(const PmlRegion& R, uint32_t x, uint32
                                           float fn[3], float fo[3]) {
     const size_t p0 = region_p(R, 0, x, y, z), nreg = (size_t)R.n[0] * R.n[1] * R.n[2];
 #pragma unroll
-    for (int n = 0; n < 3; ++n) fo[n] = __ldg((VOLT ? R.vflux : R.cflux) + p0 + n * nreg);
+    for (int n = 0; n < 3; ++n) fo[n] = (VOLT ? R.vflux : R.cflux)[p0 + n * nreg];
     if (R.cidx) {
         const float4* row = R.ctab + 6 * (uint32_t)__ldg(R.cidx + p0) + (VOLT ? 0 : 3);
         const float4 ka = __ldg(row), kb = __ldg(row + 1), kf = __ldg(row + 2);
@@ -675,6 +675,7 @@ __device__ __forceinline__ void pml_e_body(const FusedGrid& g, const PmlSet& ps,
 }
 template <bool IDX>
 __global__ void __launch_bounds__(256, PML_MINB) k_pml_e(const FusedGrid g, const PmlSet ps, const PmlSet pn, float* V0w, uint32_t items) {
+    step_begin();
     pml_e_body<IDX>(g, ps, pn, V0w, items, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -742,6 +743,7 @@ __device__ __forceinline__ void pml_h_body(const FusedGrid& g, const PmlSet& ps,
 }
 template <bool IDX>
 __global__ void __launch_bounds__(256, PML_MINB) k_pml_h(const FusedGrid g, const PmlSet ps, const PmlSet pn, uint32_t items) {
+    step_begin();
     pml_h_body<IDX>(g, ps, pn, items, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -774,6 +776,7 @@ struct PassNfSample {
 };
 template <class A, class B>
 __global__ void __launch_bounds__(256, PML_MINB) k_pair(const A a, uint32_t na, const B b, uint32_t nb) {
+    step_begin();
     const uint32_t i = blockIdx.x, m = min(na, nb);
     if (i < 2 * m) {
         if (i & 1u) b.run(i >> 1);
