@@ -39,7 +39,6 @@ struct BatchTile { uint32_t m, xs, y0, z0; };
 template <bool IDX, bool TF>
 __global__ void __launch_bounds__(TT_THREADS, 2)
 k_fused_tma_batch(const BatchMember* __restrict__ mem, const BatchTile* __restrict__ tiles, uint32_t ntiles) {
-    step_begin();
     TmaSmem& S = tt_smem();
     tt_init(S);
     TmaRing rg;                                        // pipeline state across the CTA's tiles
@@ -60,7 +59,6 @@ struct SegMap { const uint32_t* seg; const uint32_t* first; };
 
 template <class Op>
 __global__ void __launch_bounds__(256) k_seg(const Op* __restrict__ ops, SegMap sm, uint32_t k, uint32_t a, uint32_t b) {
-    step_begin();
     const uint32_t s = sm.seg[blockIdx.x];
     ops[s].run(blockIdx.x - sm.first[s], k, a, b);
 }

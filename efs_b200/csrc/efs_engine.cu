@@ -92,10 +92,14 @@ void ck(cudaError_t err, const char* what) {
 }
 
 // Launch of a timestep's kernel.  early: it may be put on the device while the
-// kernel ahead of it in the stream is still running (step_begin waits for that
-// kernel); captured into a graph as the same kind of edge.
+// kernel ahead of it in the stream is still running, and k begins with
+// step_begin; captured into a graph as the same kind of edge.
 template <class... P, class... A>
 void launch_k(bool early, void (*k)(P...), dim3 grid, dim3 threads, size_t smem, cudaStream_t stream, A&&... args) {
+    if (!early) {
+        k<<<grid, threads, smem, stream>>>(static_cast<P>(args)...);
+        return;
+    }
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -105,7 +109,7 @@ void launch_k(bool early, void (*k)(P...), dim3 grid, dim3 threads, size_t smem,
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &at;
-    cfg.numAttrs = early ? 1 : 0;
+    cfg.numAttrs = 1;
     ck(cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...), "kernel launch");
 }
 
@@ -571,8 +575,8 @@ struct efs_engine {
                            s.app_off.as<uint32_t>(), s.app_perm.as<uint32_t>(), s.state.as<float>()};
     }
     void launch_ade_apply(const AdeSide& s, float* F) {
-        if (s.app_runs) launch_k(early, k_ade_apply_runs, blocks(s.app_n, ADE_BLOCK), ADE_T, 0, stream, F, ade_apply_dev(s));
-        else launch_k(early, k_ade_apply_grouped, blocks(s.app_n, 256), 256, 0, stream, F, ade_apply_dev(s));
+        if (s.app_runs) launch_k(false, k_ade_apply_runs, blocks(s.app_n, ADE_BLOCK), ADE_T, 0, stream, F, ade_apply_dev(s));
+        else launch_k(false, k_ade_apply_grouped, blocks(s.app_n, 256), 256, 0, stream, F, ade_apply_dev(s));
     }
 
     // H cells whose curl reads an E value rewritten by a sparse post-update
@@ -716,45 +720,45 @@ struct efs_engine {
 
         // --- pre-voltage ---
         if (ss_on)     // reads the fields before the UPML pre-update
-            launch_k(early, k_steady_state, blocks(ss_n, T), T, 0, stream, V, st, k, ss_idx.as<uint32_t>(), ss_n, ss_period,
+            launch_k(false, k_steady_state, blocks(ss_n, T), T, 0, stream, V, st, k, ss_idx.as<uint32_t>(), ss_n, ss_period,
                                                               ss_e1.as<float>(), ss_e2.as<float>());
         if (nf_held.on) {            // samples of step k-1 (its fields are this step's inputs) beside the UPML E pass
             const PassNfSample a{V, C, nf_held.j, nf};
             const uint32_t na = blocks(nf.np, T), nb = blocks(pml_items(), T);
             if (indexed) pair(a, na, pml_e_pass<true>(p), nb);
             else pair(a, na, pml_e_pass<false>(p), nb);
-            if (nf_held.j == NF_K - 1) launch_k(early, k_nf2ff_flush, blocks(nf.np, T), T, 0, stream, st, k - 1 - nf_held.j, nf_held.j + 1, nf);
+            if (nf_held.j == NF_K - 1) launch_k(false, k_nf2ff_flush, blocks(nf.np, T), T, 0, stream, st, k - 1 - nf_held.j, nf_held.j + 1, nf);
             nf_held.on = false;
         } else if (split) {
             launch_pml_e(p);
         }
         mark(1);
-        if (ade_v.live()) launch_k(early, k_ade, blocks(ade_v.n, ADE_BLOCK), ADE_T, 0, stream, V, ade_dev(ade_v, vfl));
+        if (ade_v.live()) launch_k(false, k_ade, blocks(ade_v.n, ADE_BLOCK), ADE_T, 0, stream, V, ade_dev(ade_v, vfl));
         MurDev md = mur_dev(vfl);
         if (mur_fast) launch_mur_adopt(p);
-        if (mur_gen) launch_k(early, k_mur_pre, blocks(mur_gen, T), T, 0, stream, V, md);
+        if (mur_gen) launch_k(false, k_mur_pre, blocks(mur_gen, T), T, 0, stream, V, md);
         RlcDev rd = rlc_dev();
-        if (rlc_on) launch_k(early, k_rlc_pre, blocks(rlc_n, T), T, 0, stream, rd);
+        if (rlc_on) launch_k(false, k_rlc_pre, blocks(rlc_n, T), T, 0, stream, rd);
         // ADE(curr) reads H and the current flux, which the E side never
         // touches: it runs before the fused kernel overwrites the flux.
-        if (ade_c.live()) launch_k(early, k_ade, blocks(ade_c.n, ADE_BLOCK), ADE_T, 0, stream, C, ade_dev(ade_c, cfl));
-        if (tf_n && !sweep) launch_k(early, k_tfsf_face, blocks(tf_n, T), T, 0, stream, st, k, tf_dev());   // TFSF face values of this step
+        if (ade_c.live()) launch_k(false, k_ade, blocks(ade_c.n, ADE_BLOCK), ADE_T, 0, stream, C, ade_dev(ade_c, cfl));
+        if (tf_n && !sweep) launch_k(false, k_tfsf_face, blocks(tf_n, T), T, 0, stream, st, k, tf_dev());   // TFSF face values of this step
         mark(2);
         if (sweep) launch_sweep(p, true);
         else launch_fused_tma(p);
         mark(3);
         // --- post-voltage / apply (on the updated E) ---
-        if (tf_n && sweep) launch_k(early, k_tfsf_face_points, blocks(tf_n, T), T, 0, stream, V1, st, k, tf_dev());
-        if (tfsf_on && tfsf_v.groups) launch_k(early, k_point_sources<1>, blocks(tfsf_v.groups, T), T, 0, stream, V1, st, k, point_dev(tfsf_v, tfsf_signal, tfsf_len, tfsf_period));
+        if (tf_n && sweep) launch_k(false, k_tfsf_face_points, blocks(tf_n, T), T, 0, stream, V1, st, k, tf_dev());
+        if (tfsf_on && tfsf_v.groups) launch_k(early, early ? k_point_sources<1, true> : k_point_sources<1, false>, blocks(tfsf_v.groups, T), T, 0, stream, V1, st, k, point_dev(tfsf_v, tfsf_signal, tfsf_len, tfsf_period));
         if (pbc_on) for (auto& a : pbc_axes) launch_pbc(a, true, V1);
-        if (mur_gen) launch_k(early, k_mur_post, blocks(mur_gen, T), T, 0, stream, V1, md);
+        if (mur_gen) launch_k(false, k_mur_post, blocks(mur_gen, T), T, 0, stream, V1, md);
         if (exc_on && exc_groups) {
             PointSources s{exc_groups, exc_target.as<uint32_t>(), exc_off.as<uint32_t>(), exc_delay.as<uint32_t>(),
                            exc_amp.as<float>(), nullptr, exc_signal.as<float>(), exc_len, exc_period};
-            launch_k(early, k_point_sources<0>, blocks(exc_groups, T), T, 0, stream, V1, st, k, s);
+            launch_k(early, early ? k_point_sources<0, true> : k_point_sources<0, false>, blocks(exc_groups, T), T, 0, stream, V1, st, k, s);
         }
-        if (mur_gen) launch_k(early, k_mur_apply, blocks(mur_napply, T), T, 0, stream, V1, md);
-        if (rlc_on) launch_k(early, k_rlc_apply, blocks(rlc_groups, T), T, 0, stream, V1, rd);
+        if (mur_gen) launch_k(false, k_mur_apply, blocks(mur_napply, T), T, 0, stream, V1, md);
+        if (rlc_on) launch_k(false, k_rlc_apply, blocks(rlc_groups, T), T, 0, stream, V1, rd);
         if (ade_apply && ade_v.live()) launch_ade_apply(ade_v, V1);
         mark(4);
         // --- H of the UPML cells and of the cells next to those E writes ---
@@ -768,7 +772,7 @@ struct efs_engine {
         else if (defer_n) launch_deferred(p);
         mark(5);
         // --- post-current (on the updated H) ---
-        if (tfsf_on && tfsf_c.groups) launch_k(early, k_point_sources<1>, blocks(tfsf_c.groups, T), T, 0, stream, C1, st, k, point_dev(tfsf_c, tfsf_signal, tfsf_len, tfsf_period));
+        if (tfsf_on && tfsf_c.groups) launch_k(early, early ? k_point_sources<1, true> : k_point_sources<1, false>, blocks(tfsf_c.groups, T), T, 0, stream, C1, st, k, point_dev(tfsf_c, tfsf_signal, tfsf_len, tfsf_period));
         if (pbc_on) for (auto& a : pbc_axes) launch_pbc(a, false, C1);
         if (ade_apply && ade_c.live()) launch_ade_apply(ade_c, C1);
         mark(6);
@@ -780,11 +784,11 @@ struct efs_engine {
             if (nf_pair && split && !last) {
                 nf_held = NfHeld{true, j};           // sampled beside the next step's UPML E pass
             } else {
-                launch_k(early, k_nf2ff_sample, blocks(nf.np, T), T, 0, stream, V1, C1, j, nf);
-                if (j == NF_K - 1 || last) launch_k(early, k_nf2ff_flush, blocks(nf.np, T), T, 0, stream, st, k - j, j + 1, nf);
+                launch_k(false, k_nf2ff_sample, blocks(nf.np, T), T, 0, stream, V1, C1, j, nf);
+                if (j == NF_K - 1 || last) launch_k(false, k_nf2ff_flush, blocks(nf.np, T), T, 0, stream, st, k - j, j + 1, nf);
             }
         }
-        if (ring_on) launch_k(early, k_gather_ring, blocks(ring_n, 64), 64, 0, stream, V1, C1, st, k, ring_dev());
+        if (ring_on) launch_k(early, early ? k_gather_ring<true> : k_gather_ring<false>, blocks(ring_n, 64), 64, 0, stream, V1, C1, st, k, ring_dev());
         mark(7);
     }
     struct NfHeld { bool on; uint32_t j; };
@@ -802,12 +806,12 @@ struct efs_engine {
     }
     template <class A, class B>
     void pair(const A& a, uint32_t na, const B& b, uint32_t nb) {
-        if (na + nb) launch_k(early, k_pair<A, B>, na + nb, 256, 0, stream, a, na, b, nb);
+        if (na + nb) launch_k(false, k_pair<A, B>, na + nb, 256, 0, stream, a, na, b, nb);
     }
     void launch_mur_adopt(int p) {
         const uint32_t T = 256, nb = blocks(mur_threads(), T);
-        if (indexed) launch_k(early, k_mur_adopt<true>, nb, T, 0, stream, fused_grid(p), vbuf(p), mur_adopt_dev());
-        else launch_k(early, k_mur_adopt<false>, nb, T, 0, stream, fused_grid(p), vbuf(p), mur_adopt_dev());
+        if (indexed) launch_k(early, early ? k_mur_adopt<true, true> : k_mur_adopt<true, false>, nb, T, 0, stream, fused_grid(p), vbuf(p), mur_adopt_dev());
+        else launch_k(early, early ? k_mur_adopt<false, true> : k_mur_adopt<false, false>, nb, T, 0, stream, fused_grid(p), vbuf(p), mur_adopt_dev());
     }
     // The adopt bits of the material index: UPML cells and the Mur targets of
     // k_mur_adopt.  A dense engine gets an array for them when it has any.
@@ -829,8 +833,8 @@ struct efs_engine {
     }
     void launch_deferred(int p) {
         const uint32_t T = 256;
-        if (indexed) launch_k(early, k_deferred_h<true>, blocks(defer_n, T), T, 0, stream, fused_grid(p), defer_cells.as<uint32_t>(), defer_n);
-        else launch_k(early, k_deferred_h<false>, blocks(defer_n, T), T, 0, stream, fused_grid(p), defer_cells.as<uint32_t>(), defer_n);
+        if (indexed) launch_k(false, k_deferred_h<true>, blocks(defer_n, T), T, 0, stream, fused_grid(p), defer_cells.as<uint32_t>(), defer_n);
+        else launch_k(false, k_deferred_h<false>, blocks(defer_n, T), T, 0, stream, fused_grid(p), defer_cells.as<uint32_t>(), defer_n);
     }
     // `steps` timesteps (at most 64) launched one kernel at a time with the
     // phase marks; accumulates device ms per phase into ms[EFS_PHASES].  Same
@@ -847,7 +851,7 @@ struct efs_engine {
                 enqueue_step(k, q, k + 1 == steps, ev.data() + (size_t)k * (EFS_PHASES + 1));
                 q = pnext(q);
             }
-            launch_k(early, k_advance, 1, 1, 0, stream, state.as<StepState>(), steps);
+            launch_k(early, early ? k_advance<true> : k_advance<false>, 1, 1, 0, stream, state.as<StepState>(), steps);
             ck(cudaGetLastError(), "phase run");
             sync("phase run");
             for (uint32_t k = 0; k < steps; ++k)
@@ -903,7 +907,7 @@ struct efs_engine {
                "smem attr");
             attr_set = true;
         }
-        launch_k(early, k_fused_tma<IDX>, g, TT_THREADS, TT_SMEM_BYTES, stream, t[0], t[1], t[2], t[3], t[4], t[5], fg);
+        launch_k(false, k_fused_tma<IDX>, g, TT_THREADS, TT_SMEM_BYTES, stream, t[0], t[1], t[2], t[3], t[4], t[5], fg);
     }
     void launch_fused_tma(int p) {
         const FusedGrid fg = fused_grid(p);
@@ -957,15 +961,15 @@ struct efs_engine {
         const FusedGrid fg = fused_grid(p);
         const PmlSet ps = pml_set(p), pn = pml_set(1 - p);
         const uint32_t t = pml_items(), T = 256;
-        if (indexed) launch_k(early, k_pml_e<true>, blocks(t, T), T, 0, stream, fg, ps, pn, vbuf(p), t);
-        else launch_k(early, k_pml_e<false>, blocks(t, T), T, 0, stream, fg, ps, pn, vbuf(p), t);
+        if (indexed) launch_k(false, k_pml_e<true>, blocks(t, T), T, 0, stream, fg, ps, pn, vbuf(p), t);
+        else launch_k(false, k_pml_e<false>, blocks(t, T), T, 0, stream, fg, ps, pn, vbuf(p), t);
     }
     void launch_pml_h(int p) {
         const FusedGrid fg = fused_grid(p);
         const PmlSet ps = pml_set(p), pn = pml_set(1 - p);
         const uint32_t t = pml_items(), T = 256;
-        if (indexed) launch_k(early, k_pml_h<true>, blocks(t, T), T, 0, stream, fg, ps, pn, t);
-        else launch_k(early, k_pml_h<false>, blocks(t, T), T, 0, stream, fg, ps, pn, t);
+        if (indexed) launch_k(false, k_pml_h<true>, blocks(t, T), T, 0, stream, fg, ps, pn, t);
+        else launch_k(false, k_pml_h<false>, blocks(t, T), T, 0, stream, fg, ps, pn, t);
     }
 
     PointSources point_dev(const PointSet& p, const DevBuf& sig, uint32_t len, uint32_t period) const {
@@ -996,7 +1000,7 @@ struct efs_engine {
         p.Nx = Nx; p.Ny = Ny; p.Nz = Nz; p.Pz = Pz; p.cosP = a.c; p.sinP = a.s;
         p.imag = pbc_imag.as<float>() + a.imag_off;
         dim3 b(16, 16), gr(blocks(p.b0, 16), blocks(p.b1, 16));
-        if (p.b0 && p.b1) launch_k(early, k_pbc, gr, b, 0, stream, F, p);
+        if (p.b0 && p.b1) launch_k(false, k_pbc, gr, b, 0, stream, F, p);
     }
 
     void iterate(uint32_t n) {
@@ -1026,7 +1030,7 @@ struct efs_engine {
         try {
             int q = p;
             for (uint32_t k = 0; k < m; ++k) { enqueue_step(k, q, k + 1 == m); q = pnext(q); }
-            launch_k(early, k_advance, 1, 1, 0, stream, state.as<StepState>(), m);
+            launch_k(early, early ? k_advance<true> : k_advance<false>, 1, 1, 0, stream, state.as<StepState>(), m);
         } catch (...) {
             cudaStreamEndCapture(stream, &graph);
             throw;

@@ -191,9 +191,9 @@ __device__ __forceinline__ void mur_adopt_body(const FusedGrid& g, float* V, con
     d.saved[e] = v;
     if (kind & MUR_LAST) V[d.target[e]] = v;
 }
-template <bool IDX>
+template <bool IDX, bool EARLY>
 __global__ void __launch_bounds__(256) k_mur_adopt(const FusedGrid g, float* V, const MurAdoptDev d) {
-    step_begin();
+    if (EARLY) step_begin();
     mur_adopt_body<IDX>(g, V, d, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void k_mat_mur(uint32_t* mat, uint32_t N, const MurAdoptDev d) {
@@ -235,7 +235,6 @@ __device__ __forceinline__ void deferred_h_body(const FusedGrid& g, const uint32
 }
 template <bool IDX>
 __global__ void __launch_bounds__(256) k_deferred_h(const FusedGrid g, const uint32_t* cells, uint32_t n) {
-    step_begin();
     deferred_h_body<IDX>(g, cells, n, blockIdx.x * blockDim.x + threadIdx.x);
 }
 

@@ -12,12 +12,13 @@
 namespace efs {
 
 constexpr int MAX_PML = 24;     // UPML regions handled by the fused update
-// Every kernel of a timestep begins with this.  Where it was launched early
-// (launch_k in efs_engine.cu), its successor may be put on the SMs from here on
-// and its own work starts once every kernel ahead has ended and its writes are
-// visible, so a launch's latency overlaps the kernel ahead.  Field, flux and
-// state loads of these kernels are plain loads: the non-coherent path (__ldg)
-// is for data no timestep writes.
+// Kernels that may be launched early (launch_k in efs_engine.cu; template
+// argument EARLY) begin with this: the kernel behind may be put on the SMs from
+// here on, and this one's work starts once every kernel ahead has ended and its
+// writes are visible, so a launch's latency overlaps the kernel ahead.  Their
+// field and state loads are plain loads: the non-coherent path (__ldg) is for
+// data that nothing writes while they wait.  Kernels never launched early go
+// without it.
 __device__ __forceinline__ void step_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -130,9 +131,9 @@ __device__ __forceinline__ void point_sources_body(float* F, const StepState* st
     }
     F[t] = v;
 }
-template <int KIND>
+template <int KIND, bool EARLY>
 __global__ void k_point_sources(float* F, const StepState* st, uint32_t k, const PointSources s) {
-    step_begin();
+    if (EARLY) step_begin();
     point_sources_body<KIND>(F, st, k, s, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -174,9 +175,9 @@ __device__ __forceinline__ void mur_apply_body(float* V, const MurDev& m, uint32
     if (i >= m.napply) return;
     V[m.apply_target[i]] = m.saved[m.apply_src[i]];
 }
-__global__ void k_mur_pre(const float* V, const MurDev m) { step_begin(); mur_pre_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
-__global__ void k_mur_post(const float* V, const MurDev m) { step_begin(); mur_post_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
-__global__ void k_mur_apply(float* V, const MurDev m) { step_begin(); mur_apply_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
+__global__ void k_mur_pre(const float* V, const MurDev m) { mur_pre_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
+__global__ void k_mur_post(const float* V, const MurDev m) { mur_post_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
+__global__ void k_mur_apply(float* V, const MurDev m) { mur_apply_body(V, m, blockIdx.x * blockDim.x + threadIdx.x); }
 
 // Lorentz/Drude ADE state update (src/webgpu-fdtd.mjs:405-454), all orders
 // and directions of one field flattened into one list of entries.  The
@@ -263,7 +264,6 @@ __device__ __forceinline__ void ade_body(const float* F, const AdeDev& a, uint32
     }
 }
 __global__ void __launch_bounds__(ADE_T) k_ade(const float* F, const AdeDev a) {
-    step_begin();
     ade_body(F, a, blockIdx.x * ADE_T + threadIdx.x);
 }
 
@@ -319,11 +319,9 @@ __device__ __forceinline__ void ade_apply_grouped_body(float* F, const AdeApplyD
     F[t] = v;
 }
 __global__ void __launch_bounds__(ADE_T) k_ade_apply_runs(float* F, const AdeApplyDev a) {
-    step_begin();
     ade_apply_runs_body(F, a, blockIdx.x * ADE_T + threadIdx.x);
 }
 __global__ void __launch_bounds__(256) k_ade_apply_grouped(float* F, const AdeApplyDev a) {
-    step_begin();
     ade_apply_grouped_body(F, a, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -337,7 +335,6 @@ struct RlcDev {
     float* vdn; float* jn; float* vil;
 };
 __global__ void k_rlc_pre(const RlcDev r) {
-    step_begin();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= r.n) return;
     float* V = r.vdn + 3 * (size_t)i;
@@ -349,7 +346,6 @@ __global__ void k_rlc_pre(const RlcDev r) {
     }
 }
 __global__ void k_rlc_apply(float* F, const RlcDev r) {
-    step_begin();
     uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
     if (gi >= r.ngroups) return;
     const uint32_t g = r.gtarget[gi];
@@ -380,7 +376,6 @@ __global__ void k_rlc_apply(float* F, const RlcDev r) {
 // sample counter is derived from numTS so the kernel needs no atomics.
 __global__ void k_steady_state(const float* V, const StepState* st, uint32_t k, const uint32_t* idx,
                                uint32_t n, uint32_t period, float* e1, float* e2) {
-    step_begin();
     if (!st->ss_recording) return;
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -399,7 +394,6 @@ struct PbcDev {
     float* imag;       // Bloch imaginary parts of this axis, already offset
 };
 __global__ void k_pbc(float* F, const PbcDev p) {
-    step_begin();
     const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i1 = blockIdx.y * blockDim.y + threadIdx.y;
     if (i0 >= p.b0 || i1 >= p.b1) return;
@@ -449,12 +443,14 @@ __device__ __forceinline__ void gather_ring_body(const float* V, const float* C,
     float* ring = r.ring;
     const uint32_t t = idx[i];
     float* row = ring + (size_t)s * G * 2;
-    row[2 * i] = V[t];
-    row[2 * i + 1] = C[t];
+    const float v = V[t], c = C[t];             // both loads before a store
+    row[2 * i] = v;
+    row[2 * i + 1] = c;
 }
+template <bool EARLY>
 __global__ void k_gather_ring(const float* V, const float* C, const StepState* st, uint32_t k,
                               const RingDev r) {
-    step_begin();
+    if (EARLY) step_begin();
     gather_ring_body(V, C, st, k, r, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void k_gather(const float* V, const float* C, const uint32_t* idx, uint32_t G, float* out) {
@@ -464,7 +460,11 @@ __global__ void k_gather(const float* V, const float* C, const uint32_t* idx, ui
     out[2 * i + 1] = C[idx[i]];
 }
 
-__global__ void k_advance(StepState* st, uint32_t n) { step_begin(); st->numTS += n; }
+template <bool EARLY>
+__global__ void k_advance(StepState* st, uint32_t n) {
+    if (EARLY) step_begin();
+    st->numTS += n;
+}
 
 // ---------------------------------------------------------------------------
 // NF2FF running DFT (src/webgpu-engine.mjs:675-799) for F frequencies.  The
@@ -518,11 +518,9 @@ __device__ __forceinline__ void tfsf_face_points_body(float* F, const StepState*
     if (i < t.n) F[t.target[i]] = __fadd_rn(F[t.target[i]], tfsf_face_value(st, k, t, i));
 }
 __global__ void k_tfsf_face_points(float* F, const StepState* st, uint32_t k, const TfsfFaceDev t) {
-    step_begin();
     tfsf_face_points_body(F, st, k, t, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void k_tfsf_face(const StepState* st, uint32_t k, const TfsfFaceDev t) {
-    step_begin();
     tfsf_face_body(st, k, t, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void k_fill(float* p, size_t n, float v) {
@@ -599,7 +597,6 @@ __device__ __forceinline__ void nf2ff_sample_body(const float* V, const float* C
 }
 __global__ void __launch_bounds__(256) k_nf2ff_sample(const float* V, const float* C, uint32_t slot,
                                                       const Nf2ffDev d) {
-    step_begin();
     nf2ff_sample_body(V, C, slot, d, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -674,7 +671,6 @@ __device__ __forceinline__ void nf2ff_flush_block(const StepState* st, uint32_t 
     }
 }
 __global__ void __launch_bounds__(256) k_nf2ff_flush(const StepState* st, uint32_t k0, uint32_t cnt, const Nf2ffDev d) {
-    step_begin();
     nf2ff_flush_block(st, k0, cnt, d, blockIdx.x);
 }
 

@@ -516,7 +516,6 @@ __global__ void __launch_bounds__(TT_THREADS, 2)
 k_fused_tma(const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmE,
             const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmD,
             const __grid_constant__ CUtensorMap tmE1, const __grid_constant__ CUtensorMap tmH1, const FusedGrid g) {
-    step_begin();
     const uint32_t xs = blockIdx.z * g.xchunk;
     if (xs >= g.Nx) return;                                  // uniform per CTA
     TmaSmem& S = tt_smem();
@@ -586,7 +585,7 @@ __device__ __forceinline__ void pml_fetch(const PmlRegion& R, uint32_t x, uint32
                                           float fn[3], float fo[3]) {
     const size_t p0 = region_p(R, 0, x, y, z), nreg = (size_t)R.n[0] * R.n[1] * R.n[2];
 #pragma unroll
-    for (int n = 0; n < 3; ++n) fo[n] = (VOLT ? R.vflux : R.cflux)[p0 + n * nreg];
+    for (int n = 0; n < 3; ++n) fo[n] = __ldg((VOLT ? R.vflux : R.cflux) + p0 + n * nreg);
     if (R.cidx) {
         const float4* row = R.ctab + 6 * (uint32_t)__ldg(R.cidx + p0) + (VOLT ? 0 : 3);
         const float4 ka = __ldg(row), kb = __ldg(row + 1), kf = __ldg(row + 2);
@@ -675,7 +674,6 @@ __device__ __forceinline__ void pml_e_body(const FusedGrid& g, const PmlSet& ps,
 }
 template <bool IDX>
 __global__ void __launch_bounds__(256, PML_MINB) k_pml_e(const FusedGrid g, const PmlSet ps, const PmlSet pn, float* V0w, uint32_t items) {
-    step_begin();
     pml_e_body<IDX>(g, ps, pn, V0w, items, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -743,7 +741,6 @@ __device__ __forceinline__ void pml_h_body(const FusedGrid& g, const PmlSet& ps,
 }
 template <bool IDX>
 __global__ void __launch_bounds__(256, PML_MINB) k_pml_h(const FusedGrid g, const PmlSet ps, const PmlSet pn, uint32_t items) {
-    step_begin();
     pml_h_body<IDX>(g, ps, pn, items, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -776,7 +773,6 @@ struct PassNfSample {
 };
 template <class A, class B>
 __global__ void __launch_bounds__(256, PML_MINB) k_pair(const A a, uint32_t na, const B b, uint32_t nb) {
-    step_begin();
     const uint32_t i = blockIdx.x, m = min(na, nb);
     if (i < 2 * m) {
         if (i & 1u) b.run(i >> 1);
