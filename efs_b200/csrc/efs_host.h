@@ -1,13 +1,15 @@
-// Host-side planning helpers of the engine (plain C++17, no CUDA): the
-// threaded stable radix sort that orders point lists by device index, the
-// grouping of entries by target built on it, and the chunked host-thread
-// loop.  Compiled into libefs.so and, on its own, into the CPU test of these
-// helpers (tests/test_host_plan.py).
+// Host-side helpers of the engine (plain C++17, no CUDA): the threaded stable
+// radix sort that orders point lists by device index, the grouping of entries
+// by target built on it, the chunked host-thread loop, and the copy through
+// staging buffers of large read-backs.  Compiled into libefs.so and, on its own, into the CPU test of these
+// helpers (tests/test_host_plan.py, tests/test_staged_copy.py).
 #pragma once
 
 #include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <cstring>
 #include <thread>
 #include <vector>
 
@@ -93,6 +95,58 @@ inline void group_by(const std::vector<uint32_t>& tgt, std::vector<uint32_t>& ut
         }
     }
     if (n) off.push_back(n);
+}
+
+// `bytes` bytes into dst in chunks through `slots` staging buffers: fetch(c, n)
+// starts chunk c (n bytes) into buffer c % slots, wait(c) returns once it has
+// arrived, T threads copy each arrived chunk out (every thread a part of it)
+// while later chunks are on their way.  fetch and wait run on the caller's
+// thread and may throw; chunks started and not yet waited for are then left to
+// the caller.
+template <class Fetch, class Wait>
+void staged_copy(void* dst, size_t bytes, const uint8_t* const* buf, unsigned slots, size_t chunk, unsigned T, Fetch&& fetch,
+                 Wait&& wait) {
+    const size_t nc = (bytes + chunk - 1) / chunk;
+    auto size = [&](size_t c) { return std::min(chunk, bytes - c * chunk); };
+    std::atomic<size_t> ready{0};                      // chunks that have arrived
+    std::atomic<bool> stop{false};
+    std::vector<std::atomic<unsigned>> done(slots);    // threads that have copied their part of the buffer's chunk
+    for (auto& d : done) d = 0;
+    auto work = [&](unsigned t) {
+        for (size_t c = 0; c < nc; ++c) {
+            while (ready.load(std::memory_order_acquire) <= c) {
+                if (stop.load(std::memory_order_relaxed)) return;
+                std::this_thread::yield();
+            }
+            const size_t n = size(c), lo = n * t / T, hi = n * (t + 1) / T;
+            memcpy(static_cast<uint8_t*>(dst) + c * chunk + lo, buf[c % slots] + lo, hi - lo);
+            done[c % slots].fetch_add(1, std::memory_order_release);
+        }
+    };
+    std::vector<std::thread> th;
+    auto join = [&] { for (auto& x : th) x.join(); };
+    try {
+        th.reserve(T);
+        for (unsigned t = 0; t < T; ++t) th.emplace_back(work, t);
+        size_t started = 0;
+        for (size_t c = 0; c < nc; ++c) {
+            for (; started < nc && started < c + slots; ++started) {
+                auto& d = done[started % slots];
+                if (started >= slots) {                // the buffer's previous chunk has been copied out
+                    while (d.load(std::memory_order_acquire) < T) std::this_thread::yield();
+                    d = 0;
+                }
+                fetch(started, size(started));
+            }
+            wait(c);
+            ready.store(c + 1, std::memory_order_release);
+        }
+    } catch (...) {
+        stop = true;
+        join();
+        throw;
+    }
+    join();
 }
 
 }  // namespace efs_host
