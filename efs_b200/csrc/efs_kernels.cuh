@@ -40,6 +40,10 @@ struct PmlRegion {
     // has more than 65535 distinct cell tuples): per cell a row index, per row
     // six float4 {vv, vvfo, vvfn, ii, iifo, iifn} x 3 components (+ pad).
     const uint16_t* cidx; const float4* ctab;
+    // Work items of the UPML passes: -1: the region's own rows in order; r >= 0:
+    // its rows alternate with region r's (two z slabs over the same rows);
+    // -2: listed with an earlier region.
+    int mate;
 };
 // Regions by coordinate: bit r of xm[x] says that region r's x range holds x,
 // and so for y and z (zero beyond the grid), so the regions of a cell are three

@@ -551,18 +551,27 @@ constexpr uint32_t PML_ZC = EFS_PML_ZC;     // z cells per thread
 constexpr int PML_MINB = EFS_PML_MINB;      // resident 256-thread blocks per SM the register budget is set for
 
 // Work item i -> region r, row (x, y), first z and cell count (PML_ZC cells
-// per item along z, items in region order).
+// per item along z, items in region order, mated regions row by row: the high
+// slab's end of a row and the low slab's start of the next lie in one 64-byte
+// DRAM access, see FIELD_SHIFT).
 __device__ __forceinline__ bool pml_item(const PmlSet& ps, uint32_t i, int& r, uint32_t& x, uint32_t& y, uint32_t& z,
                                          uint32_t& cnt) {
     for (r = 0; r < ps.count; ++r) {
         const PmlRegion& R = ps.r[r];
-        const uint32_t zc = (R.n[2] + PML_ZC - 1) / PML_ZC;
-        const uint32_t items = R.n[0] * R.n[1] * zc;
+        if (R.mate == -2) continue;
+        const uint32_t zc = (R.n[2] + PML_ZC - 1) / PML_ZC, rc = R.mate >= 0 ? 2 * zc : zc;   // items of a row
+        const uint32_t items = R.n[0] * R.n[1] * rc;
         if (i < items) {
-            const uint32_t row = i / zc, zi = i - row * zc;
+            const uint32_t row = i / rc;
+            uint32_t zi = i - row * rc, s2 = R.s[2];
             x = R.s[0] + row / R.n[1];
             y = R.s[1] + row % R.n[1];
-            z = R.s[2] + zi * PML_ZC;
+            if (zi >= zc) {                              // the mate's half of the row
+                zi -= zc;
+                r = R.mate;
+                s2 = ps.r[r].s[2];
+            }
+            z = s2 + zi * PML_ZC;
             cnt = min(PML_ZC, R.n[2] - zi * PML_ZC);
             return true;
         }
