@@ -91,6 +91,11 @@ struct OpAde {
     const float* F; AdeDev a;
     __device__ void run(uint32_t blk, uint32_t, uint32_t, uint32_t) const { ade_body(F, a, blk * blockDim.x + threadIdx.x); }
 };
+template <bool IDX>
+struct OpAdeAdopt {
+    FusedGrid g; float* V; AdeDev a;
+    __device__ void run(uint32_t blk, uint32_t, uint32_t, uint32_t) const { ade_adopt_body<IDX>(g, V, a, blk * blockDim.x + threadIdx.x); }
+};
 struct OpTfsfFace {
     const StepState* st; TfsfFaceDev t;
     __device__ void run(uint32_t blk, uint32_t k, uint32_t, uint32_t) const { tfsf_face_body(st, k, t, blk * blockDim.x + threadIdx.x); }
@@ -180,7 +185,7 @@ struct efs_batch {
     uint32_t phase = 0;
     DevBuf members[2], tiles[4];               // tile lists by tile_class
     uint32_t ntiles[4] = {0, 0, 0, 0};
-    SegLaunch mur_adopt_i[2], mur_adopt_d[2], mur_pre[2], mur_post[2], mur_apply[2], exc[2], tfsf_v[2], tfsf_c[2], ade_v[2], ade_c[2], ade_apply_v[2], ade_apply_c[2],
+    SegLaunch ade_adopt_i[2], ade_adopt_d[2], mur_adopt_i[2], mur_adopt_d[2], mur_pre[2], mur_post[2], mur_apply[2], exc[2], tfsf_v[2], tfsf_c[2], ade_v[2], ade_c[2], ade_apply_v[2], ade_apply_c[2],
         ring[2], nf_sample[2], nf_flush[2],
         deferred_i[2], deferred_d[2], pml_e_i[2], pml_e_d[2], pml_h_i[2], pml_h_d[2], tfsf_face[2], advance;   // _i / _d: index / dense members
     bool any_nf = false;
@@ -276,6 +281,8 @@ struct efs_batch {
         any_nf = false;
         for (int s = 0; s < 2; ++s) {
             std::vector<BatchMember> bm(E);
+            std::vector<std::pair<uint32_t, OpAdeAdopt<true>>> vai;
+            std::vector<std::pair<uint32_t, OpAdeAdopt<false>>> vad;
             std::vector<std::pair<uint32_t, OpMurAdopt<true>>> vmi;
             std::vector<std::pair<uint32_t, OpMurAdopt<false>>> vmd;
             std::vector<std::pair<uint32_t, OpMurPre>> mpre;
@@ -338,14 +345,18 @@ struct efs_batch {
                 if (e->tfsf_on && e->tfsf_c.groups)
                     vtc.push_back({e->tfsf_c.groups, OpPoints<1>{C1, st, e->point_dev(e->tfsf_c, e->tfsf_signal, e->tfsf_len, e->tfsf_period)}});
                 // ADE: one thread per group of ADE_V entries; reads the pre-update fields and the old flux
-                if (e->ade_v.live())
+                if (e->ade_adopt) {
+                    const AdeDev ad = e->ade_dev(e->ade_v, e->vflux_ptrs[p].as<const float*>());
+                    if (e->indexed) vai.push_back({e->ade_v.n, OpAdeAdopt<true>{fg, V, ad}});
+                    else vad.push_back({e->ade_v.n, OpAdeAdopt<false>{fg, V, ad}});
+                } else if (e->ade_v.live())
                     vav.push_back({(e->ade_v.n + ADE_V - 1) / ADE_V, OpAde{V, e->ade_dev(e->ade_v, e->vflux_ptrs[p].as<const float*>())}});
                 if (e->ade_c.live())
                     vac.push_back({(e->ade_c.n + ADE_V - 1) / ADE_V, OpAde{e->cbuf(p), e->ade_dev(e->ade_c, e->cflux_ptrs[p].as<const float*>())}});
                 // ADE apply step: threads of ADE_V entries (runs form) or one per location (grouped form)
                 for (int side = 0; side < 2; ++side) {
                     const efs_engine::AdeSide& as = side == 0 ? e->ade_v : e->ade_c;
-                    if (!e->ade_apply || !as.live()) continue;
+                    if (!e->ade_apply || !as.live() || (side == 0 && e->ade_adopt)) continue;
                     const uint32_t thr = as.app_runs ? (as.app_n + ADE_V - 1) / ADE_V : as.app_n;
                     (side == 0 ? vpv : vpc).push_back({thr, OpAdeApply{side == 0 ? V1 : C1, e->ade_apply_dev(as), as.app_runs ? 1u : 0u}});
                 }
@@ -372,6 +383,8 @@ struct efs_batch {
                 }
             }
             upload_raw(members[s], bm.data(), bm.size() * sizeof(BatchMember));
+            build_seg(ade_adopt_i[s], vai);
+            build_seg(ade_adopt_d[s], vad);
             build_seg(mur_adopt_i[s], vmi);
             build_seg(mur_adopt_d[s], vmd);
             build_seg(mur_pre[s], mpre);
@@ -432,6 +445,8 @@ struct efs_batch {
         launch_seg<OpPmlE<true>>(pml_e_i[s], k);  // UPML E (the pre-update reads of UPML cells are redirected
         launch_seg<OpPmlE<false>>(pml_e_d[s], k); // to the old flux, which this pass does not write)
         mark(1);
+        launch_seg<OpAdeAdopt<true>>(ade_adopt_i[s], k);
+        launch_seg<OpAdeAdopt<false>>(ade_adopt_d[s], k);
         launch_seg<OpAde>(ade_v[s], k);          // pre-voltage, as the single engine: ADE(volt), Mur pre
         launch_seg<OpMurAdopt<true>>(mur_adopt_i[s], k);
         launch_seg<OpMurAdopt<false>>(mur_adopt_d[s], k);

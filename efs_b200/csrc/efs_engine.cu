@@ -37,6 +37,7 @@
 #include <cudaTypedefs.h>
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -337,12 +338,16 @@ struct efs_engine {
         bool live() const { return n && !(zero && clean); }
     };
     AdeSide ade_v, ade_c;
+    bool ade_adopt = false;      // plan: the voltage side runs as k_ade_adopt
+    uint32_t ade_nruns = 0;      // runs of the voltage side (without the sentinel)
+    void plan_ade_adopt();
     bool ade_apply = false;      // opt-in: subtract the ADE state from E / H after the update (no reference counterpart)
 
     // RLC
     bool rlc_on = false;
     DevBuf rlc_gtarget, rlc_goff, rlc_type, rlc_p, rlc_vdn, rlc_jn, rlc_vil;
     uint32_t rlc_n = 0, rlc_groups = 0;
+    std::vector<uint32_t> h_rlc_targets;   // every element's field location
     std::vector<uint32_t> rlc_perm;   // device element order -> caller's element order
     std::vector<uint32_t> mur_perm;   // device Mur entry order -> caller's entry order
 
@@ -587,8 +592,6 @@ struct efs_engine {
         }
         plan_tfsf_faces();
         plan_mur();
-        build_deferred();
-        mark_adopted();
         for (AdeSide* s : {&ade_v, &ade_c}) {
             if (!s->n) continue;
             std::vector<AdeRun> runs;
@@ -611,11 +614,15 @@ struct efs_engine {
                 for (size_t k = r; k < runs.size() && runs[k].entry < i1; ++k) lor |= runs[k].coef & 0x80000000u;
                 qr[q] = (uint32_t)r | lor;
             }
+            if (s == &ade_v) ade_nruns = (uint32_t)runs.size();
             runs.push_back(AdeRun{s->n, 0, 0, 0});      // sentinel: ends the last run
             upload(s->runs, runs);
             upload(s->grp_run, qr);
             if (ade_apply) build_ade_apply(*s);
         }
+        plan_ade_adopt();
+        build_deferred();
+        mark_adopted();
         plan_dirty = false;
         ++plan_gen;
     }
@@ -695,7 +702,7 @@ struct efs_engine {
         if (exc_on) add(h_exc_targets);
         if (mur_gen) add(h_mur_gen_apply);
         if (rlc_on) add(h_rlc_series);
-        if (ade_apply && ade_v.live()) add(ade_v.h_field);
+        if (ade_apply && ade_v.live() && !ade_adopt) add(ade_v.h_field);
         const uint32_t nl[3] = {Nx, Ny, Nz};
         if (pbc_on)
             for (auto& a : pbc_axes) {
@@ -817,7 +824,8 @@ struct efs_engine {
             launch_pml_e(p);
         }
         mark(1);
-        if (ade_v.live()) launch_k(false, k_ade, blocks(ade_v.n, ADE_BLOCK), ADE_T, 0, stream, V, ade_dev(ade_v, vfl));
+        if (ade_adopt) launch_ade_adopt(p, vfl);
+        else if (ade_v.live()) launch_k(false, k_ade, blocks(ade_v.n, ADE_BLOCK), ADE_T, 0, stream, V, ade_dev(ade_v, vfl));
         MurDev md = mur_dev(vfl);
         if (mur_fast) launch_mur_adopt(p);
         if (mur_gen) launch_k(false, k_mur_pre, blocks(mur_gen, T), T, 0, stream, V, md);
@@ -843,7 +851,7 @@ struct efs_engine {
         }
         if (mur_gen) launch_k(false, k_mur_apply, blocks(mur_napply, T), T, 0, stream, V1, md);
         if (rlc_on) launch_k(false, k_rlc_apply, blocks(rlc_groups, T), T, 0, stream, V1, rd);
-        if (ade_apply && ade_v.live()) launch_ade_apply(ade_v, V1);
+        if (ade_apply && ade_v.live() && !ade_adopt) launch_ade_apply(ade_v, V1);
         mark(4);
         // --- H of the UPML cells and of the cells next to those E writes ---
         if (sweep) {
@@ -897,11 +905,16 @@ struct efs_engine {
         if (indexed) launch_k(early, early ? k_mur_adopt<true, true> : k_mur_adopt<true, false>, nb, T, 0, stream, fused_grid(p), vbuf(p), mur_adopt_dev());
         else launch_k(early, early ? k_mur_adopt<false, true> : k_mur_adopt<false, false>, nb, T, 0, stream, fused_grid(p), vbuf(p), mur_adopt_dev());
     }
-    // The adopt bits of the material index: UPML cells and the Mur targets of
-    // k_mur_adopt.  A dense engine gets an array for them when it has any.
+    void launch_ade_adopt(int p, const float* const* vfl) {
+        const uint32_t T = 256, nb = blocks(ade_v.n, T);
+        if (indexed) launch_k(false, k_ade_adopt<true>, nb, T, 0, stream, fused_grid(p), vbuf(p), ade_dev(ade_v, vfl));
+        else launch_k(false, k_ade_adopt<false>, nb, T, 0, stream, fused_grid(p), vbuf(p), ade_dev(ade_v, vfl));
+    }
+    // The adopt bits of the material index: UPML cells, the Mur targets of
+    // k_mur_adopt and the ADE cells of k_ade_adopt.  A dense engine gets an array for them when it has any.
     void mark_adopted() {
         if (!mat.p) {
-            if (pml.empty() && !mur_fast) return;
+            if (pml.empty() && !mur_fast && !ade_adopt) return;
             alloc(mat, Nd * 4, true, FIELD_SHIFT);
         } else {
             k_mat_clear<<<(unsigned)std::min<size_t>(blocks(Nd, 256), 148 * 16), 256, 0, stream>>>(mat.as<uint32_t>(), Nd);
@@ -913,6 +926,8 @@ struct efs_engine {
                                                                   R->n[2], cells);
         }
         if (mur_fast) k_mat_mur<<<blocks(mur_n, 256), 256, 0, stream>>>(mat.as<uint32_t>(), (uint32_t)Nd, mur_adopt_dev());
+        if (ade_adopt)
+            k_mat_ade<<<blocks(ade_nruns, 8), 256, 0, stream>>>(mat.as<uint32_t>(), (uint32_t)Nd, ade_v.runs.as<AdeRun>(), ade_nruns);
         ck(cudaGetLastError(), "adopt bits");
     }
     void launch_deferred(int p) {
@@ -1755,6 +1770,42 @@ void efs_engine::plan_mur() {
     }
 }
 
+// The voltage side's state and apply steps run ahead of the core update when
+// every entry has a cell of its own and nothing comes between the core update
+// and the apply step there (no UPML, TFSF, Mur cell, excitation, lumped element
+// or periodic axis), nor reads the cell's E_old after them (Mur).
+void efs_engine::plan_ade_adopt() {
+    ade_adopt = false;
+    if (!ade_apply || !ade_v.live() || !ade_v.app_runs || pbc_on) return;
+    const size_t words = (3 * Nd + 31) / 32;
+    std::unique_ptr<uint32_t, decltype(&free)> B((uint32_t*)calloc(words, 4), &free);
+    if (!B) fail(EFS_ERR_OOM, "ADE plan: out of host memory");
+    uint32_t* b = B.get();
+    auto mark = [&](const uint32_t* p, size_t n) {
+        parallel_chunks(n, host_threads(n), [&](unsigned, size_t lo, size_t hi) {
+            for (size_t i = lo; i < hi; ++i) __atomic_fetch_or(&b[p[i] >> 5], 1u << (p[i] & 31), __ATOMIC_RELAXED);
+        });
+    };
+    if (tfsf_on)
+        parallel_chunks(h_tfsf_v.size(), host_threads(h_tfsf_v.size()), [&](unsigned, size_t lo, size_t hi) {
+            for (size_t i = lo; i < hi; ++i) {
+                const uint32_t f = dev_index(h_tfsf_v[i].field_idx);
+                __atomic_fetch_or(&b[f >> 5], 1u << (f & 31), __ATOMIC_RELAXED);
+            }
+        });
+    if (exc_on) mark(h_exc_targets.data(), h_exc_targets.size());
+    if (rlc_on) mark(h_rlc_targets.data(), h_rlc_targets.size());
+    if (mur_on) { mark(h_mur_normal.data(), mur_n); mark(h_mur_shifted.data(), mur_n); }
+    const std::vector<uint32_t>& f = ade_v.h_field;
+    std::atomic<bool> ok{true};
+    parallel_chunks(f.size(), host_threads(f.size()), [&](unsigned, size_t lo, size_t hi) {
+        bool good = true;
+        for (size_t i = lo; i < hi && good; ++i) good = !((b[f[i] >> 5] >> (f[i] & 31)) & 1u) && redirect(f[i]).sel == 0;
+        if (!good) ok = false;
+    });
+    ade_adopt = ok;
+}
+
 efs_status efs_configure_tfsf(efs_engine* e, const float* signal, uint32_t L, uint32_t period, const efs_tfsf_point* vp,
                               uint32_t nv, const efs_tfsf_point* cp, uint32_t nc) {
     return guard(e, [&] {
@@ -1860,6 +1911,7 @@ efs_status efs_configure_rlc(efs_engine* e, uint32_t n, const efs_rlc_element* e
         for (uint32_t i = 0; i < n; ++i) { type2[i] = type[perm[i]]; memcpy(&p2[9 * (size_t)i], &p[9 * (size_t)perm[i]], 36); }
         e->upload(e->rlc_gtarget, ut); e->upload(e->rlc_goff, goff);
         e->h_rlc_series.clear();
+        e->h_rlc_targets = tgt;
         for (uint32_t i = 0; i < n; ++i) if (el[i].type_flag == 1) e->h_rlc_series.push_back(tgt[i]);
         e->upload(e->rlc_type, type2); e->upload(e->rlc_p, p2);
         e->alloc(e->rlc_vdn, 3 * (size_t)n * 4); e->alloc(e->rlc_jn, 3 * (size_t)n * 4); e->alloc(e->rlc_vil, (size_t)n * 4);
@@ -2522,7 +2574,7 @@ efs_status efs_kernels_per_step(efs_engine* e, uint32_t* out) {
         // E and H sweeps, the TFSF faces added after the first
         uint32_t k = sweep ? 2 + (e->tf_n > 0) : 1 + split + ((e->defer_n > 0) || split);
         k += e->ss_on + e->ade_v.live() + e->ade_c.live() + e->mur_fast + 3 * (e->mur_gen > 0) + 2 * e->rlc_on;
-        if (e->ade_apply) k += e->ade_v.live() + e->ade_c.live();
+        if (e->ade_apply) k += (e->ade_v.live() && !e->ade_adopt) + e->ade_c.live();
         k += (e->tfsf_on && e->tfsf_v.groups) + (e->tfsf_on && e->tfsf_c.groups) + (e->exc_on && e->exc_groups > 0);
         k += e->pbc_on ? 2 * (uint32_t)e->pbc_axes.size() : 0;
         k += (e->nf_on && !(e->nf_pair && split)) + e->ring_on;   // paired samples ride on the UPML E pass

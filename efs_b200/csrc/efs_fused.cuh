@@ -29,8 +29,8 @@ constexpr int PML_MAX_OVERLAP = 4;
 // The material index of a cell carries, in its top three bits, the E components
 // (bit 29 + n) whose E_new is known before the core update and stands in place
 // of E_old in the step's old-E buffer: the core update adopts it as is.  These
-// are all components of UPML cells (k_pml_e) and the Mur targets that
-// k_mur_adopt computes.  With dense coefficients the array holds these bits alone.
+// are all components of UPML cells (k_pml_e), the Mur targets that k_mur_adopt
+// computes and the applied ADE values that k_ade_adopt computes.  With dense coefficients the array holds these bits alone.
 constexpr uint32_t MAT_BITS = 29, MAT_MASK = (1u << MAT_BITS) - 1u;
 
 struct FusedGrid {
@@ -118,7 +118,30 @@ __device__ __forceinline__ void coeffs_f(const FusedGrid& g, size_t c, uint32_t 
     }
 }
 
-// Adopt bits of the material index (one launch per UPML region; Mur targets).
+// E_new of one field value from the old fields: the core update of component n
+// at a cell (v: its old value), with the neighbours at index 0 the cell itself.
+template <bool IDX>
+__device__ __forceinline__ float core_e(const FusedGrid& g, uint32_t f, float v) {
+    const uint32_t N = (uint32_t)g.N, NyNz = (uint32_t)g.NyNz, Pz = g.Pz;
+    const uint32_t n = f / N, cell = f - n * N, x = cell / NyNz, r = cell - x * NyNz, y = r / Pz, z = r - y * Pz;
+    const uint32_t p = n == 2 ? 0u : n + 1u, q = p == 2 ? 0u : p + 1u;       // E_n: H_q along p, H_p along q
+    const uint32_t dp = p == 0 ? (x ? NyNz : 0u) : p == 1 ? (y ? Pz : 0u) : (z ? 1u : 0u);
+    const uint32_t dq = q == 0 ? (x ? NyNz : 0u) : q == 1 ? (y ? Pz : 0u) : (z ? 1u : 0u);
+    const float *Hq = g.H0 + q * N + cell, *Hp = g.H0 + p * N + cell;
+    const float curl = curl4(Hq[0], *(Hq - dp), Hp[0], *(Hp - dq));
+    float cv, ci;
+    if (IDX) {
+        const float* row = g.table + (size_t)(g.mat[cell] & MAT_MASK) * 12;
+        cv = __ldg(row + n);
+        ci = __ldg(row + 3 + n);
+    } else {
+        cv = __ldg(g.vv + f);
+        ci = __ldg(g.vi + f);
+    }
+    return upd(v, cv, ci, curl);
+}
+
+// Adopt bits of the material index (one launch per UPML region; Mur targets; ADE cells).
 __global__ void k_mat_clear(uint32_t* mat, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) mat[i] &= MAT_MASK;
 }
@@ -157,25 +180,9 @@ struct MurAdoptDev {
 };
 template <bool IDX>
 __device__ __forceinline__ float mur_value(const FusedGrid& g, const float* V, const MurAdoptDev& d, uint32_t i) {
-    const uint32_t N = (uint32_t)g.N, NyNz = (uint32_t)g.NyNz, Pz = g.Pz;
     const uint32_t t = d.target[i], s = d.shifted[i];
     const float c = d.coeff[i], vt = V[t], vs = V[s];
-    const uint32_t n = s / N, cell = s - n * N, x = cell / NyNz, r = cell - x * NyNz, y = r / Pz, z = r - y * Pz;
-    const uint32_t p = n == 2 ? 0u : n + 1u, q = p == 2 ? 0u : p + 1u;       // E_n: H_q along p, H_p along q
-    const uint32_t dp = p == 0 ? (x ? NyNz : 0u) : p == 1 ? (y ? Pz : 0u) : (z ? 1u : 0u);   // self at index 0
-    const uint32_t dq = q == 0 ? (x ? NyNz : 0u) : q == 1 ? (y ? Pz : 0u) : (z ? 1u : 0u);
-    const float *Hq = g.H0 + q * N + cell, *Hp = g.H0 + p * N + cell;
-    const float curl = curl4(Hq[0], *(Hq - dp), Hp[0], *(Hp - dq));
-    float cv, ci;
-    if (IDX) {
-        const float* row = g.table + (size_t)(g.mat[cell] & MAT_MASK) * 12;
-        cv = __ldg(row + n);
-        ci = __ldg(row + 3 + n);
-    } else {
-        cv = __ldg(g.vv + s);
-        ci = __ldg(g.vi + s);
-    }
-    return __fadd_rn(__fsub_rn(vs, __fmul_rn(c, vt)), __fmul_rn(c, upd(vs, cv, ci, curl)));
+    return __fadd_rn(__fsub_rn(vs, __fmul_rn(c, vt)), __fmul_rn(c, core_e<IDX>(g, s, vs)));
 }
 template <bool IDX>
 __device__ __forceinline__ void mur_adopt_body(const FusedGrid& g, float* V, const MurAdoptDev& d, uint32_t i) {
@@ -199,6 +206,45 @@ __global__ void __launch_bounds__(256) k_mur_adopt(const FusedGrid g, float* V, 
 __global__ void k_mat_mur(uint32_t* mat, uint32_t N, const MurAdoptDev d) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < d.n && d.kind[i] & MUR_LAST) atomicOr(mat + d.target[i] % N, 1u << (MAT_BITS + d.target[i] / N));
+}
+
+// ADE state update and apply step of the voltage side ahead of the core update:
+// an entry's new state follows from E_old, and what the apply step leaves at
+// its cell, E_new - state, from that and the old fields, so one kernel computes
+// both, writes the value over E_old and the core update adopts it.  It replaces
+// the state pass, the apply pass and the second H update of every cell next to
+// an entry (in a medium, of the whole medium).  Used when every entry has its
+// own cell and nothing else acts on those cells (plan_ade_adopt).
+//
+// One entry per thread: an entry's loads are coalesced along its run.
+// Bound by DRAM and its loads' latency.  200x200x100 with 1.6 M entries: the
+// state and apply passes and their deferred H, 21 + 16 + 9 us a step, became 26;
+// the step 159 -> 143 us.
+template <bool IDX>
+__device__ __forceinline__ void ade_adopt_body(const FusedGrid& g, float* V, const AdeDev& a, uint32_t i) {
+    if (i >= a.n) return;
+    const float st = a.state[i];
+    uint32_t r = __ldg(a.grp_run + i / ADE_V) & 0x7fffffffu;
+    AdeRun run = a.runs[r];
+    for (uint32_t next = a.runs[r + 1].entry; i >= next; next = a.runs[r + 1].entry) run = a.runs[++r];
+    const uint32_t f = run.idx + (i - run.entry);
+    const float v = V[f];
+    float l = run.coef >> 31 ? a.lor[i] : 0.f;
+    const float en = core_e<IDX>(g, f, v);
+    const float s = ade_one(v, st, l, run.coef, a.coef[run.coef & 0x7fffffffu]);
+    a.state[i] = s;
+    if (run.coef >> 31) a.lor[i] = l;
+    V[f] = __fsub_rn(en, s);
+}
+template <bool IDX>
+__global__ void __launch_bounds__(256) k_ade_adopt(const FusedGrid g, float* V, const AdeDev a) {
+    ade_adopt_body<IDX>(g, V, a, blockIdx.x * blockDim.x + threadIdx.x);
+}
+__global__ void k_mat_ade(uint32_t* mat, uint32_t N, const AdeRun* runs, uint32_t nruns) {
+    const uint32_t r = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;      // a warp per run
+    if (r >= nruns) return;
+    const uint32_t cnt = runs[r + 1].entry - runs[r].entry, f = runs[r].idx, n = f / N;
+    for (uint32_t k = threadIdx.x % 32; k < cnt; k += 32) atomicOr(mat + (f + k - n * N), 1u << (MAT_BITS + n));
 }
 
 // H update of the deferred cells, after the E-side sparse operations: reads
