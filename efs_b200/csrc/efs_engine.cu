@@ -621,6 +621,7 @@ struct efs_engine {
             if (ade_apply) build_ade_apply(*s);
         }
         plan_ade_adopt();
+        plan_ring();
         build_deferred();
         mark_adopted();
         plan_dirty = false;
@@ -836,17 +837,21 @@ struct efs_engine {
         if (ade_c.live()) launch_k(false, k_ade, blocks(ade_c.n, ADE_BLOCK), ADE_T, 0, stream, C, ade_dev(ade_c, cfl));
         if (tf_n && !sweep) launch_k(false, k_tfsf_face, blocks(tf_n, T), T, 0, stream, st, k, tf_dev());   // TFSF face values of this step
         mark(2);
-        if (sweep) launch_sweep(p, true);
-        else launch_fused_tma(p);
+        const bool exc_rides = sweep && exc_may_ride();
+        if (sweep) {
+            launch_sweep_e(p, k, exc_rides);
+            ring_held = false;
+        } else {
+            launch_fused_tma(p);
+        }
         mark(3);
         // --- post-voltage / apply (on the updated E) ---
         if (tf_n && sweep) launch_k(false, k_tfsf_face_points, blocks(tf_n, T), T, 0, stream, V1, st, k, tf_dev());
         if (tfsf_on && tfsf_v.groups) launch_k(early, early ? k_point_sources<1, true> : k_point_sources<1, false>, blocks(tfsf_v.groups, T), T, 0, stream, V1, st, k, point_dev(tfsf_v, tfsf_signal, tfsf_len, tfsf_period));
         if (pbc_on) for (auto& a : pbc_axes) launch_pbc(a, true, V1);
         if (mur_gen) launch_k(false, k_mur_post, blocks(mur_gen, T), T, 0, stream, V1, md);
-        if (exc_on && exc_groups) {
-            PointSources s{exc_groups, exc_target.as<uint32_t>(), exc_off.as<uint32_t>(), exc_delay.as<uint32_t>(),
-                           exc_amp.as<float>(), nullptr, exc_signal.as<float>(), exc_len, exc_period};
+        if (exc_on && exc_groups && !exc_rides) {
+            const PointSources s = exc_dev();
             launch_k(early, early ? k_point_sources<0, true> : k_point_sources<0, false>, blocks(exc_groups, T), T, 0, stream, V1, st, k, s);
         }
         if (mur_gen) launch_k(false, k_mur_apply, blocks(mur_napply, T), T, 0, stream, V1, md);
@@ -855,7 +860,7 @@ struct efs_engine {
         mark(4);
         // --- H of the UPML cells and of the cells next to those E writes ---
         if (sweep) {
-            launch_sweep(p, false);
+            launch_sweep_h(p);
         } else if (split && defer_n) {
             const uint32_t na = blocks(pml_items(), T), nb = blocks(defer_n, T);
             if (indexed) pair(pml_h_pass<true>(p), na, deferred_pass<true>(p), nb);
@@ -880,11 +885,35 @@ struct efs_engine {
                 if (j == NF_K - 1 || last) launch_k(false, k_nf2ff_flush, blocks(nf.np, T), T, 0, stream, st, k - j, j + 1, nf);
             }
         }
-        if (ring_on) launch_k(early, early ? k_gather_ring<true> : k_gather_ring<false>, blocks(ring_n, 64), 64, 0, stream, V1, C1, st, k, ring_dev());
+        if (ring_on && sweep && ring_rides && !last) ring_held = true;   // sampled beside the next step's E sweep
+        else if (ring_on) launch_k(early, early ? k_gather_ring<true> : k_gather_ring<false>, blocks(ring_n, 64), 64, 0, stream, V1, C1, st, k, ring_dev());
         mark(7);
     }
     struct NfHeld { bool on; uint32_t j; };
     NfHeld nf_held{false, 0};     // capture: NF2FF samples of the previous step not yet issued
+    bool ring_held = false;       // and its probe ring samples
+    bool ring_rides = false;      // plan: nothing rewrites a probed E between a step's end and the next E sweep
+    std::vector<uint32_t> h_ring; // probed field indices (device order)
+    // A step's samples may wait for the next E sweep when no probed E is a target
+    // that k_mur_adopt or k_ade_adopt puts into the old fields ahead of it.
+    void plan_ring() {
+        ring_rides = ring_on;
+        if (mur_fast)                                    // targets k_mur_adopt writes ahead of the sweep (ascending)
+            for (uint32_t f : h_ring) ring_rides = ring_rides && !std::binary_search(h_mur_normal.begin(), h_mur_normal.end(), f);
+        if (ade_adopt && ring_rides) {
+            std::vector<uint32_t> probed(h_ring);
+            std::sort(probed.begin(), probed.end());
+            for (uint32_t f : ade_v.h_field) ring_rides = ring_rides && !std::binary_search(probed.begin(), probed.end(), f);
+        }
+    }
+    PointSources exc_dev() const {
+        return PointSources{exc_groups, exc_target.as<uint32_t>(), exc_off.as<uint32_t>(), exc_delay.as<uint32_t>(),
+                            exc_amp.as<float>(), nullptr, exc_signal.as<float>(), exc_len, exc_period};
+    }
+    // nothing acts on the new E before the excitation, and a block has a thread for every target
+    bool exc_may_ride() const {
+        return exc_on && exc_groups && exc_groups <= SW_EXC && !(tfsf_on && tfsf_v.groups) && !tf_n && !pbc_on && !mur_gen;
+    }
     bool nf_pair = false;         // plan: no NF2FF sample reads a UPML cell
     // passes of the paired launches (k_pair, 256-thread blocks)
     template <bool IDX> PassPmlE<IDX> pml_e_pass(int p) const {
@@ -943,7 +972,7 @@ struct efs_engine {
         build_plan();
         std::vector<cudaEvent_t> ev((size_t)steps * (EFS_PHASES + 1));
         for (auto& x : ev) ck(cudaEventCreate(&x), "event");
-        nf_held.on = false;
+        nf_held.on = ring_held = false;
         try {
             int q = cur;
             for (uint32_t k = 0; k < steps; ++k) {
@@ -1036,18 +1065,33 @@ struct efs_engine {
     // 20.0 / 19.7; 256^3 287 / 253, 16 members batched 205 / 149).
     bool early = false;              // of the step being enqueued
     bool use_sweep() const { return !xchunk && skip_plane == ~0u && (!indexed || Nd * 52 <= SWEEP_BYTES); }
+    uint32_t sweep_blocks() const { return Nx * sweep_plane_blocks(Ny, Pz); }
+    // E sweep of step k, with the excitation and the probe ring samples of step k-1 (ring_held) riding
     template <bool IDX, bool PML>
-    void launch_sweep_k(int p, bool volt) {
-        const FusedGrid fg = fused_grid(p);
-        const PmlSet ps = pml_set(p), pn = pml_set(1 - p);
-        const uint32_t nb = Nx * sweep_plane_blocks(Ny, Pz);
-        if (volt) launch_k(early, k_sweep_e<IDX, PML>, nb, SW_T, 0, stream, fg, ps, pn);
-        else launch_k(early, k_sweep_h<IDX, PML>, nb, SW_T, 0, stream, fg, ps, pn);
+    void launch_sweep_e_k(int p, const SweepRiders& rd) {
+        launch_k(early, k_sweep_e<IDX, PML>, rd.nb + blocks(rd.ring.G, SW_T), SW_T, 0, stream, fused_grid(p), pml_set(p), pml_set(1 - p), rd);
     }
-    void launch_sweep(int p, bool volt) {
+    void launch_sweep_e(int p, uint32_t k, bool exc) {
+        SweepRiders rd;
+        memset(&rd, 0, sizeof(rd));
+        rd.st = state.as<StepState>();
+        rd.k = k;
+        rd.ring_k = k - 1;
+        rd.nb = sweep_blocks();
+        if (exc) rd.exc = exc_dev();
+        if (ring_held) rd.ring = ring_dev();
         const bool hp = !pml.empty();
-        if (indexed) { if (hp) launch_sweep_k<true, true>(p, volt); else launch_sweep_k<true, false>(p, volt); }
-        else { if (hp) launch_sweep_k<false, true>(p, volt); else launch_sweep_k<false, false>(p, volt); }
+        if (indexed) { if (hp) launch_sweep_e_k<true, true>(p, rd); else launch_sweep_e_k<true, false>(p, rd); }
+        else { if (hp) launch_sweep_e_k<false, true>(p, rd); else launch_sweep_e_k<false, false>(p, rd); }
+    }
+    template <bool IDX, bool PML>
+    void launch_sweep_h_k(int p) {
+        launch_k(early, k_sweep_h<IDX, PML>, sweep_blocks(), SW_T, 0, stream, fused_grid(p), pml_set(p), pml_set(1 - p));
+    }
+    void launch_sweep_h(int p) {
+        const bool hp = !pml.empty();
+        if (indexed) { if (hp) launch_sweep_h_k<true, true>(p); else launch_sweep_h_k<true, false>(p); }
+        else { if (hp) launch_sweep_h_k<false, true>(p); else launch_sweep_h_k<false, false>(p); }
     }
     // UPML cells are updated by k_pml_e / k_pml_h around the fused kernel
     bool pml_split() const { return !pml.empty(); }
@@ -1125,7 +1169,7 @@ struct efs_engine {
         if (graphs.size() > 12) drop_graphs();
         cudaGraph_t graph;
         ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "BeginCapture");
-        nf_held.on = false;
+        nf_held.on = ring_held = false;
         try {
             int q = p;
             for (uint32_t k = 0; k < m; ++k) { enqueue_step(k, q, k + 1 == m); q = pnext(q); }
@@ -1192,7 +1236,7 @@ void alloc_fields(efs_engine* e, const uint32_t dims[3]) {
     e->ade_apply = false;
     e->gd_n = 0;
     e->Nx = dims[0]; e->Ny = dims[1]; e->Nz = dims[2]; e->N = N; e->Pz = Pz; e->Nd = Nd;
-    e->h_exc_targets.clear(); e->h_tfsf_v_targets.clear(); e->h_rlc_series.clear();
+    e->h_exc_targets.clear(); e->h_tfsf_v_targets.clear(); e->h_rlc_series.clear(); e->h_ring.clear();
     e->h_tfsf_v.clear();
     e->tf = TfsfFace{0, {0, 0}};
     e->tf_n = 0;
@@ -1910,7 +1954,7 @@ efs_status efs_configure_rlc(efs_engine* e, uint32_t n, const efs_rlc_element* e
         std::vector<float> p2(9 * (size_t)n);
         for (uint32_t i = 0; i < n; ++i) { type2[i] = type[perm[i]]; memcpy(&p2[9 * (size_t)i], &p[9 * (size_t)perm[i]], 36); }
         e->upload(e->rlc_gtarget, ut); e->upload(e->rlc_goff, goff);
-        e->h_rlc_series.clear();
+        e->h_rlc_series.clear(); e->h_ring.clear();
         e->h_rlc_targets = tgt;
         for (uint32_t i = 0; i < n; ++i) if (el[i].type_flag == 1) e->h_rlc_series.push_back(tgt[i]);
         e->upload(e->rlc_type, type2); e->upload(e->rlc_p, p2);
@@ -2058,6 +2102,7 @@ efs_status efs_configure_probe_gather_buffered(efs_engine* e, const uint32_t* id
         std::vector<uint32_t> di(n);
         for (uint32_t i = 0; i < n; ++i) di[i] = e->dev_index(idx[i]);
         e->upload(e->ring_idx, di);
+        e->h_ring = di;
         e->alloc(e->ring, (size_t)maxS * n * 2 * 4);
         e->ring_n = n; e->ring_max = maxS; e->ring_interval = interval;
         e->ring_q0 = e->numTS / interval;    // multiples already passed at configure time
@@ -2542,8 +2587,9 @@ efs_status efs_time_core(efs_engine* e, uint32_t reps, float* ms) {
         };
         const int p = e->cur;
         const bool sweep = e->use_sweep();
+        e->ring_held = false;
         const float a = timed([&] {
-            if (sweep) { e->launch_sweep(p, true); e->launch_sweep(p, false); }
+            if (sweep) { e->launch_sweep_e(p, 0, false); e->launch_sweep_h(p); }
             else e->launch_fused_tma(p);
         });
         const float b = e->pml_split() && !sweep ? timed([&] { e->launch_pml_e(p); }) + timed([&] { e->launch_pml_h(p); }) : 0.f;
@@ -2575,9 +2621,9 @@ efs_status efs_kernels_per_step(efs_engine* e, uint32_t* out) {
         uint32_t k = sweep ? 2 + (e->tf_n > 0) : 1 + split + ((e->defer_n > 0) || split);
         k += e->ss_on + e->ade_v.live() + e->ade_c.live() + e->mur_fast + 3 * (e->mur_gen > 0) + 2 * e->rlc_on;
         if (e->ade_apply) k += (e->ade_v.live() && !e->ade_adopt) + e->ade_c.live();
-        k += (e->tfsf_on && e->tfsf_v.groups) + (e->tfsf_on && e->tfsf_c.groups) + (e->exc_on && e->exc_groups > 0);
+        k += (e->tfsf_on && e->tfsf_v.groups) + (e->tfsf_on && e->tfsf_c.groups) + (e->exc_on && e->exc_groups > 0 && !(sweep && e->exc_may_ride()));
         k += e->pbc_on ? 2 * (uint32_t)e->pbc_axes.size() : 0;
-        k += (e->nf_on && !(e->nf_pair && split)) + e->ring_on;   // paired samples ride on the UPML E pass
+        k += (e->nf_on && !(e->nf_pair && split)) + (e->ring_on && !(sweep && e->ring_rides));   // riders of other launches are not counted
         *out = k;
     });
 }

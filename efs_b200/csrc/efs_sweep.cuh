@@ -171,10 +171,40 @@ __device__ __forceinline__ void sweep_h_body(const FusedGrid& g, const PmlSet& p
     sweep_store(g.H1, N, c, q.both, hn);
 }
 
+// What rides on the E sweep's launch instead of a launch of its own (a small
+// grid's step is launches; a step of 26x11x32 fell from 5.9 to 4.7 us, 81^3 with
+// Mur from 13.0 to 11.8, 86x87x71 with UPML from 19.6 to 16.7, 121x109x97 with
+// dense coefficients from 26.8 to 25.8, each with a port and a probe ring):
+//  * the excitation (exc.ngroups > 0), when it is the first operation on the new
+//    E: the block that wrote a target's cell adds to it, after its stores;
+//  * the probe ring's samples of the step before, whose fields are this step's
+//    inputs: blocks behind the sweep's own (ring_k: that step; ring.G == 0: none).
+struct SweepRiders {
+    const StepState* st;
+    uint32_t k, ring_k, nb;                               // step; step sampled; blocks of the sweep itself
+    PointSources exc;
+    RingDev ring;
+};
+constexpr uint32_t SW_EXC = SW_T;                         // most excitation targets that ride (a thread each)
+
 template <bool IDX, bool PML>
-__global__ void __launch_bounds__(SW_T, 4) k_sweep_e(const FusedGrid g, const PmlSet ps, const PmlSet pn) {
+__global__ void __launch_bounds__(SW_T, 4) k_sweep_e(const FusedGrid g, const PmlSet ps, const PmlSet pn, const SweepRiders rd) {
     if (!PML) step_begin();
-    sweep_e_body<IDX, PML>(g, ps, pn, blockIdx.x);
+    const uint32_t blk = blockIdx.x;
+    if (blk >= rd.nb) {
+        gather_ring_body(g.V0, g.H0, rd.st, rd.ring_k, rd.ring, (blk - rd.nb) * SW_T + threadIdx.x);
+        return;
+    }
+    sweep_e_body<IDX, PML>(g, ps, pn, blk);
+    if (rd.exc.ngroups) {
+        const uint32_t bpp = sweep_plane_blocks(g.Ny, g.Pz), x = blk / bpp, first = (blk - x * bpp) * 2 * SW_T;
+        bool mine = false;                                // the thread's target lies in the block's run of cells
+        if (threadIdx.x < rd.exc.ngroups) {
+            const uint32_t cell = rd.exc.target[threadIdx.x] % (uint32_t)g.N, off = cell - x * (uint32_t)g.NyNz;
+            mine = cell >= x * (uint32_t)g.NyNz && off < (uint32_t)g.NyNz && off - first < 2 * SW_T && off >= first;
+        }
+        if (__syncthreads_or(mine) && mine) point_sources_body<0>(g.V1, rd.st, rd.k, rd.exc, threadIdx.x);
+    }
 }
 template <bool IDX, bool PML>
 __global__ void __launch_bounds__(SW_T, 4) k_sweep_h(const FusedGrid g, const PmlSet ps, const PmlSet pn) {
