@@ -63,6 +63,22 @@ __global__ void __launch_bounds__(256) k_seg(const Op* __restrict__ ops, SegMap 
     ops[s].run(blockIdx.x - sm.first[s], k, a, b);
 }
 
+// Segmented launches of several ops that are independent of one another, in one:
+// the first op's blocks come first.
+template <class Op> struct SegArg { const Op* ops; SegMap sm; uint32_t n, k, a, b; };
+template <class Op>
+__device__ __forceinline__ bool run_seg(const SegArg<Op>& s, uint32_t& blk) {
+    if (blk >= s.n) { blk -= s.n; return false; }
+    const uint32_t g = s.sm.seg[blk];
+    s.ops[g].run(blk - s.sm.first[g], s.k, s.a, s.b);
+    return true;
+}
+template <class... Ops>
+__global__ void __launch_bounds__(256) k_segs(SegArg<Ops>... s) {
+    uint32_t blk = blockIdx.x;
+    (void)(run_seg(s, blk) || ...);
+}
+
 template <bool IDX>
 struct OpMurAdopt {
     FusedGrid g; float* V; MurAdoptDev d;
@@ -189,6 +205,11 @@ struct efs_batch {
         ring[2], nf_sample[2], nf_flush[2],
         deferred_i[2], deferred_d[2], pml_e_i[2], pml_e_d[2], pml_h_i[2], pml_h_d[2], tfsf_face[2], advance;   // _i / _d: index / dense members
     bool any_nf = false;
+    bool any_pml = false;
+    bool mur_first = false;                    // no UPML member, and no ADE pass to read E before k_mur_adopt writes its targets
+    uint32_t tails = 0;                        // operations every member may leave to the next step's first launch
+    bool pts_merge = false;                    // TFSF voltage points and the excitation act on different E, nothing between them
+    efs_engine::Held held;                     // and what the step just enqueued left
     std::map<uint32_t, cudaGraphExec_t> graphs;
 
     ~efs_batch() {
@@ -228,6 +249,16 @@ struct efs_batch {
     template <class Op>
     void launch_seg(const SegLaunch& L, uint32_t k, uint32_t a = 0, uint32_t b = 0) {
         if (L.blocks) launch_k(false, k_seg<Op>, L.blocks, SEG_T, 0, stream, L.ops.as<Op>(), L.map(), k, a, b);
+    }
+
+    template <class Op>
+    SegArg<Op> seg_arg(const SegLaunch& L, bool on, uint32_t k, uint32_t a = 0, uint32_t b = 0) const {
+        return SegArg<Op>{L.ops.as<Op>(), L.map(), on ? L.blocks : 0u, k, a, b};
+    }
+    template <class... Ops>
+    void launch_segs(const SegArg<Ops>&... s) {
+        const uint32_t n = (s.n + ...);
+        if (n) launch_k(false, k_segs<Ops...>, n, SEG_T, 0, stream, s...);
     }
 
     void check_members() {
@@ -278,7 +309,24 @@ struct efs_batch {
         gen.resize(E);
         for (size_t i = 0; i < E; ++i) { mem[i]->build_plan(); cur0[i] = mem[i]->cur; gen[i] = mem[i]->plan_gen; }
         phase = 0;
-        any_nf = false;
+        any_nf = any_pml = false;
+        for (const efs_engine* e : mem) any_pml |= e->pml_split();
+        mur_first = !any_pml;
+        for (const efs_engine* e : mem) mur_first &= !e->ade_v.live();
+        tails = efs_engine::TAIL_NF | efs_engine::TAIL_RING | efs_engine::TAIL_TC;
+        pts_merge = true;
+        for (const efs_engine* e : mem) {
+            const uint32_t has = (e->nf_on ? efs_engine::TAIL_NF : 0) | (e->ring_on ? efs_engine::TAIL_RING : 0) |
+                                 (e->tfsf_on && e->tfsf_c.groups ? efs_engine::TAIL_TC : 0);
+            if (has) tails &= e->tails_clear(mur_first) | ~has;
+            if (e->tfsf_on && e->tfsf_v.groups && e->mur_gen) pts_merge = false;
+            if (e->tfsf_on && e->tfsf_v.groups && e->exc_on) {
+                std::vector<uint32_t> t(e->h_tfsf_v_targets);
+                std::sort(t.begin(), t.end());
+                for (uint32_t f : e->h_exc_targets) pts_merge = pts_merge && !std::binary_search(t.begin(), t.end(), f);
+            }
+            if (e->exc_on && e->mur_gen) pts_merge = false;
+        }
         for (int s = 0; s < 2; ++s) {
             std::vector<BatchMember> bm(E);
             std::vector<std::pair<uint32_t, OpAdeAdopt<true>>> vai;
@@ -442,17 +490,28 @@ struct efs_batch {
     void enqueue_step(uint32_t k, int s, bool last, cudaEvent_t* marks = nullptr) {
         auto mark = [&](int i) { if (marks) ck(cudaEventRecord(marks[i], stream), "phase mark"); };
         mark(0);
-        launch_seg<OpPmlE<true>>(pml_e_i[s], k);  // UPML E (the pre-update reads of UPML cells are redirected
-        launch_seg<OpPmlE<false>>(pml_e_d[s], k); // to the old flux, which this pass does not write)
+        // UPML E (the pre-update reads of UPML cells are redirected to the old flux, which this pass does
+        // not write) or, with neither UPML nor ADE, Mur ahead of the core update, beside the face values
+        // of the core update and what step k-1 left: 16 members of 40-96 lines take 131 us a step, 148
+        // with a launch for each
+        const auto nfs = seg_arg<OpNfSample>(nf_sample[s ^ 1], held.nf, k - 1, held.j);
+        const auto tcs = seg_arg<OpPoints<1>>(tfsf_c[s ^ 1], held.tc, k - 1);
+        const auto rgs = seg_arg<OpRing>(ring[s ^ 1], held.ring, k - 1);
+        const auto tfs = seg_arg<OpTfsfFace>(tfsf_face[s], true, k);
+        if (any_pml) launch_segs(seg_arg<OpPmlE<true>>(pml_e_i[s], true, k), seg_arg<OpPmlE<false>>(pml_e_d[s], true, k), nfs, tcs, rgs, tfs);
+        else launch_segs(seg_arg<OpMurAdopt<true>>(mur_adopt_i[s], mur_first, k), seg_arg<OpMurAdopt<false>>(mur_adopt_d[s], mur_first, k), nfs, tcs, rgs, tfs);
+        if (held.nf && held.j == NF_K - 1) launch_seg<OpNfFlush>(nf_flush[s ^ 1], k, k - 1 - held.j, held.j + 1);
+        held = efs_engine::Held{};
         mark(1);
         launch_seg<OpAdeAdopt<true>>(ade_adopt_i[s], k);
         launch_seg<OpAdeAdopt<false>>(ade_adopt_d[s], k);
         launch_seg<OpAde>(ade_v[s], k);          // pre-voltage, as the single engine: ADE(volt), Mur pre
-        launch_seg<OpMurAdopt<true>>(mur_adopt_i[s], k);
-        launch_seg<OpMurAdopt<false>>(mur_adopt_d[s], k);
+        if (!mur_first) {
+            launch_seg<OpMurAdopt<true>>(mur_adopt_i[s], k);
+            launch_seg<OpMurAdopt<false>>(mur_adopt_d[s], k);
+        }
         launch_seg<OpMurPre>(mur_pre[s], k);
         launch_seg<OpAde>(ade_c[s], k);          // ADE(curr) before the core update rewrites H and the flux
-        launch_seg<OpTfsfFace>(tfsf_face[s], k); // TFSF face values the core update adds
         mark(2);
         const BatchMember* bm = members[s].as<BatchMember>();
         launch_tiles<true, true>(3, bm);
@@ -460,9 +519,13 @@ struct efs_batch {
         launch_tiles<false, true>(2, bm);
         launch_tiles<false, false>(0, bm);
         mark(3);
-        launch_seg<OpPoints<1>>(tfsf_v[s], k);
-        launch_seg<OpMurPost>(mur_post[s], k);
-        launch_seg<OpPoints<0>>(exc[s], k);
+        if (pts_merge) {
+            launch_segs(seg_arg<OpPoints<1>>(tfsf_v[s], true, k), seg_arg<OpPoints<0>>(exc[s], true, k));
+        } else {
+            launch_seg<OpPoints<1>>(tfsf_v[s], k);
+            launch_seg<OpMurPost>(mur_post[s], k);
+            launch_seg<OpPoints<0>>(exc[s], k);
+        }
         launch_seg<OpMurApply>(mur_apply[s], k);
         launch_seg<OpAdeApply>(ade_apply_v[s], k);
         mark(4);
@@ -471,15 +534,22 @@ struct efs_batch {
         launch_seg<OpDeferred<true>>(deferred_i[s], k);
         launch_seg<OpDeferred<false>>(deferred_d[s], k);
         mark(5);
-        launch_seg<OpPoints<1>>(tfsf_c[s], k);
+        if (!last && (tails & efs_engine::TAIL_TC)) held.tc = true;
+        else launch_seg<OpPoints<1>>(tfsf_c[s], k);
         launch_seg<OpAdeApply>(ade_apply_c[s], k);
         mark(6);
         if (any_nf) {
             const uint32_t j = k % NF_K;
-            launch_seg<OpNfSample>(nf_sample[s], k, j);
-            if (j == NF_K - 1 || last) launch_seg<OpNfFlush>(nf_flush[s], k, k - j, j + 1);
+            if (!last && (tails & efs_engine::TAIL_NF)) {
+                held.nf = true;
+                held.j = j;
+            } else {
+                launch_seg<OpNfSample>(nf_sample[s], k, j);
+                if (j == NF_K - 1 || last) launch_seg<OpNfFlush>(nf_flush[s], k, k - j, j + 1);
+            }
         }
-        launch_seg<OpRing>(ring[s], k);
+        if (!last && (tails & efs_engine::TAIL_RING)) held.ring = true;
+        else launch_seg<OpRing>(ring[s], k);
         mark(7);
     }
     // `steps` (<= 64) timesteps launched one kernel at a time with phase marks;
@@ -492,6 +562,7 @@ struct efs_batch {
         }
         std::vector<cudaEvent_t> ev((size_t)steps * (EFS_PHASES + 1));
         for (auto& x : ev) ck(cudaEventCreate(&x), "event");
+        held = efs_engine::Held{};
         try {
             for (uint32_t k = 0; k < steps; ++k)
                 enqueue_step(k, (int)((phase + k) & 1), k + 1 == steps, ev.data() + (size_t)k * (EFS_PHASES + 1));
@@ -526,6 +597,7 @@ struct efs_batch {
         if (graphs.size() > 12) drop_graphs();
         cudaGraph_t graph;
         ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "BeginCapture");
+        held = efs_engine::Held{};
         try {
             for (uint32_t k = 0; k < m; ++k) enqueue_step(k, (int)((phase + k) & 1), k + 1 == m);
             launch_seg<OpAdvance>(advance, 0, m);

@@ -582,7 +582,6 @@ struct efs_engine {
     // Rebuild everything that depends on more than one configure call.
     void build_plan() {
         if (!plan_dirty) return;
-        nf_pair = nf2ff_clear_of_pml();
         for (int p = 0; p < 2; ++p) {
             std::vector<float*> vp, cp;
             for (auto& r : pml) { vp.push_back(r->vf(p)); cp.push_back(r->cf(p)); }
@@ -622,6 +621,7 @@ struct efs_engine {
         }
         plan_ade_adopt();
         plan_ring();
+        tails = pml_split() ? tails_clear(false) : 0;
         build_deferred();
         mark_adopted();
         plan_dirty = false;
@@ -791,10 +791,10 @@ struct efs_engine {
     //
     // Latency-bound passes are paired into one launch (k_pair): the UPML H
     // pass with the deferred H (both after the E-side point operations; no
-    // deferred cell is a UPML cell), and, when no NF2FF sample reads a UPML
-    // cell (plan flag nf_pair), a step's NF2FF samples with the next step's
-    // UPML E pass (k_pml_e rewrites only UPML cells of those inputs, in place);
-    // the samples of a batch's last step run on their own.
+    // deferred cell is a UPML cell), and the UPML E pass with the TFSF face
+    // values of its step and with what the step before left for it (tails:
+    // NF2FF samples, TFSF current points, probe ring); a batch's last step
+    // leaves nothing.
     void enqueue_step(uint32_t k, int p, bool last, cudaEvent_t* marks = nullptr) {
         auto mark = [&](int i) { if (marks) ck(cudaEventRecord(marks[i], stream), "phase mark"); };
         mark(0);
@@ -814,15 +814,15 @@ struct efs_engine {
         if (ss_on)     // reads the fields before the UPML pre-update
             launch_k(false, k_steady_state, blocks(ss_n, T), T, 0, stream, V, st, k, ss_idx.as<uint32_t>(), ss_n, ss_period,
                                                               ss_e1.as<float>(), ss_e2.as<float>());
-        if (nf_held.on) {            // samples of step k-1 (its fields are this step's inputs) beside the UPML E pass
-            const PassNfSample a{V, C, nf_held.j, nf};
-            const uint32_t na = blocks(nf.np, T), nb = blocks(pml_items(), T);
-            if (indexed) pair(a, na, pml_e_pass<true>(p), nb);
-            else pair(a, na, pml_e_pass<false>(p), nb);
-            if (nf_held.j == NF_K - 1) launch_k(false, k_nf2ff_flush, blocks(nf.np, T), T, 0, stream, st, k - 1 - nf_held.j, nf_held.j + 1, nf);
-            nf_held.on = false;
-        } else if (split) {
-            launch_pml_e(p);
+        if (split) {                 // the UPML E pass, beside what step k-1 left and the face values
+            const PassTails t = tails_pass(k, V, C);
+            const PassNfSample a{V, C, held.j, nf};
+            const uint32_t na = held.nf ? blocks(nf.np, T) : 0, nb = blocks(pml_items(), T);
+            if (!na && !t.blocks()) launch_pml_e(p);
+            else if (indexed) pair(a, na, PassThen<PassPmlE<true>, PassTails>{pml_e_pass<true>(p), nb, t}, nb + t.blocks());
+            else pair(a, na, PassThen<PassPmlE<false>, PassTails>{pml_e_pass<false>(p), nb, t}, nb + t.blocks());
+            if (held.nf && held.j == NF_K - 1) launch_k(false, k_nf2ff_flush, blocks(nf.np, T), T, 0, stream, st, k - 1 - held.j, held.j + 1, nf);
+            held = Held{};
         }
         mark(1);
         if (ade_adopt) launch_ade_adopt(p, vfl);
@@ -835,12 +835,12 @@ struct efs_engine {
         // ADE(curr) reads H and the current flux, which the E side never
         // touches: it runs before the fused kernel overwrites the flux.
         if (ade_c.live()) launch_k(false, k_ade, blocks(ade_c.n, ADE_BLOCK), ADE_T, 0, stream, C, ade_dev(ade_c, cfl));
-        if (tf_n && !sweep) launch_k(false, k_tfsf_face, blocks(tf_n, T), T, 0, stream, st, k, tf_dev());   // TFSF face values of this step
+        if (tf_n && !sweep && !split) launch_k(false, k_tfsf_face, blocks(tf_n, T), T, 0, stream, st, k, tf_dev());   // TFSF face values of this step
         mark(2);
         const bool exc_rides = sweep && exc_may_ride();
         if (sweep) {
             launch_sweep_e(p, k, exc_rides);
-            ring_held = false;
+            held = Held{};
         } else {
             launch_fused_tma(p);
         }
@@ -869,7 +869,8 @@ struct efs_engine {
         else if (defer_n) launch_deferred(p);
         mark(5);
         // --- post-current (on the updated H) ---
-        if (tfsf_on && tfsf_c.groups) launch_k(early, early ? k_point_sources<1, true> : k_point_sources<1, false>, blocks(tfsf_c.groups, T), T, 0, stream, C1, st, k, point_dev(tfsf_c, tfsf_signal, tfsf_len, tfsf_period));
+        if (split && !last && (tails & TAIL_TC)) held.tc = true;
+        else if (tfsf_on && tfsf_c.groups) launch_k(early, early ? k_point_sources<1, true> : k_point_sources<1, false>, blocks(tfsf_c.groups, T), T, 0, stream, C1, st, k, point_dev(tfsf_c, tfsf_signal, tfsf_len, tfsf_period));
         if (pbc_on) for (auto& a : pbc_axes) launch_pbc(a, false, C1);
         if (ade_apply && ade_c.live()) launch_ade_apply(ade_c, C1);
         mark(6);
@@ -878,20 +879,93 @@ struct efs_engine {
             // surface samples of this step; the accumulators take every NF_K steps
             // and the batch's last step (nothing stays pending between batches)
             const uint32_t j = k % NF_K;
-            if (nf_pair && split && !last) {
-                nf_held = NfHeld{true, j};           // sampled beside the next step's UPML E pass
+            if (split && !last && (tails & TAIL_NF)) {
+                held.nf = true;
+                held.j = j;
             } else {
                 launch_k(false, k_nf2ff_sample, blocks(nf.np, T), T, 0, stream, V1, C1, j, nf);
                 if (j == NF_K - 1 || last) launch_k(false, k_nf2ff_flush, blocks(nf.np, T), T, 0, stream, st, k - j, j + 1, nf);
             }
         }
-        if (ring_on && sweep && ring_rides && !last) ring_held = true;   // sampled beside the next step's E sweep
+        if (ring_on && !last && (sweep ? ring_rides : split && (tails & TAIL_RING))) held.ring = true;
         else if (ring_on) launch_k(early, early ? k_gather_ring<true> : k_gather_ring<false>, blocks(ring_n, 64), 64, 0, stream, V1, C1, st, k, ring_dev());
         mark(7);
     }
-    struct NfHeld { bool on; uint32_t j; };
-    NfHeld nf_held{false, 0};     // capture: NF2FF samples of the previous step not yet issued
-    bool ring_held = false;       // and its probe ring samples
+    // What a step left for the next step's first launch, while a batch of steps is enqueued.
+    struct Held { bool nf = false, tc = false, ring = false; uint32_t j = 0; };
+    Held held;
+    PassTails tails_pass(uint32_t k, const float* V, float* C) const {
+        PassTails a;
+        memset(&a, 0, sizeof(a));
+        a.C = C; a.V = V; a.st = state.as<StepState>();
+        a.k = k; a.k1 = k - 1;
+        if (held.tc) { a.tc = point_dev(tfsf_c, tfsf_signal, tfsf_len, tfsf_period); a.nb_tc = blocks(tfsf_c.groups, 256); }
+        if (held.ring) { a.ring = ring_dev(); a.nb_ring = blocks(ring_n, 256); }
+        if (tf_n) { a.face = tf_dev(); a.nb_face = blocks(tf_n, 256); }
+        return a;
+    }
+    // Which of a step's last operations may run beside the next step's first
+    // launch: the UPML E pass, or, with_mur, k_mur_adopt.  The box of the cells
+    // that the TFSF current points write stands for the points, and the planes
+    // of the Mur targets for the targets.
+    //  TAIL_NF, TAIL_RING: the samples read no E that the launch writes;
+    //  TAIL_TC: the points' H is read neither by the launch nor by the samples,
+    //  and nothing acts on H between the two.
+    enum { TAIL_NF = 1, TAIL_RING = 2, TAIL_TC = 4 };
+    uint32_t tails = 0;                                    // plan: with the UPML E pass
+    uint32_t tc_lo[3] = {0, 0, 0}, tc_hi[3] = {0, 0, 0};   // cells of the current points
+    uint32_t tails_clear(bool with_mur) const {
+        const bool tc = tfsf_on && tfsf_c.groups;
+        uint32_t ok = (nf_on ? TAIL_NF : 0) | (ring_on ? TAIL_RING : 0) | (tc && !pbc_on && !(ade_apply && ade_c.live()) ? TAIL_TC : 0);
+        const uint32_t Nd32 = (uint32_t)Nd;
+        struct Cell { uint32_t x[3]; };
+        auto cell_of = [&](uint32_t f) {
+            const uint32_t c = f % Nd32, row = c / Pz;
+            return Cell{{row / Ny, row % Ny, c % Pz}};
+        };
+        // cells [a, a + more] against the box grown by `grow` at its high ends
+        auto meets = [&](const uint32_t a[3], uint32_t more, uint32_t grow) {
+            bool m = true;
+            for (int d = 0; d < 3; ++d) m &= a[d] <= tc_hi[d] + grow && tc_lo[d] <= a[d] + more;
+            return m;
+        };
+        std::vector<uint8_t> plane[3];                     // planes that hold Mur targets
+        if (with_mur && mur_fast)
+            for (int d = 0; d < 3; ++d) plane[d].assign((d == 0 ? Nx : d == 1 ? Ny : Pz) + 1, 0);
+        if (with_mur && mur_fast)
+            for (size_t i = 0; i < h_mur_normal.size(); ++i) {
+                const Cell t = cell_of(h_mur_normal[i]), s = cell_of(h_mur_shifted[i]);
+                int d = 0;
+                while (d < 2 && t.x[d] == s.x[d]) ++d;
+                plane[d][t.x[d]] = 1;
+                if (meets(t.x, 0, 1) || meets(s.x, 0, 1)) ok &= ~TAIL_TC;
+            }
+        for (auto& R : pml) {
+            bool m = true;
+            for (int d = 0; d < 3; ++d) m &= R->s[d] <= tc_hi[d] + 1 && tc_lo[d] < R->s[d] + R->n[d];
+            if (m) ok &= ~TAIL_TC;
+        }
+        if (!nf2ff_clear_of_pml()) ok &= ~TAIL_NF;
+        if (nf_on)
+            for (size_t i = 0; i + 2 < h_nf_pts.size(); i += 3) {
+                const uint32_t* x = &h_nf_pts[i];
+                if (meets(x, 1, 0)) ok &= ~TAIL_TC;
+                for (int d = 0; d < 3; ++d)
+                    if (!plane[d].empty() && (plane[d][x[d]] || plane[d][x[d] + 1])) ok &= ~TAIL_NF;
+            }
+        if (ring_on)
+            for (uint32_t f : h_ring) {
+                const Cell t = cell_of(f);
+                if (meets(t.x, 0, 0)) ok &= ~TAIL_TC;
+                if (with_mur && mur_fast && std::binary_search(h_mur_normal.begin(), h_mur_normal.end(), f)) ok &= ~TAIL_RING;
+                for (auto& R : pml) {
+                    bool in = true;
+                    for (int d = 0; d < 3; ++d) in &= t.x[d] >= R->s[d] && t.x[d] < R->s[d] + R->n[d];
+                    if (in) ok &= ~TAIL_RING;
+                }
+            }
+        return ok;
+    }
     bool ring_rides = false;      // plan: nothing rewrites a probed E between a step's end and the next E sweep
     std::vector<uint32_t> h_ring; // probed field indices (device order)
     // A step's samples may wait for the next E sweep when no probed E is a target
@@ -914,7 +988,6 @@ struct efs_engine {
     bool exc_may_ride() const {
         return exc_on && exc_groups && exc_groups <= SW_EXC && !(tfsf_on && tfsf_v.groups) && !tf_n && !pbc_on && !mur_gen;
     }
-    bool nf_pair = false;         // plan: no NF2FF sample reads a UPML cell
     // passes of the paired launches (k_pair, 256-thread blocks)
     template <bool IDX> PassPmlE<IDX> pml_e_pass(int p) const {
         return PassPmlE<IDX>{fused_grid(p), pml_set(p), pml_set(1 - p), vbuf(p), pml_items()};
@@ -972,7 +1045,7 @@ struct efs_engine {
         build_plan();
         std::vector<cudaEvent_t> ev((size_t)steps * (EFS_PHASES + 1));
         for (auto& x : ev) ck(cudaEventCreate(&x), "event");
-        nf_held.on = ring_held = false;
+        held = Held{};
         try {
             int q = cur;
             for (uint32_t k = 0; k < steps; ++k) {
@@ -1066,7 +1139,7 @@ struct efs_engine {
     bool early = false;              // of the step being enqueued
     bool use_sweep() const { return !xchunk && skip_plane == ~0u && (!indexed || Nd * 52 <= SWEEP_BYTES); }
     uint32_t sweep_blocks() const { return Nx * sweep_plane_blocks(Ny, Pz); }
-    // E sweep of step k, with the excitation and the probe ring samples of step k-1 (ring_held) riding
+    // E sweep of step k, with the excitation and the probe ring samples of step k-1 (held) riding
     template <bool IDX, bool PML>
     void launch_sweep_e_k(int p, const SweepRiders& rd) {
         launch_k(early, k_sweep_e<IDX, PML>, rd.nb + blocks(rd.ring.G, SW_T), SW_T, 0, stream, fused_grid(p), pml_set(p), pml_set(1 - p), rd);
@@ -1079,7 +1152,7 @@ struct efs_engine {
         rd.ring_k = k - 1;
         rd.nb = sweep_blocks();
         if (exc) rd.exc = exc_dev();
-        if (ring_held) rd.ring = ring_dev();
+        if (held.ring) rd.ring = ring_dev();
         const bool hp = !pml.empty();
         if (indexed) { if (hp) launch_sweep_e_k<true, true>(p, rd); else launch_sweep_e_k<true, false>(p, rd); }
         else { if (hp) launch_sweep_e_k<false, true>(p, rd); else launch_sweep_e_k<false, false>(p, rd); }
@@ -1169,7 +1242,7 @@ struct efs_engine {
         if (graphs.size() > 12) drop_graphs();
         cudaGraph_t graph;
         ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "BeginCapture");
-        nf_held.on = ring_held = false;
+        held = Held{};
         try {
             int q = p;
             for (uint32_t k = 0; k < m; ++k) { enqueue_step(k, q, k + 1 == m); q = pnext(q); }
@@ -1860,6 +1933,11 @@ efs_status efs_configure_tfsf(efs_engine* e, const float* signal, uint32_t L, ui
         for (uint32_t i = 0; i < nv; ++i) vt[i] = vp[i].field_idx;
         e->check_idx3(vt.data(), nv, "TFSF field_idx");
         build_points(e, e->tfsf_c, cp, nc);
+        for (int d = 0; d < 3; ++d) { e->tc_lo[d] = ~0u; e->tc_hi[d] = 0; }
+        for (uint32_t i = 0; i < nc; ++i) {
+            const uint32_t c = cp[i].field_idx % (uint32_t)e->N, row = c / e->Nz, x[3] = {row / e->Ny, row % e->Ny, c % e->Nz};
+            for (int d = 0; d < 3; ++d) { e->tc_lo[d] = std::min(e->tc_lo[d], x[d]); e->tc_hi[d] = std::max(e->tc_hi[d], x[d]); }
+        }
         // the voltage side's point set and targets are built by the plan
         // (plan_tfsf_faces), once the core update's z faces are chosen
         e->h_tfsf_v.assign(vp, vp + nv);
@@ -2587,7 +2665,7 @@ efs_status efs_time_core(efs_engine* e, uint32_t reps, float* ms) {
         };
         const int p = e->cur;
         const bool sweep = e->use_sweep();
-        e->ring_held = false;
+        e->held = efs_engine::Held{};
         const float a = timed([&] {
             if (sweep) { e->launch_sweep_e(p, 0, false); e->launch_sweep_h(p); }
             else e->launch_fused_tma(p);
@@ -2619,11 +2697,12 @@ efs_status efs_kernels_per_step(efs_engine* e, uint32_t* out) {
         const bool sweep = e->use_sweep(), split = e->pml_split() && !sweep;
         // E and H sweeps, the TFSF faces added after the first
         uint32_t k = sweep ? 2 + (e->tf_n > 0) : 1 + split + ((e->defer_n > 0) || split);
+        const uint32_t held = split ? e->tails : 0;
         k += e->ss_on + e->ade_v.live() + e->ade_c.live() + e->mur_fast + 3 * (e->mur_gen > 0) + 2 * e->rlc_on;
         if (e->ade_apply) k += (e->ade_v.live() && !e->ade_adopt) + e->ade_c.live();
-        k += (e->tfsf_on && e->tfsf_v.groups) + (e->tfsf_on && e->tfsf_c.groups) + (e->exc_on && e->exc_groups > 0 && !(sweep && e->exc_may_ride()));
+        k += (e->tfsf_on && e->tfsf_v.groups) + (e->tfsf_on && e->tfsf_c.groups && !(held & efs_engine::TAIL_TC)) + (e->tf_n && !sweep && !split) + (e->exc_on && e->exc_groups > 0 && !(sweep && e->exc_may_ride()));
         k += e->pbc_on ? 2 * (uint32_t)e->pbc_axes.size() : 0;
-        k += (e->nf_on && !(e->nf_pair && split)) + (e->ring_on && !(sweep && e->ring_rides));   // riders of other launches are not counted
+        k += (e->nf_on && !(held & efs_engine::TAIL_NF)) + (e->ring_on && !(sweep ? e->ring_rides : (held & efs_engine::TAIL_RING) != 0));   // riders of other launches are not counted
         *out = k;
     });
 }

@@ -776,9 +776,34 @@ struct PassDeferred {
     FusedGrid g; const uint32_t* cells; uint32_t n;
     __device__ void run(uint32_t blk) const { deferred_h_body<IDX>(g, cells, n, blk * 256u + threadIdx.x); }
 };
+// The last operations of the step before (TFSF current points, probe ring; k1:
+// that step, whose fields V, C are this step's inputs) and the TFSF face values
+// of step k, each in whole blocks behind the UPML E pass; apart they are
+// launches of 4 to 8 us each (a step of 200x200x100 dispersive took 142 us with
+// them apart and takes 136, 256^3 240 and 237, 320x320x160 384 and 381).
+struct PassTails {
+    float* C; const float* V; const StepState* st;
+    uint32_t k, k1, nb_tc, nb_ring, nb_face;
+    PointSources tc; RingDev ring; TfsfFaceDev face;
+    __device__ void run(uint32_t blk) const {
+        if (blk < nb_tc) return point_sources_body<1>(C, st, k1, tc, blk * 256u + threadIdx.x);
+        blk -= nb_tc;
+        if (blk < nb_ring) return gather_ring_body(V, C, st, k1, ring, blk * 256u + threadIdx.x);
+        tfsf_face_body(st, k, face, (blk - nb_ring) * 256u + threadIdx.x);
+    }
+    uint32_t blocks() const { return nb_tc + nb_ring + nb_face; }
+};
 struct PassNfSample {
     const float* V; const float* C; uint32_t slot; Nf2ffDev d;
     __device__ void run(uint32_t blk) const { nf2ff_sample_body(V, C, slot, d, blk * 256u + threadIdx.x); }
+};
+template <class A, class B>
+struct PassThen {                       // na blocks of A, then B's
+    A a; uint32_t na; B b;
+    __device__ void run(uint32_t blk) const {
+        if (blk < na) a.run(blk);
+        else b.run(blk - na);
+    }
 };
 template <class A, class B>
 __global__ void __launch_bounds__(256, PML_MINB) k_pair(const A a, uint32_t na, const B b, uint32_t nb) {
