@@ -15,6 +15,13 @@
 //   TFSF(curr) | PBC(curr) | [ADE apply to H]                             (sparse)
 //   NF2FF sample/flush | probe ring
 //
+// Forms of it: on a grid that stays in L2 the core update is two sweeps that
+// take the UPML cells with them (efs_sweep.cuh); a grid of a cluster's size runs
+// all steps of a batch in one launch (efs_resident.cuh); Mur targets and applied
+// ADE media that nothing else touches are computed ahead of the core update,
+// which adopts them (k_mur_adopt, k_ade_adopt); a step's last passes may run
+// beside the next step's first (tails_clear).
+//
 // Reads that the reference makes between the UPML pre-update and the core
 // update (ADE, Mur pre) are redirected to the region's flux array, which is
 // what the field holds at that moment, so fusing pre/post into the UPML
@@ -31,6 +38,7 @@
 #include "efs_fused.cuh"
 #include "efs_tma.cuh"
 #include "efs_sweep.cuh"
+#include "efs_resident.cuh"
 #include "efs_host.h"
 
 #include <cuda_runtime.h>
@@ -621,6 +629,7 @@ struct efs_engine {
         }
         plan_ade_adopt();
         plan_ring();
+        plan_resident();
         tails = pml_split() ? tails_clear(false) : 0;
         build_deferred();
         mark_adopted();
@@ -1138,6 +1147,58 @@ struct efs_engine {
     // 20.0 / 19.7; 256^3 287 / 253, 16 members batched 205 / 149).
     bool early = false;              // of the step being enqueued
     bool use_sweep() const { return !xchunk && skip_plane == ~0u && (!indexed || Nd * 52 <= SWEEP_BYTES); }
+    // Batches of steps that run in one launch (efs_resident.cuh): grids of a cluster's size on which
+    // only the excitation and the probe ring act beside the sweeps.
+    uint32_t resident_threads() const { return std::max(32u, blocks((uint32_t)(Nd / 2), 32 * RS_CTAS) * 32); }
+    bool resident() const {
+        return resident_fits && use_sweep() && pml.empty() && !mur_on && !tf_n && !tfsf_on && !pbc_on && !rlc_on && !ss_on && !nf_on &&
+               !ade_v.live() && !ade_c.live() && (!exc_on || exc_groups <= resident_threads()) && (!ring_on || ring_n <= resident_threads());
+    }
+    static cudaLaunchConfig_t resident_config(uint32_t T, cudaLaunchAttribute* at, cudaStream_t stream) {
+        at->id = cudaLaunchAttributeClusterDimension;
+        at->val.clusterDim.x = RS_CTAS;
+        at->val.clusterDim.y = at->val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = RS_CTAS;
+        cfg.blockDim = T;
+        cfg.dynamicSmemBytes = resident_smem(T);
+        cfg.stream = stream;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cfg;
+    }
+    void (*resident_kernel() const)(FusedGrid, Resident) {
+        if (resident_threads() <= RS_T / 2) return indexed ? k_resident<true, RS_T / 2> : k_resident<false, RS_T / 2>;
+        return indexed ? k_resident<true, RS_T> : k_resident<false, RS_T>;
+    }
+    // The plan's half of the rule: the device has room for the cluster.
+    void plan_resident() {
+        resident_fits = use_sweep() && Nd / 2 <= RS_PAIRS;
+        if (!resident_fits) return;
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = resident_config(resident_threads(), &at, stream);
+        int clusters = 0;
+        resident_fits = cudaFuncSetAttribute(resident_kernel(), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaFuncSetAttribute(resident_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)resident_smem(RS_T)) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&clusters, resident_kernel(), &cfg) == cudaSuccess && clusters > 0;
+        if (!resident_fits) cudaGetLastError();            // sweeps then
+    }
+    bool resident_fits = false;
+    void launch_resident(uint32_t steps, int p) {
+        Resident r;
+        memset(&r, 0, sizeof(r));
+        const int q = steps & 1 ? pnext(p) : p;
+        r.st = state.as<StepState>();
+        r.steps = steps;
+        r.V = vbuf(q);
+        r.H = cbuf(q);
+        if (exc_on) r.exc = exc_dev();
+        if (ring_on) r.ring = ring_dev();
+        const uint32_t T = resident_threads();
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = resident_config(T, &at, stream);
+        ck(cudaLaunchKernelEx(&cfg, resident_kernel(), fused_grid(p), r), "launch");
+    }
     uint32_t sweep_blocks() const { return Nx * sweep_plane_blocks(Ny, Pz); }
     // E sweep of step k, with the excitation and the probe ring samples of step k-1 (held) riding
     template <bool IDX, bool PML>
@@ -1245,8 +1306,10 @@ struct efs_engine {
         held = Held{};
         try {
             int q = p;
-            for (uint32_t k = 0; k < m; ++k) { enqueue_step(k, q, k + 1 == m); q = pnext(q); }
-            launch_k(early, early ? k_advance<true> : k_advance<false>, 1, 1, 0, stream, state.as<StepState>(), m);
+            if (resident()) launch_resident(m, p);
+            else for (uint32_t k = 0; k < m; ++k) { enqueue_step(k, q, k + 1 == m); q = pnext(q); }
+            const bool adv = early && !resident();
+            launch_k(adv, adv ? k_advance<true> : k_advance<false>, 1, 1, 0, stream, state.as<StepState>(), m);
         } catch (...) {
             cudaStreamEndCapture(stream, &graph);
             throw;
@@ -2693,6 +2756,7 @@ efs_status efs_kernels_per_step(efs_engine* e, uint32_t* out) {
         e->need_init();
         if (!out) fail(EFS_ERR_INVALID, "out must be non-null");
         e->build_plan();
+        if (e->resident()) { *out = 1; return; }   // one launch, for all steps of a batch
         // fused kernel, UPML E pass, UPML H pass and deferred H (one paired launch when both)
         const bool sweep = e->use_sweep(), split = e->pml_split() && !sweep;
         // E and H sweeps, the TFSF faces added after the first
