@@ -518,11 +518,13 @@ def run_b200(args):
             "peak_kind": "of " + peak_kind}
     step_bytes = workloads.job_bytes_per_step(job)
     # our kernels in the timed region: per timestep plan + per captured graph (64
-    # steps each) one counter update and ceil(m/16) NF2FF accumulator passes +
+    # steps each) one counter update, the NF2FF samples and TFSF current points of its
+    # last step (otherwise part of the next step's first launch) and ceil(m/16) NF2FF
+    # accumulator passes +
     # the two energy-reduction kernels per step
     chunks = [64] * (BATCH // 64) + ([BATCH % 64] if BATCH % 64 else [])
     nf_passes = sum(math.ceil(m / 16) for m in chunks) if job.get("nf2ff") else 0
-    launches = args.steps * (BATCH * eng.kernelsPerStep() + len(chunks) + nf_passes + 2)
+    launches = args.steps * (BATCH * eng.kernelsPerStep() + 3 * len(chunks) + nf_passes + 2)
     phases = eng.timePhases(32)              # per-phase device ms per timestep, launched kernel by kernel
     tfsf_faces = [int(v) for v in eng.debugRead("tfsf_faces")]
     far = None

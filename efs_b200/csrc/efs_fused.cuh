@@ -89,10 +89,6 @@ __device__ __forceinline__ float pml_chain_pp(const PmlSet& ps, const PmlSet& pn
     return v;
 }
 
-// Regions (bit mask) whose extent along `axis` contains coordinate c.
-__device__ __forceinline__ uint32_t axis_mask(const PmlSet& ps, uint32_t cand, int axis, uint32_t c) {
-    return cand & __ldg((axis == 0 ? ps.xm : axis == 1 ? ps.ym : ps.zm) + c);
-}
 // Regions that hold the cell.
 __device__ __forceinline__ uint32_t cell_mask(const PmlSet& ps, uint32_t x, uint32_t y, uint32_t z) {
     return __ldg(ps.xm + x) & __ldg(ps.ym + y) & __ldg(ps.zm + z);

@@ -68,20 +68,6 @@ __device__ __forceinline__ bool in_region(const PmlRegion& r, uint32_t x, uint32
     return (x - r.s[0]) < r.n[0] && (y - r.s[1]) < r.n[1] && (z - r.s[2]) < r.n[2];
 }
 
-// Regions intersecting the box [lo, hi] (inclusive), as a bit mask.  Blocks
-// compute this once so cells of tiles that touch no UPML region skip the
-// per-cell membership tests entirely.
-__device__ __forceinline__ uint32_t region_mask(const PmlSet& ps, const uint32_t lo[3], const uint32_t hi[3]) {
-    uint32_t m = 0;
-    for (int r = 0; r < ps.count; ++r) {
-        bool hit = true;
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-            hit = hit && (hi[d] >= ps.r[r].s[d]) && (lo[d] < ps.r[r].s[d] + ps.r[r].n[d]);
-        if (hit) m |= 1u << r;
-    }
-    return m;
-}
 __device__ __forceinline__ size_t region_p(const PmlRegion& r, uint32_t n, uint32_t x, uint32_t y, uint32_t z) {
     size_t nyz = (size_t)r.n[1] * r.n[2];
     return (size_t)n * r.n[0] * nyz + (size_t)(x - r.s[0]) * nyz + (size_t)(y - r.s[1]) * r.n[2] + (z - r.s[2]);

@@ -339,8 +339,9 @@ efs_status efs_time_phases(efs_engine* e, uint32_t steps, float* ms);
 
 /* Diagnostics: kernel launches one timestep enqueues with the current
  * configuration (a captured batch of n steps adds one counter update and,
- * with NF2FF configured, ceil(n/16) accumulator passes and, when the samples
- * ride on the next step's UPML E pass, one sample pass for its last step). */
+ * with NF2FF configured, ceil(n/16) accumulator passes, and its last step runs
+ * on their own the operations that otherwise ride on the next step's first
+ * launch).  A grid that runs all steps of a batch in one launch reports 1. */
 efs_status efs_kernels_per_step(efs_engine* e, uint32_t* out);
 
 /* --- batched form ------------------------------------------------------
