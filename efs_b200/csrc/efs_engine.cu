@@ -938,17 +938,24 @@ struct efs_engine {
             for (int d = 0; d < 3; ++d) m &= a[d] <= tc_hi[d] + grow && tc_lo[d] <= a[d] + more;
             return m;
         };
+        // Mur targets and the cells they shift to lie on planes: the plane is decoded with one division an
+        // entry, the cell only where the plane crosses the box
         std::vector<uint8_t> plane[3];                     // planes that hold Mur targets
-        if (with_mur && mur_fast)
-            for (int d = 0; d < 3; ++d) plane[d].assign((d == 0 ? Nx : d == 1 ? Ny : Pz) + 1, 0);
-        if (with_mur && mur_fast)
+        if (with_mur && mur_fast && (ok & (TAIL_NF | TAIL_TC))) {
+            const uint32_t stride[3] = {Ny * Pz, Pz, 1}, len[3] = {Nx, Ny, Pz};
+            for (int d = 0; d < 3; ++d) plane[d].assign(len[d] + 1, 0);
             for (size_t i = 0; i < h_mur_normal.size(); ++i) {
-                const Cell t = cell_of(h_mur_normal[i]), s = cell_of(h_mur_shifted[i]);
-                int d = 0;
-                while (d < 2 && t.x[d] == s.x[d]) ++d;
-                plane[d][t.x[d]] = 1;
-                if (meets(t.x, 0, 1) || meets(s.x, 0, 1)) ok &= ~TAIL_TC;
+                const uint32_t f = h_mur_normal[i], g = h_mur_shifted[i], delta = f > g ? f - g : g - f;
+                const int d = delta == stride[0] ? 0 : delta == stride[1] ? 1 : 2;
+                const uint32_t c = f >= 2 * Nd32 ? f - 2 * Nd32 : f >= Nd32 ? f - Nd32 : f;
+                const uint32_t at = d == 0 ? c / stride[0] : d == 1 ? c / Pz % Ny : c % Pz;
+                plane[d][at] = 1;
+                const bool wraps = f > g ? at == 0 : at + 1 == len[d];             // g is not the neighbour along d
+                if ((ok & TAIL_TC) && (delta != stride[d] || wraps || (at <= tc_hi[d] + 2 && tc_lo[d] <= at + 1)) &&
+                    (meets(cell_of(f).x, 0, 1) || meets(cell_of(g).x, 0, 1)))
+                    ok &= ~TAIL_TC;
             }
+        }
         for (auto& R : pml) {
             bool m = true;
             for (int d = 0; d < 3; ++d) m &= R->s[d] <= tc_hi[d] + 1 && tc_lo[d] < R->s[d] + R->n[d];
