@@ -1891,7 +1891,7 @@ void efs_engine::plan_mur() {
     constexpr uint8_t WRITES = 1, READS = 2, GROUPED = 4;     // shared: target shared; shifted cell is a target; in a group
     parallel_chunks(n, W, [&](unsigned, size_t lo, size_t hi) {
         for (size_t i = lo; i < hi; ++i) {
-            ok[i] = !pbc_on && !has(F.get(), t[i]) && !has(F.get(), sh[i]) && redirect(t[i]).sel == 0 && redirect(sh[i]).sel == 0 &&
+            ok[i] = !pbc_on && !has(F.get(), t[i]) && !has(F.get(), sh[i]) && (pml.empty() || (redirect(t[i]).sel == 0 && redirect(sh[i]).sel == 0)) &&
                     !std::binary_search(exc.begin(), exc.end(), t[i]);
             if (i + 1 == n || t[i + 1] != t[i]) kind[i] = MUR_LAST;
             shared[i] = ((i > 0 && t[i - 1] == t[i]) || (i + 1 < n && t[i + 1] == t[i]) ? WRITES : 0) | (has(T.get(), sh[i]) ? READS : 0);
@@ -1902,9 +1902,8 @@ void efs_engine::plan_mur() {
         if (shared[i] & READS) read.push_back(sh[i]);
     std::sort(read.begin(), read.end());
     read.erase(std::unique(read.begin(), read.end()), read.end());
-    parallel_chunks(n, W, [&](unsigned, size_t lo, size_t hi) {
-        for (size_t i = lo; i < hi; ++i) if (std::binary_search(read.begin(), read.end(), t[i])) shared[i] |= WRITES;
-    });
+    for (uint32_t r : read)
+        for (size_t i = std::lower_bound(t.begin(), t.end(), r) - t.begin(); i < n && t[i] == r; ++i) shared[i] |= WRITES;
     // entries that share cells: connected through their targets
     std::vector<uint32_t> ents, slot;
     for (size_t i = 0; i < n; ++i)
