@@ -208,7 +208,9 @@ struct efs_batch {
     bool any_pml = false;
     bool mur_first = false;                    // no UPML member, and no ADE pass to read E before k_mur_adopt writes its targets
     uint32_t tails = 0;                        // operations every member may leave to the next step's first launch
-    bool pts_merge = false;                    // TFSF voltage points and the excitation act on different E, nothing between them
+    // TFSF voltage points, Mur post and the excitation in one launch: in no member do two of them meet (the points
+    // and the excitation act on different E, and a member with either has no Mur post)
+    bool pts_merge = false;
     efs_engine::Held held;                     // and what the step just enqueued left
     std::map<uint32_t, cudaGraphExec_t> graphs;
 
@@ -519,8 +521,8 @@ struct efs_batch {
         launch_tiles<false, true>(2, bm);
         launch_tiles<false, false>(0, bm);
         mark(3);
-        if (pts_merge) {
-            launch_segs(seg_arg<OpPoints<1>>(tfsf_v[s], true, k), seg_arg<OpPoints<0>>(exc[s], true, k));
+        if (pts_merge) {                         // Mur post: of members that have neither of the two
+            launch_segs(seg_arg<OpPoints<1>>(tfsf_v[s], true, k), seg_arg<OpMurPost>(mur_post[s], true, k), seg_arg<OpPoints<0>>(exc[s], true, k));
         } else {
             launch_seg<OpPoints<1>>(tfsf_v[s], k);
             launch_seg<OpMurPost>(mur_post[s], k);
