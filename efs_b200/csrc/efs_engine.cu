@@ -2101,7 +2101,7 @@ efs_status efs_configure_rlc(efs_engine* e, uint32_t n, const efs_rlc_element* e
         std::vector<float> p2(9 * (size_t)n);
         for (uint32_t i = 0; i < n; ++i) { type2[i] = type[perm[i]]; memcpy(&p2[9 * (size_t)i], &p[9 * (size_t)perm[i]], 36); }
         e->upload(e->rlc_gtarget, ut); e->upload(e->rlc_goff, goff);
-        e->h_rlc_series.clear(); e->h_ring.clear();
+        e->h_rlc_series.clear();
         e->h_rlc_targets = tgt;
         for (uint32_t i = 0; i < n; ++i) if (el[i].type_flag == 1) e->h_rlc_series.push_back(tgt[i]);
         e->upload(e->rlc_type, type2); e->upload(e->rlc_p, p2);
