@@ -1,8 +1,9 @@
 // Host-side helpers of the engine (plain C++17, no CUDA): the threaded stable
 // radix sort that orders point lists by device index, the grouping of entries
 // by target built on it, the chunked host-thread loop, and the copy through
-// staging buffers of large read-backs.  Compiled into libefs.so and, on its own, into the CPU test of these
-// helpers (tests/test_host_plan.py, tests/test_staged_copy.py).
+// staging buffers of large read-backs.  Compiled into libefs.so and, on its
+// own, into the CPU tests of these helpers (tests/test_host_plan.py,
+// tests/test_staged_copy.py, tests/test_few_threads.py).
 #pragma once
 
 #include <algorithm>
@@ -10,6 +11,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -100,7 +102,8 @@ inline void group_by(const std::vector<uint32_t>& tgt, std::vector<uint32_t>& ut
 // `bytes` bytes into dst in chunks through `slots` staging buffers: fetch(c, n)
 // starts chunk c (n bytes) into buffer c % slots, wait(c) returns once it has
 // arrived, T threads copy each arrived chunk out (every thread a part of it)
-// while later chunks are on their way.  fetch and wait run on the caller's
+// while later chunks are on their way; fewer where the host gives fewer, the
+// caller's alone where it gives none.  fetch and wait run on the caller's
 // thread and may throw; chunks started and not yet waited for are then left to
 // the caller.
 template <class Fetch, class Wait>
@@ -108,6 +111,7 @@ void staged_copy(void* dst, size_t bytes, const uint8_t* const* buf, unsigned sl
                  Wait&& wait) {
     const size_t nc = (bytes + chunk - 1) / chunk;
     auto size = [&](size_t c) { return std::min(chunk, bytes - c * chunk); };
+    auto out = [&](size_t c, size_t lo, size_t hi) { memcpy(static_cast<uint8_t*>(dst) + c * chunk + lo, buf[c % slots] + lo, hi - lo); };
     std::atomic<size_t> ready{0};                      // chunks that have arrived
     std::atomic<bool> stop{false};
     std::vector<std::atomic<unsigned>> done(slots);    // threads that have copied their part of the buffer's chunk
@@ -118,16 +122,20 @@ void staged_copy(void* dst, size_t bytes, const uint8_t* const* buf, unsigned sl
                 if (stop.load(std::memory_order_relaxed)) return;
                 std::this_thread::yield();
             }
-            const size_t n = size(c), lo = n * t / T, hi = n * (t + 1) / T;
-            memcpy(static_cast<uint8_t*>(dst) + c * chunk + lo, buf[c % slots] + lo, hi - lo);
+            const size_t n = size(c);                  // T is final before the first chunk is ready
+            out(c, n * t / T, n * (t + 1) / T);
             done[c % slots].fetch_add(1, std::memory_order_release);
         }
     };
     std::vector<std::thread> th;
     auto join = [&] { for (auto& x : th) x.join(); };
+    th.reserve(T);
     try {
-        th.reserve(T);
         for (unsigned t = 0; t < T; ++t) th.emplace_back(work, t);
+    } catch (const std::exception&) {                  // those that there are
+    }
+    T = (unsigned)th.size();
+    try {
         size_t started = 0;
         for (size_t c = 0; c < nc; ++c) {
             for (; started < nc && started < c + slots; ++started) {
@@ -139,6 +147,7 @@ void staged_copy(void* dst, size_t bytes, const uint8_t* const* buf, unsigned sl
                 fetch(started, size(started));
             }
             wait(c);
+            if (T == 0) out(c, 0, size(c));
             ready.store(c + 1, std::memory_order_release);
         }
     } catch (...) {
