@@ -3,7 +3,8 @@
 // by target built on it, the chunked host-thread loop, and the copy through
 // staging buffers of large read-backs.  Compiled into libefs.so and, on its
 // own, into the CPU tests of these helpers (tests/test_host_plan.py,
-// tests/test_staged_copy.py, tests/test_few_threads.py).
+// tests/test_staged_copy.py, tests/test_few_threads.py,
+// tests/test_few_threads_loop.py).
 #pragma once
 
 #include <algorithm>
@@ -25,14 +26,20 @@ inline unsigned host_threads(size_t n) {
 }
 
 // f(t, lo, hi) on T contiguous chunks of [0, n), chunk t on its own thread
-// (chunk 0 on the caller's).  f must not throw.
+// (chunk 0 on the caller's, as are those the host gives no thread for).  f must
+// not throw.
 template <class F>
 void parallel_chunks(size_t n, unsigned T, F&& f) {
     if (T <= 1) { f(0u, (size_t)0, n); return; }
     std::vector<std::thread> th;
     th.reserve(T - 1);
-    for (unsigned t = 1; t < T; ++t) th.emplace_back([&, t] { f(t, n * t / T, n * (t + 1) / T); });
+    unsigned t = 1;
+    try {
+        for (; t < T; ++t) th.emplace_back([&f, n, T, t] { f(t, n * t / T, n * (t + 1) / T); });
+    } catch (const std::exception&) {                  // chunk t has no thread
+    }
     f(0u, (size_t)0, n / T);
+    for (; t < T; ++t) f(t, n * t / T, n * (t + 1) / T);
     for (auto& x : th) x.join();
 }
 
