@@ -592,8 +592,8 @@ struct efs_batch {
         for (efs_engine* e : mem) ck(cudaStreamWaitEvent(e->stream, ev_done, 0), "wait");
     }
 
-    cudaGraphExec_t graph_for(uint32_t m) {
-        const uint32_t key = m * 2 + phase;
+    cudaGraphExec_t graph_for(uint32_t m, uint32_t ph) {
+        const uint32_t key = m * 2 + ph;
         auto it = graphs.find(key);
         if (it != graphs.end()) return it->second;
         if (graphs.size() > 12) drop_graphs();
@@ -601,7 +601,7 @@ struct efs_batch {
         ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "BeginCapture");
         held = efs_engine::Held{};
         try {
-            for (uint32_t k = 0; k < m; ++k) enqueue_step(k, (int)((phase + k) & 1), k + 1 == m);
+            for (uint32_t k = 0; k < m; ++k) enqueue_step(k, (int)((ph + k) & 1), k + 1 == m);
             launch_seg<OpAdvance>(advance, 0, m);
         } catch (...) {
             cudaStreamEndCapture(stream, &graph);
@@ -614,6 +614,24 @@ struct efs_batch {
         ck(err, "cudaGraphInstantiate");
         graphs[key] = ge;
         return ge;
+    }
+
+    // Plan and capture what iterate(n) launches, without a step.
+    void capture(uint32_t n) {
+        if (stale()) plan();
+        uint32_t ph = phase;
+        for (uint32_t m; n > 0; n -= m) {
+            m = std::min(n, 64u);
+            graph_for(m, ph);
+            ph ^= m & 1;
+        }
+    }
+    // Plane depth (0: the plan's own) and CTAs per SM from the next plan on.
+    void shape(uint32_t x, uint32_t c) {
+        if (x != xchunk || (x == 0 && c != ctas_per_sm)) planned = false;   // the tiles depend on the depth, the plan's depth on the CTAs
+        if (c != ctas_per_sm) drop_graphs();
+        xchunk = x;
+        ctas_per_sm = c;
     }
 
     // Members stepped or reconfigured outside the batch since the plan: re-plan.
@@ -633,7 +651,7 @@ struct efs_batch {
         const uint32_t CH = 64;
         while (n > 0) {
             const uint32_t m = std::min(n, CH);
-            ck(cudaGraphLaunch(graph_for(m), stream), "cudaGraphLaunch");
+            ck(cudaGraphLaunch(graph_for(m, phase), stream), "cudaGraphLaunch");
             for (efs_engine* e : mem) {
                 e->numTS += m;
                 if (m & 1) e->cur ^= 1;
@@ -726,11 +744,8 @@ efs_status efs_batch_sync(efs_batch* b) { return bguard(b, [&] { b->sync(); }); 
 
 efs_status efs_batch_set_shape(efs_batch* b, uint32_t xchunk, uint32_t ctas_per_sm) {
     return bguard(b, [&] {
-        if (xchunk == 0 || ctas_per_sm == 0 || ctas_per_sm > 2) fail(EFS_ERR_INVALID, "xchunk > 0 and ctas_per_sm in 1..2");
-        if (xchunk != b->xchunk) b->planned = false;    // tiles depend on the plane depth
-        b->xchunk = xchunk;
-        if (ctas_per_sm != b->ctas_per_sm) b->drop_graphs();
-        b->ctas_per_sm = ctas_per_sm;
+        if (ctas_per_sm == 0 || ctas_per_sm > 2) fail(EFS_ERR_INVALID, "ctas_per_sm must be 1 or 2");
+        b->shape(xchunk, ctas_per_sm);
     });
 }
 
@@ -749,39 +764,38 @@ efs_status efs_batch_autotune(efs_batch* b, uint32_t steps, uint32_t* xchunk, ui
         cudaEvent_t e0, e1;
         ck(cudaEventCreate(&e0), "event");
         ck(cudaEventCreate(&e1), "event");
-        float best = 1e30f;
-        uint32_t bx = b->xchunk, bc = b->ctas_per_sm;
+        const uint32_t depths[4] = {8, 16, 32, 64};
+        float best = 1e30f, own = 0.f;                   // of the candidates; of the depth the plan chooses
+        uint32_t bx = 0, bc = 0;
+        const uint32_t x0 = b->xchunk, c0 = b->ctas_per_sm;
         try {
-            b->iterate(steps);                           // warm the plan, graphs and caches once
-            for (uint32_t c : {2u, 1u})
-                for (uint32_t x : {8u, 16u, 32u, 64u}) {
-                    if (x != b->xchunk) b->planned = false;
-                    if (c != b->ctas_per_sm) b->drop_graphs();
-                    b->xchunk = x;
-                    b->ctas_per_sm = c;
-                    b->iterate(steps);                   // plan + capture outside the timed run
-                    ck(cudaEventRecord(e0, b->stream), "record");
-                    b->iterate(steps);
-                    ck(cudaEventRecord(e1, b->stream), "record");
-                    ck(cudaEventSynchronize(e1), "sync");
-                    float t = 0;
-                    ck(cudaEventElapsedTime(&t, e0, e1), "elapsed");
-                    if (t < best) { best = t; bx = x; bc = c; }
-                }
+            for (int i = 0; i < 9; ++i) {                // the plan's own depth, then the candidates
+                const uint32_t x = i ? depths[(i - 1) % 4] : 0, c = i < 5 ? 2 : 1;
+                b->shape(x, c);
+                if (i < 8) b->iterate(steps);            // warm-up (17 * steps timesteps in all)
+                b->capture(steps);                       // plan and capture outside the timed run
+                ck(cudaEventRecord(e0, b->stream), "record");
+                b->iterate(steps);
+                ck(cudaEventRecord(e1, b->stream), "record");
+                ck(cudaEventSynchronize(e1), "sync");
+                float t = 0;
+                ck(cudaEventElapsedTime(&t, e0, e1), "elapsed");
+                if (i == 0) own = t;
+                else if (t < best) { best = t; bx = x; bc = c; }
+            }
         } catch (...) {
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
+            b->shape(x0, c0);
             throw;
         }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        if (bx != b->xchunk) b->planned = false;
-        if (bc != b->ctas_per_sm) b->drop_graphs();
-        b->xchunk = bx;
-        b->ctas_per_sm = bc;
+        if (own <= best) b->shape(0, 2);
+        else b->shape(bx, bc);
         if (xchunk) *xchunk = bx;
         if (ctas_per_sm) *ctas_per_sm = bc;
-        if (ms_per_step) *ms_per_step = best / steps;
+        if (ms_per_step) *ms_per_step = std::min(own, best) / steps;
         b->sync();
     });
 }

@@ -537,6 +537,7 @@ class CudaBatch:
         self._ck(self._lib.efs_batch_sync(self._h))
 
     def setShape(self, xchunk, ctas_per_sm=2):
+        """Plane depth (0: chosen by the plan) and CTAs per SM of the core update; results do not depend on them."""
         self._ck(self._lib.efs_batch_set_shape(self._h, int(xchunk), int(ctas_per_sm)))
 
     def timePhases(self, steps=16):
@@ -548,7 +549,9 @@ class CudaBatch:
 
     def autotune(self, steps=16):
         """Pick plane depth and CTAs per SM by timing real steps (advances the
-        members by 17*steps timesteps; results are the same under every shape)."""
+        members by 17*steps timesteps; results are the same under every shape).
+        Reports the fastest candidate; where the plan's own depth is faster
+        still, the batch keeps that, and ms_per_step is its time."""
         x, c, ms = C.c_uint32(), C.c_uint32(), C.c_float()
         self._ck(self._lib.efs_batch_autotune(self._h, int(steps), C.byref(x), C.byref(c), C.byref(ms)))
         return {"xchunk": x.value, "ctas_per_sm": c.value, "ms_per_step": ms.value}

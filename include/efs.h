@@ -366,12 +366,17 @@ const char* efs_batch_last_error(const efs_batch* b);
 efs_status efs_batch_iterate(efs_batch* b, uint32_t n);
 efs_status efs_batch_sync(efs_batch* b);
 /* Plane depth (x-planes per work tile) and resident CTAs per SM (1 or 2) of
- * the persistent launch; results do not depend on them. */
+ * the persistent launch; results do not depend on them.  Depth 0 (the state
+ * of a new batch) leaves the depth to the plan, which chooses it from the
+ * members' grids. */
 efs_status efs_batch_set_shape(efs_batch* b, uint32_t xchunk, uint32_t ctas_per_sm);
 /* Autotuner: times `steps` real timesteps for each candidate shape (plane
- * depth 8/16/32/64 x 1-2 CTAs per SM), keeps the fastest and reports it.
- * The timed steps advance the members (bit-identical under every shape):
- * the batch moves forward by 17*steps timesteps in all. */
+ * depth 8/16/32/64 x 1-2 CTAs per SM) and for the depth the plan chooses
+ * itself, and keeps the fastest.  xchunk and ctas_per_sm report the fastest
+ * candidate, ms_per_step the time of the shape kept (the plan's own choice
+ * where no candidate beat it).  The timed steps advance the members
+ * (bit-identical under every shape): the batch moves forward by 17*steps
+ * timesteps in all. */
 efs_status efs_batch_autotune(efs_batch* b, uint32_t steps, uint32_t* xchunk, uint32_t* ctas_per_sm, float* ms_per_step);
 /* Diagnostics: device ms per timestep of each phase of a batched step, over
  * `steps` (1..64) timesteps launched kernel by kernel (phases as in
