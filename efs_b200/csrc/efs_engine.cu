@@ -2707,7 +2707,7 @@ efs_status efs_debug_set_wait(efs_engine* e, uint64_t wait_ns, uint32_t skip_pla
 
 efs_status efs_set_plane_depth(efs_engine* e, uint32_t xchunk) {
     return guard(e, [&] {
-        if (xchunk == 0 || xchunk > 65535) fail(EFS_ERR_INVALID, "plane depth must be in 1 .. 65535");
+        if (xchunk > 65535) fail(EFS_ERR_INVALID, "plane depth must be in 0 .. 65535");
         e->xchunk = xchunk;
         e->dirty();
     });

@@ -486,8 +486,9 @@ class CudaEngine:
         return dict(zip(PHASES, (round(v, 4) for v in ms)))
 
     def setPlaneDepth(self, xchunk):
-        """Tuning (efs_set_plane_depth): x-planes per CTA of the fused kernel
-        (default: chosen from the grid); results are bit-identical under every depth."""
+        """Tuning (efs_set_plane_depth): x-planes per CTA of the fused kernel,
+        which a depth above 0 selects on every grid; 0 (the default) leaves form
+        and depth to the engine.  Results are bit-identical under every depth."""
         self._ck(self._lib.efs_set_plane_depth(self._h, int(xchunk)))
 
     def timeCore(self, reps=10):

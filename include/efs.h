@@ -316,10 +316,13 @@ efs_status efs_time_core(efs_engine* e, uint32_t reps, float* ms);
  * (src/webgpu-engine.mjs:1129-1131). */
 efs_status efs_debug_set_wait(efs_engine* e, uint64_t wait_ns, uint32_t skip_plane);
 
-/* Tuning: x-planes each CTA of the fused kernel streams (1 .. 65535; by
- * default chosen from the grid so that its waves of CTAs fill the device).  Results are bit-identical under every depth; it moves the CTA
- * seams and trades halo re-reads against parallelism.  Kept across init.
- * No counterpart in the reference. */
+/* Tuning: x-planes each CTA of the fused kernel streams (1 .. 65535; 0, the
+ * state of a new engine: chosen from the grid so that its waves of CTAs fill
+ * the device).  Results are bit-identical under every depth; it moves the CTA
+ * seams and trades halo re-reads against parallelism.  A depth above 0 also
+ * selects the fused kernel on grids that otherwise run as E and H sweeps or
+ * whole batches of steps in one launch, which are faster there; 0 gives those
+ * forms back.  Kept across init.  No counterpart in the reference. */
 efs_status efs_set_plane_depth(efs_engine* e, uint32_t xchunk);
 
 /* Diagnostics: device time per timestep of each phase of the step, over
