@@ -817,7 +817,7 @@ struct efs_engine {
         const float* const* vfl = vflux_ptrs[p].as<const float*>();
         const float* const* cfl = cflux_ptrs[p].as<const float*>();
         const bool sweep = use_sweep(), split = pml_split() && !sweep;
-        early = sweep && pml.empty();
+        const bool early = launches_early();
 
         // --- pre-voltage ---
         if (ss_on)     // reads the fields before the UPML pre-update
@@ -1020,6 +1020,7 @@ struct efs_engine {
     }
     void launch_mur_adopt(int p) {
         const uint32_t T = 256, nb = blocks(mur_threads(), T);
+        const bool early = launches_early();
         if (indexed) launch_k(early, early ? k_mur_adopt<true, true> : k_mur_adopt<true, false>, nb, T, 0, stream, fused_grid(p), vbuf(p), mur_adopt_dev());
         else launch_k(early, early ? k_mur_adopt<false, true> : k_mur_adopt<false, false>, nb, T, 0, stream, fused_grid(p), vbuf(p), mur_adopt_dev());
     }
@@ -1068,6 +1069,7 @@ struct efs_engine {
                 enqueue_step(k, q, k + 1 == steps, ev.data() + (size_t)k * (EFS_PHASES + 1));
                 q = pnext(q);
             }
+            const bool early = launches_early();
             launch_k(early, early ? k_advance<true> : k_advance<false>, 1, 1, 0, stream, state.as<StepState>(), steps);
             ck(cudaGetLastError(), "phase run");
             sync("phase run");
@@ -1152,7 +1154,7 @@ struct efs_engine {
     // kernel ahead drains (us per timestep, early / not: cavity 5.8 / 6.1, 81^3
     // with Mur 12.9 / 14.9, dense 121x109x97 26.5 / 29.1; with UPML 86x87x71
     // 20.0 / 19.7; 256^3 287 / 253, 16 members batched 205 / 149).
-    bool early = false;              // of the step being enqueued
+    bool launches_early() const { return use_sweep() && pml.empty(); }
     bool use_sweep() const { return !xchunk && skip_plane == ~0u && (!indexed || Nd * 52 <= SWEEP_BYTES); }
     // Batches of steps that run in one launch (efs_resident.cuh): grids of a cluster's size on which
     // only the excitation and the probe ring act beside the sweeps.
@@ -1210,7 +1212,7 @@ struct efs_engine {
     // E sweep of step k, with the excitation and the probe ring samples of step k-1 (held) riding
     template <bool IDX, bool PML>
     void launch_sweep_e_k(int p, const SweepRiders& rd) {
-        launch_k(early, k_sweep_e<IDX, PML>, rd.nb + blocks(rd.ring.G, SW_T), SW_T, 0, stream, fused_grid(p), pml_set(p), pml_set(1 - p), rd);
+        launch_k(launches_early(), k_sweep_e<IDX, PML>, rd.nb + blocks(rd.ring.G, SW_T), SW_T, 0, stream, fused_grid(p), pml_set(p), pml_set(1 - p), rd);
     }
     void launch_sweep_e(int p, uint32_t k, bool exc) {
         SweepRiders rd;
@@ -1227,7 +1229,7 @@ struct efs_engine {
     }
     template <bool IDX, bool PML>
     void launch_sweep_h_k(int p) {
-        launch_k(early, k_sweep_h<IDX, PML>, sweep_blocks(), SW_T, 0, stream, fused_grid(p), pml_set(p), pml_set(1 - p));
+        launch_k(launches_early(), k_sweep_h<IDX, PML>, sweep_blocks(), SW_T, 0, stream, fused_grid(p), pml_set(p), pml_set(1 - p));
     }
     void launch_sweep_h(int p) {
         const bool hp = !pml.empty();
@@ -1315,7 +1317,7 @@ struct efs_engine {
             int q = p;
             if (resident()) launch_resident(m, p);
             else for (uint32_t k = 0; k < m; ++k) { enqueue_step(k, q, k + 1 == m); q = pnext(q); }
-            const bool adv = early && !resident();
+            const bool adv = launches_early() && !resident();
             launch_k(adv, adv ? k_advance<true> : k_advance<false>, 1, 1, 0, stream, state.as<StepState>(), m);
         } catch (...) {
             cudaStreamEndCapture(stream, &graph);
