@@ -68,7 +68,11 @@ namespace {
 // row's low slab share one access; the passes list the two slabs row by row
 // (512^3: both passes 283 -> 194 us alone; the step, with the samples and the
 // deferred H beside them, 1.583 -> 1.542 ms; either half of the change alone
-// gains nothing).
+// gains nothing).  Allocations are made before the absorber is known, so every
+// grid has the shift.  Step with and without it, us: six Mur faces 256^3 165 and
+// 178, 200x190x250 103 and 103; walls alone 320^3 283 and 280; z slabs of 6
+// cells at 256^3 200 and 225, of 12 240 and 244, of 16 245 and 241, of 32 302
+// and 298; 8 cells at 250x240x250 199 and 199; 32 filters batched 680 and 679.
 constexpr size_t FIELD_SHIFT = 32;
 // Far field: a launch's angles, its blocks (148 SMs x 2 x 6 waves), the workspace an engine keeps between calls.
 constexpr uint32_t FF_SLAB = 1u << 18, FF_BLOCKS = 1776;
@@ -554,11 +558,12 @@ struct efs_engine {
             s.r[r].ctab = R.cidx.p ? R.ctab.as<float4>() : nullptr;
             s.r[r].mate = -1;
         }
-        for (int a = 0; a < s.count; ++a)                // thin z slabs over the same rows are listed row by row
+        // z slabs over the same rows are listed row by row (FIELD_SHIFT; one region after the other / row by row, us a step at
+        // 256^3: 6 cells 211 / 200, 12 258 / 240, 20 280 / 265, 32 315 / 302, 48 380 / 363; 250x256x250: 20 274 / 260, 48 381 / 366)
+        for (int a = 0; a < s.count; ++a)
             for (int b = a + 1; b < s.count && s.r[a].mate == -1; ++b) {
                 const PmlRegion &A = s.r[a], &B = s.r[b];
-                if (B.mate == -1 && A.n[2] == B.n[2] && A.n[2] <= 16 && A.n[0] == B.n[0] && A.n[1] == B.n[1] && A.s[0] == B.s[0] &&
-                    A.s[1] == B.s[1]) {
+                if (B.mate == -1 && A.n[2] == B.n[2] && A.n[0] == B.n[0] && A.n[1] == B.n[1] && A.s[0] == B.s[0] && A.s[1] == B.s[1]) {
                     s.r[a].mate = b;
                     s.r[b].mate = -2;
                 }
