@@ -2328,6 +2328,7 @@ efs_status efs_read_nf2ff(efs_engine* e, float* accE, float* accH, size_t len) {
         if (len < n) fail(EFS_ERR_INVALID, "output buffer too small");
         if (accE) e->read_back(accE, e->nf_E.p, n * 4, "read nf2ff E");
         if (accH) e->read_back(accH, e->nf_H.p, n * 4, "read nf2ff H");
+        if (!accE && !accH) e->sync("sync");
     });
 }
 
