@@ -33,10 +33,10 @@ struct BatchMember {            // one member at one step parity (tensor maps fi
 struct BatchTile { uint32_t m, xs, y0, z0; };
 
 // Persistent: CTA b runs tiles b, b + gridDim.x, ... of a list whose members
-// all use material-index (IDX) or all dense coefficients and, if !TF, whose
-// tiles meet no TFSF face corrected in the update (with both bodies in one
+// all use dense coefficients, a material index (IDX) or varied materials (IDX and
+// VARIED) and, if !TF, whose tiles meet no TFSF face corrected in the update (with both bodies in one
 // kernel it spilled registers).
-template <bool IDX, bool TF>
+template <bool IDX, bool TF, bool VARIED>
 __global__ void __launch_bounds__(TT_THREADS, 2)
 k_fused_tma_batch(const BatchMember* __restrict__ mem, const BatchTile* __restrict__ tiles, uint32_t ntiles) {
     TmaSmem& S = tt_smem();
@@ -45,7 +45,7 @@ k_fused_tma_batch(const BatchMember* __restrict__ mem, const BatchTile* __restri
     for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const BatchTile w = tiles[t];
         const BatchMember& M = mem[w.m];
-        if (!tma_tile_body<IDX, TF>(S, TmaMaps{&M.tmH, &M.tmE, &M.tmM, &M.tmD, &M.tmE1, &M.tmH1}, M.g, w.xs, w.y0, w.z0, rg))
+        if (!tma_tile_body<IDX, TF, VARIED>(S, TmaMaps{&M.tmH, &M.tmE, &M.tmM, &M.tmD, &M.tmE1, &M.tmH1}, M.g, w.xs, w.y0, w.z0, rg))
             break;
     }
     tt_done();
@@ -199,8 +199,9 @@ struct efs_batch {
     std::vector<int> cur0;
     std::vector<uint64_t> gen;                 // the members' plans this plan was made from
     uint32_t phase = 0;
-    DevBuf members[2], tiles[4];               // tile lists by tile_class
-    uint32_t ntiles[4] = {0, 0, 0, 0};
+    static constexpr int KINDS = 3;            // of members: dense, material index, varied materials
+    DevBuf members[2], tiles[2 * KINDS];       // tile lists by tile_class
+    uint32_t ntiles[2 * KINDS] = {0, 0, 0, 0, 0, 0};
     SegLaunch ade_adopt_i[2], ade_adopt_d[2], mur_adopt_i[2], mur_adopt_d[2], mur_pre[2], mur_post[2], mur_apply[2], exc[2], tfsf_v[2], tfsf_c[2], ade_v[2], ade_c[2], ade_apply_v[2], ade_apply_c[2],
         ring[2], nf_sample[2], nf_flush[2],
         deferred_i[2], deferred_d[2], pml_e_i[2], pml_e_d[2], pml_h_i[2], pml_h_d[2], tfsf_face[2], advance;   // _i / _d: index / dense members
@@ -288,18 +289,19 @@ struct efs_batch {
         }
         return pick;
     }
-    // Tile list of a work tile: bit 0: material-index member; bit 1: the tile
-    // meets a TFSF face of the core update (the test of tma_tile).
+    // Tile list of a work tile: its member's kind, + KINDS where the tile meets
+    // a TFSF face of the core update (the test of tma_tile).
     int tile_class(const efs_engine* e, uint32_t z0) const {
         bool tf = false;
         for (uint32_t f = 0; f < e->tf.n; ++f) tf |= e->tf.z[f] >= z0 && e->tf.z[f] <= z0 + TT_Z;
-        return (e->indexed ? 1 : 0) + (tf ? 2 : 0);
+        return (e->varied ? 2 : e->indexed ? 1 : 0) + (tf ? KINDS : 0);
     }
-    template <bool IDX, bool TF>
-    void launch_tiles(int t, const BatchMember* bm) {
+    template <bool IDX, bool TF, bool VARIED>
+    void launch_tiles(const BatchMember* bm) {
+        constexpr int t = (VARIED ? 2 : IDX ? 1 : 0) + (TF ? KINDS : 0);
         if (ntiles[t])
-            launch_k(false, k_fused_tma_batch<IDX, TF>, std::min<uint32_t>(ntiles[t], ctas_per_sm * sms), TT_THREADS, TT_SMEM_BYTES, stream, 
-                bm, tiles[t].as<BatchTile>(), ntiles[t]);
+            launch_k(false, k_fused_tma_batch<IDX, TF, VARIED>, std::min<uint32_t>(ntiles[t], ctas_per_sm * sms), TT_THREADS,
+                     VARIED ? TT_SMEM_VARIED : TT_SMEM_BYTES, stream, bm, tiles[t].as<BatchTile>(), ntiles[t]);
     }
 
     void plan() {
@@ -309,7 +311,7 @@ struct efs_batch {
         xc = xchunk ? xchunk : pick_depth();
         cur0.resize(E);
         gen.resize(E);
-        for (size_t i = 0; i < E; ++i) { mem[i]->build_plan(); cur0[i] = mem[i]->cur; gen[i] = mem[i]->plan_gen; }
+        for (size_t i = 0; i < E; ++i) { mem[i]->build_plan(); mem[i]->plan_varied(); cur0[i] = mem[i]->cur; gen[i] = mem[i]->plan_gen; }
         phase = 0;
         any_nf = any_pml = false;
         for (const efs_engine* e : mem) any_pml |= e->pml_split();
@@ -465,7 +467,7 @@ struct efs_batch {
         std::vector<size_t> order(E);
         for (size_t i = 0; i < E; ++i) order[i] = i;
         std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return mem[a]->N > mem[b]->N; });
-        std::vector<BatchTile> tl[4];
+        std::vector<BatchTile> tl[2 * KINDS];
         for (size_t i : order) {
             const efs_engine* e = mem[i];
             for (uint32_t xs = 0; xs < e->Nx; xs += xc)
@@ -474,12 +476,12 @@ struct efs_batch {
         }
         // a batch of few tiles runs them all in one launch: two short ones leave two half-empty
         // last waves (16 members of 40-96 lines, 1,100 tiles: 101 us in two, 89 us in one)
-        for (int t : {0, 1})
-            if (!tl[t + 2].empty() && tl[t].size() < 4u * ctas_per_sm * sms) {
-                tl[t + 2].insert(tl[t + 2].end(), tl[t].begin(), tl[t].end());
+        for (int t = 0; t < KINDS; ++t)
+            if (!tl[t + KINDS].empty() && tl[t].size() < 4u * ctas_per_sm * sms) {
+                tl[t + KINDS].insert(tl[t + KINDS].end(), tl[t].begin(), tl[t].end());
                 tl[t].clear();
             }
-        for (int t = 0; t < 4; ++t) {
+        for (int t = 0; t < 2 * KINDS; ++t) {
             ntiles[t] = (uint32_t)tl[t].size();
             upload_raw(tiles[t], tl[t].data(), tl[t].size() * sizeof(BatchTile));
         }
@@ -516,10 +518,12 @@ struct efs_batch {
         launch_seg<OpAde>(ade_c[s], k);          // ADE(curr) before the core update rewrites H and the flux
         mark(2);
         const BatchMember* bm = members[s].as<BatchMember>();
-        launch_tiles<true, true>(3, bm);
-        launch_tiles<true, false>(1, bm);
-        launch_tiles<false, true>(2, bm);
-        launch_tiles<false, false>(0, bm);
+        launch_tiles<true, true, true>(bm);
+        launch_tiles<true, false, true>(bm);
+        launch_tiles<true, true, false>(bm);
+        launch_tiles<true, false, false>(bm);
+        launch_tiles<false, true, false>(bm);
+        launch_tiles<false, false, false>(bm);
         mark(3);
         if (pts_merge) {                         // Mur post: of members that have neither of the two
             launch_segs(seg_arg<OpPoints<1>>(tfsf_v[s], true, k), seg_arg<OpMurPost>(mur_post[s], true, k), seg_arg<OpPoints<0>>(exc[s], true, k));
@@ -713,9 +717,11 @@ efs_status efs_batch_create(efs_batch** out, efs_engine* const* engines, uint32_
         ck(cudaEventCreateWithFlags(&b->ev_done, cudaEventDisableTiming), "cudaEventCreate");
         static bool attr = false;              // the persistent kernels' dynamic shared memory, once per process
         if (!attr) {
-            for (const void* f : {(const void*)k_fused_tma_batch<true, true>, (const void*)k_fused_tma_batch<true, false>,
-                                  (const void*)k_fused_tma_batch<false, true>, (const void*)k_fused_tma_batch<false, false>})
+            for (const void* f : {(const void*)k_fused_tma_batch<true, true, false>, (const void*)k_fused_tma_batch<true, false, false>,
+                                  (const void*)k_fused_tma_batch<false, true, false>, (const void*)k_fused_tma_batch<false, false, false>})
                 ck(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT_SMEM_BYTES), "smem attr");
+            for (const void* f : {(const void*)k_fused_tma_batch<true, true, true>, (const void*)k_fused_tma_batch<true, false, true>})
+                ck(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT_SMEM_VARIED), "smem attr");
             attr = true;
         }
         b->check_members();

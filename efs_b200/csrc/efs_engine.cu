@@ -218,6 +218,8 @@ struct efs_engine {
     bool indexed = false;
     DevBuf mat, table, vv, vi, ii, iv;
     uint32_t ntable = 0;
+    bool varied = false, varied_known = false;   // plan_varied's rule; tested since the last init
+    DevBuf rows8;            // varied: the table's E and H halves in rows of 8 floats
     DevBuf state;            // StepState
     uint32_t numTS = 0;      // host mirror
     StepState hstate{};
@@ -532,6 +534,7 @@ struct efs_engine {
         g.N = Nd; g.NyNz = (size_t)Ny * Pz;
         g.V0 = vbuf(p); g.H0 = cbuf(p); g.V1 = vbuf(1 - p); g.H1 = cbuf(1 - p);
         g.mat = mat.as<uint32_t>(); g.table = table.as<float>();
+        g.rowsE = varied ? rows8.as<float>() : nullptr; g.rowsH = varied ? g.rowsE + (size_t)ntable * 8 : nullptr;
         g.vv = vv.as<float>(); g.vi = vi.as<float>(); g.ii = ii.as<float>(); g.iv = iv.as<float>();
         g.status = d_status;
         g.wait_ns = wait_ns;
@@ -635,6 +638,7 @@ struct efs_engine {
         plan_ade_adopt();
         plan_ring();
         plan_resident();
+        if (!use_sweep()) plan_varied();
         tails = pml_split() ? tails_clear(false) : 0;
         build_deferred();
         mark_adopted();
@@ -1123,15 +1127,15 @@ struct efs_engine {
         if (r != CUDA_SUCCESS) fail(EFS_ERR_CUDA, "cuTensorMapEncodeTiled failed (code " + std::to_string((int)r) + ")");
         return m;
     }
-    template <bool IDX>
+    template <bool IDX, bool VARIED>
     void launch_fused_tma_k(dim3 g, const CUtensorMap (&t)[6], const FusedGrid& fg) {
+        constexpr size_t smem = VARIED ? TT_SMEM_VARIED : TT_SMEM_BYTES;
         static bool attr_set = false;   // per instantiation; the attribute is per kernel, all devices alike
         if (!attr_set) {
-            ck(cudaFuncSetAttribute(k_fused_tma<IDX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TT_SMEM_BYTES),
-               "smem attr");
+            ck(cudaFuncSetAttribute(k_fused_tma<IDX, VARIED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
             attr_set = true;
         }
-        launch_k(false, k_fused_tma<IDX>, g, TT_THREADS, TT_SMEM_BYTES, stream, t[0], t[1], t[2], t[3], t[4], t[5], fg);
+        launch_k(false, k_fused_tma<IDX, VARIED>, g, TT_THREADS, smem, stream, t[0], t[1], t[2], t[3], t[4], t[5], fg);
     }
     void launch_fused_tma(int p) {
         const FusedGrid fg = fused_grid(p);
@@ -1143,8 +1147,9 @@ struct efs_engine {
                                   tensor_map(fg.V1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs),
                                   tensor_map(fg.H1, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bs)};
         dim3 g(blocks(Nz, TT_Z), blocks(Ny, TT_Y), blocks(Nx, fg.xchunk));
-        if (indexed) launch_fused_tma_k<true>(g, t, fg);
-        else launch_fused_tma_k<false>(g, t, fg);
+        if (varied) launch_fused_tma_k<true, true>(g, t, fg);
+        else if (indexed) launch_fused_tma_k<true, false>(g, t, fg);
+        else launch_fused_tma_k<false, false>(g, t, fg);
     }
     // E and H sweeps (efs_sweep.cuh) instead of the fused kernel and the passes
     // around it: while both parities of the fields and the material index stay
@@ -1161,6 +1166,41 @@ struct efs_engine {
     // 20.0 / 19.7; 256^3 287 / 253, 16 members batched 205 / 149).
     bool launches_early() const { return use_sweep() && pml.empty(); }
     bool use_sweep() const { return !xchunk && skip_plane == ~0u && (!indexed || Nd * 52 <= SWEEP_BYTES); }
+    // The fused kernel's form for varied materials: a table larger than L1 keeps for the other form, and most cells with
+    // another material than their x-1 neighbour, or an eighth of them with one far from every neighbour's (the other form
+    // keeps the coefficients of materials that stay; figures at tma_tile_body).  Tested when the fused kernel is planned, once per init.
+    static constexpr uint32_t VARIED_ROWS = 448;
+    void plan_varied() {
+        if (varied_known) return;
+        varied = false;
+        if (indexed && ntable >= VARIED_ROWS) {
+            DevBuf cnt;
+            alloc(cnt, 16);
+            k_varied<<<(unsigned)std::min<size_t>(blocks(Nd, 256), 148 * 8), 256, 0, stream>>>(mat.as<uint32_t>(), Nx, Ny, Nz, Pz,
+                                                                                               cnt.as<unsigned long long>());
+            ck(cudaGetLastError(), "material test");
+            unsigned long long n[2] = {0, 0};
+            ck(cudaMemcpyAsync(n, cnt.p, 16, cudaMemcpyDeviceToHost, stream), "material test");
+            sync("material test");
+            varied = 4 * n[0] >= 3 * N || 8 * n[1] >= N;
+        }
+        if (varied) {
+            try {
+                alloc(rows8, (size_t)ntable * 64, false);
+            } catch (const EfsError& err) {
+                if (err.code != EFS_ERR_OOM) throw;
+                cudaGetLastError();                        // no room: the other form
+                varied = false;
+            }
+        }
+        if (varied) {
+            float* E = rows8.as<float>();
+            k_table_rows<<<(unsigned)std::min<size_t>(blocks((size_t)ntable * 16, 256), 148 * 8), 256, 0, stream>>>(
+                table.as<float>(), ntable, E, E + (size_t)ntable * 8);
+            ck(cudaGetLastError(), "table rows");
+        }
+        varied_known = true;
+    }
     // Batches of steps that run in one launch (efs_resident.cuh): grids of a cluster's size on which
     // only the excitation and the probe ring act beside the sweeps.
     uint32_t resident_threads() const { return std::max(32u, blocks((uint32_t)(Nd / 2), 32 * RS_CTAS) * 32); }
@@ -1403,6 +1443,8 @@ void alloc_fields(efs_engine* e, const uint32_t dims[3]) {
     e->en_pending = false; e->en_last = 0.0; e->en_idx = 0;
     e->en_partial.reset(); e->en_result.reset();
     e->vv.reset(); e->vi.reset(); e->ii.reset(); e->iv.reset(); e->mat.reset(); e->table.reset();
+    e->rows8.reset();
+    e->varied = e->varied_known = false;
 }
 
 // FNV-1a over the 48-byte tuple
@@ -2788,7 +2830,7 @@ efs_status efs_kernels_per_step(efs_engine* e, uint32_t* out) {
 efs_status efs_device_bytes(const efs_engine* e, size_t* out) {
     if (!e || !out) return EFS_ERR_INVALID;
     size_t t = 0;
-    const DevBuf* all[] = {&e->volt, &e->curr, &e->volt_b, &e->curr_b, &e->defer_cells, &e->mat, &e->table, &e->vv, &e->vi, &e->ii, &e->iv};
+    const DevBuf* all[] = {&e->volt, &e->curr, &e->volt_b, &e->curr_b, &e->defer_cells, &e->mat, &e->table, &e->rows8, &e->vv, &e->vi, &e->ii, &e->iv};
     for (auto* b : all) t += b->bytes;
     for (auto& r : e->pml) {
         const DevBuf* rb[] = {&r->vv, &r->vvfo, &r->vvfn, &r->ii, &r->iifo, &r->iifn, &r->vflux, &r->cflux, &r->vflux_b, &r->cflux_b};

@@ -40,6 +40,7 @@ struct FusedGrid {
     const float* V0; const float* H0;   // fields at the start of the step
     float* V1; float* H1;               // fields after the step
     const uint32_t* mat; const float* table;   // mat: null with dense coefficients and no adopted cell
+    const float* rowsE; const float* rowsH;    // the table's E and H halves in rows of 8 floats (varied materials, else null)
     const float* vv; const float* vi; const float* ii; const float* iv;
     uint32_t* status;                   // device status word (bit 0: a bounded wait ran out)
     uint64_t wait_ns;                   // limit of every bounded mbarrier wait (about 1 s)
@@ -135,6 +136,39 @@ __device__ __forceinline__ float core_e(const FusedGrid& g, uint32_t f, float v)
         ci = __ldg(g.vi + f);
     }
     return upd(v, cv, ci, curl);
+}
+
+// Varied materials (tma_tile_body's VARIED): how many cells have another material
+// than their x-1 neighbour (out[0]), and how many of these lie more than two
+// table rows from their y-1 and their z-1 neighbour's too (out[1]).
+__global__ void __launch_bounds__(256) k_varied(const uint32_t* __restrict__ mat, uint32_t Nx, uint32_t Ny, uint32_t Nz, uint32_t Pz,
+                                                unsigned long long* out) {
+    const uint32_t plane = Ny * Pz, n = Nx * plane;
+    auto far = [](uint32_t a, uint32_t b) { return a > b ? a - b > 2u : b - a > 2u; };
+    uint32_t chg = 0, scat = 0;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t c = (uint32_t)i, x = c / plane, r = c - x * plane, y = r / Pz, z = r - y * Pz;
+        if (x == 0 || z >= Nz) continue;
+        const uint32_t m = mat[c] & MAT_MASK;
+        if (m == (mat[c - plane] & MAT_MASK)) continue;
+        ++chg;
+        scat += y > 0 && z > 0 && far(m, mat[c - Pz] & MAT_MASK) && far(m, mat[c - 1] & MAT_MASK);
+    }
+    for (int o = 16; o; o >>= 1) {
+        chg += __shfl_xor_sync(0xffffffffu, chg, o);
+        scat += __shfl_xor_sync(0xffffffffu, scat, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(out, (unsigned long long)chg);
+        atomicAdd(out + 1, (unsigned long long)scat);
+    }
+}
+// The halves of the table as rows of 8 floats (vv0 vv1 vv2 vi0 vi1 vi2 0 0, and ii, iv).
+__global__ void k_table_rows(const float* __restrict__ table, uint32_t n, float* __restrict__ E, float* __restrict__ H) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n * 16; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t r = i / 16, q = i % 16, k = q % 8;
+        (q < 8 ? E : H)[r * 8 + k] = k < 6 ? table[r * 12 + (q < 8 ? 0 : 6) + k] : 0.f;
+    }
 }
 
 // Adopt bits of the material index (one launch per UPML region; Mur targets; ADE cells).

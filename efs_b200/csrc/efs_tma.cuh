@@ -39,6 +39,7 @@
 #pragma once
 #include "efs_fused.cuh"
 #include <cuda.h>
+#include <cstddef>
 
 namespace efs {
 
@@ -74,15 +75,21 @@ struct TmaStage {
 struct TmaSmem {
     TmaStage st[TT_S];
     alignas(128) float En[2][TT_ENEW];   // E_new of planes x and x-1
-    alignas(128) float Hn[2][3 * TT_EC]; // H_new of planes x-1 and x-2, as the store box has them
     alignas(8) unsigned long long full[TT_S];
+    alignas(128) float Hn[2][3 * TT_EC]; // H_new of planes x-1 and x-2, as the store box has them (not with varied materials)
 };
 constexpr size_t TT_SMEM_BYTES = sizeof(TmaSmem) + 128;   // + slack to align the base to 128 B
+constexpr size_t TT_SMEM_VARIED = offsetof(TmaSmem, Hn) + 128;
 static_assert(2 * (TT_SMEM_BYTES + 1024) <= 228 * 1024, "two CTAs per SM");
+static_assert(2 * (TT_SMEM_VARIED + 1024) <= 196 * 1024, "two CTAs per SM and 60 KB of L1");
 
 // What a CTA keeps across the tiles it runs back to back: the stage and its
 // mbarrier phase of the next plane, and the E_new / H_new buffer it writes.
-struct TmaRing { uint32_t s = 0, ph = 0, b = 0; };
+struct TmaRing {
+    uint32_t s = 0, ph = 0, b = 0;
+    __device__ uint32_t next() const { return s + 1 == TT_S ? 0u : s + 1; }                  // of the plane after it
+    __device__ uint32_t next_ph() const { return s + 1 == TT_S ? ph ^ 1u : ph; }
+};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -236,6 +243,27 @@ __device__ __forceinline__ PairCoef pair_rows(const float* table, uint2 m) {
     }
     return k;
 }
+// The rows of a pair's cells in one half of the table (rows of 8 floats, one
+// 32-byte load each), and the pair's coefficients from them.
+struct PairRows { float a[6], b[6]; };
+__device__ __forceinline__ void ldg_row8(const float* rows, uint32_t m, float v[6]) {
+    float pad0, pad1;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(pad0), "=f"(pad1)
+        : "l"(rows + (size_t)(m & MAT_MASK) * 8));
+}
+__device__ __forceinline__ PairRows pair_rows8(const float* rows, uint2 m) {
+    PairRows r;
+    ldg_row8(rows, m.x, r.a);
+    ldg_row8(rows, m.y, r.b);
+    return r;
+}
+__device__ __forceinline__ PairCoef pair_pack(const PairRows& r) {
+    PairCoef k;
+#pragma unroll
+    for (int n = 0; n < 3; ++n) { k.v[n] = pk2(r.a[n], r.b[n]); k.i[n] = pk2(r.a[3 + n], r.b[3 + n]); }
+    return k;
+}
 // All ones in the halves of a pair (material indices m) whose component n is adopted.
 __device__ __forceinline__ f32x2 adopt_mask(uint2 m, int n) {
     const uint32_t lo = 0u - (m.x >> (MAT_BITS + n) & 1u), hi = 0u - (m.y >> (MAT_BITS + n) & 1u);
@@ -273,8 +301,17 @@ __device__ __forceinline__ PairCoef pair_dense(const float* v, const float* i, s
 //   the refill of the stage of plane x-1 and the stores of E_new(x-1), H_new(x-2).
 // A pair's coefficients stay in registers while its material does not change
 // along x.
-//
-template <bool IDX, bool TF>
+// VARIED (materials of a large table that change at most planes; the rule is
+// efs_engine::plan_varied): the rows of plane x+1 are fetched at the end of plane
+// x, once that plane has arrived, so their latency is not on the chain from a
+// plane's arrival to its barrier, as one 32-byte load per row and side instead of
+// two 16-byte loads; and H leaves straight from registers, which gives up the H
+// planes in shared memory for an L1 of 60 KB instead of 28 (L1 lines bound the
+// row misses in flight).  256^3, us a launch, VARIED / not: 1024 random materials
+// 242 / 451, 64 K 286 / 509, 1 M 493 / 922, 64 K graded in x and z 194 / 218, a
+// row per 1x2x2 cells 205 / 216; 512 random 209 / 238, 384 random 204 / 192, one
+// material 153 / 141.
+template <bool IDX, bool TF, bool VARIED>
 __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, const FusedGrid& g, uint32_t xs,
                                               uint32_t y0, uint32_t z0, TmaRing& rg) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -302,21 +339,26 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
         float hp = in ? g.H0[(size_t)(xs > 0 ? xs - 1 : 0) * NyNz + 2 * N + off] : 0.f;   // Hz(x-1)
         float kc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};        // dense coefficients, loaded a plane ahead
         if (!IDX && in) coeffs_f<false>(g, (size_t)xs * NyNz + off, 0u, 0, kc);
+        uint32_t m = 0;                                      // the cell's material (VARIED: fetched a plane ahead)
+        if (VARIED && mbar_wait_bounded(smem_u32(&S.full[rg.s]), rg.ph, g.wait_ns) && has) {
+            m = (&S.st[rg.s].M[0][0])[ei];
+            ldg_row8(g.rowsE, m, kc);
+        }
         bool out = false;
         for (int k = 0; k < nk; ++k) {
             if (k > 0 && lane == 0) {                        // planes of the interval before: E(x-1), H(x-2)
                 tma_store_4d(tm.E1, S.En[rg.b ^ 1u], (int)z0, (int)y0, (int)(xs + k) - 1, 0);
-                if (k > 1) tma_store_4d(tm.H1, S.Hn[rg.b ^ 1u], (int)z0, (int)y0, (int)(xs + k) - 2, 0);
+                if (!VARIED && k > 1) tma_store_4d(tm.H1, S.Hn[rg.b ^ 1u], (int)z0, (int)y0, (int)(xs + k) - 2, 0);
                 tma_store_commit();
             }
             __syncwarp();
-            const bool ok = mbar_wait_bounded(smem_u32(&S.full[rg.s]), rg.ph, g.wait_ns);
+            bool ok = mbar_wait_bounded(smem_u32(&S.full[rg.s]), rg.ph, g.wait_ns);
             if (ok && has) {
                 const TmaStage& st = S.st[rg.s];
                 const float* Hs = &st.H[0][0][0];
                 const float* Es = &st.E[0][0][0];
-                const uint32_t m = mats ? (&st.M[0][0])[ei] : 0u;
-                if (IDX) coeffs_f<true>(g, 0, m, 0, kc);
+                if (!VARIED) m = mats ? (&st.M[0][0])[ei] : 0u;
+                if (IDX && !VARIED) coeffs_f<true>(g, 0, m, 0, kc);
                 const float hz = Hs[2 * HPL + hi], ex0 = Es[ei], ey0 = Es[EPL + ei];
                 float ex = upd(ex0, kc[0], kc[3], curl4(hz, Hs[2 * HPL + hy_], Hs[HPL + hi], Hs[HPL + hi - 1]));
                 float ey = upd(ey0, kc[1], kc[4], curl4(Hs[hi], Hs[hi - 1], hz, hp));
@@ -328,6 +370,13 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
                 hp = hz;
                 if (!IDX && in && k + 1 < nk) coeffs_f<false>(g, (size_t)(xs + k + 1) * NyNz + off, 0u, 0, kc);
             }
+            if (VARIED && ok && k + 1 < nk) {
+                ok = mbar_wait_bounded(smem_u32(&S.full[rg.next()]), rg.next_ph(), g.wait_ns);
+                if (ok && has) {
+                    m = (&S.st[rg.next()].M[0][0])[ei];
+                    ldg_row8(g.rowsE, m, kc);
+                }
+            }
             if (lane == 0) tma_store_wait_read();            // the buffers written in the next interval are free
             __syncwarp();
             out = __syncthreads_or(!ok) != 0;
@@ -337,7 +386,7 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
         }
         if (!out && lane == 0) {                             // the last plane (E only if owned) and H before it
             if (xl < xe) tma_store_4d(tm.E1, S.En[rg.b ^ 1u], (int)z0, (int)y0, (int)xl, 0);
-            if (nk > 1) tma_store_4d(tm.H1, S.Hn[rg.b ^ 1u], (int)z0, (int)y0, (int)xl - 1, 0);
+            if (!VARIED && nk > 1) tma_store_4d(tm.H1, S.Hn[rg.b ^ 1u], (int)z0, (int)y0, (int)xl - 1, 0);
             tma_store_commit();
         }
         __syncwarp();
@@ -386,12 +435,18 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
     bool chg = false;                                        // it changed from plane x-2 to x-1
     f32x2 ad[3] = {0ull, 0ull, 0ull};                        // the pair's adopted components, as bit masks
     if (!IDX) ke = pair_dense(g.vv, g.vi, N, cell, in);
+    PairRows re, rh;                                         // VARIED: rows of E(x) and H(x-1), and the pair's material at x
+    uint2 mv = make_uint2(0u, 0u);
+    if (VARIED && mbar_wait_bounded(smem_u32(&S.full[rg.s]), rg.ph, g.wait_ns)) {
+        mv = *reinterpret_cast<const uint2*>(&S.st[rg.s].M[0][0] + ei);
+        re = pair_rows8(g.rowsE, mv);
+    }
     bool timed_out = false;
     int k = 0;
 
     for (; k < nk; ++k) {
-        if (IDX && chg) kh = pair_rows<6>(g.table, mp);      // H(x-1): known before the plane arrives
-        const bool ok = mbar_wait_bounded(smem_u32(&S.full[rg.s]), rg.ph, g.wait_ns);
+        if (IDX && !VARIED && chg) kh = pair_rows<6>(g.table, mp);      // H(x-1): known before the plane arrives
+        bool ok = mbar_wait_bounded(smem_u32(&S.full[rg.s]), rg.ph, g.wait_ns);
         if (ok) {
             const TmaStage& st = S.st[rg.s];
             const float* Hs = &st.H[0][0][0];
@@ -400,7 +455,12 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
             const float* Ep = S.En[rg.b ^ 1u];
             f32x2 hc[3], en[3];
             // ---- E_new(x) of the pair
-            if (mats) {
+            if (VARIED) {
+                ke = pair_pack(re);
+                if (own && k > 0) kh = pair_pack(rh);
+#pragma unroll
+                for (int n = 0; n < 3; ++n) ad[n] = adopt_mask(mv, n);
+            } else if (mats) {
                 const uint2 mc = *reinterpret_cast<const uint2*>(&st.M[0][0] + ei);
                 chg = k == 0 || mc.x != mp.x || mc.y != mp.y;
                 if (chg) {
@@ -443,8 +503,17 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
                         const uint32_t m = y + 1 >= Ny ? 3u : (z + 1 >= Nz ? 1u : 0u) | (z + 2 >= Nz ? 2u : 0u);
                         hn[0] = pick2(hn[0], hp[0], m); hn[1] = pick2(hn[1], hp[1], m); hn[2] = pick2(hn[2], hp[2], m);
                     }
-                    float* Hn = S.Hn[rg.b];                  // UPML cells among them are rewritten by k_pml_h
-                    st2(Hn + si, hn[0]); st2(Hn + TT_EC + si, hn[1]); st2(Hn + 2 * TT_EC + si, hn[2]);
+                    if (!VARIED) {                           // UPML cells among them are rewritten by k_pml_h
+                        float* Hn = S.Hn[rg.b];
+                        st2(Hn + si, hn[0]); st2(Hn + TT_EC + si, hn[1]); st2(Hn + 2 * TT_EC + si, hn[2]);
+                    } else if (in) {
+                        float* H1 = g.H1 + (cell - NyNz);
+                        if (z + 1 < Nz) {
+                            st2(H1, hn[0]); st2(H1 + N, hn[1]); st2(H1 + 2 * N, hn[2]);
+                        } else {                             // the pair's second cell is padding
+                            H1[0] = lo2(hn[0]); H1[N] = lo2(hn[1]); H1[2 * N] = lo2(hn[2]);
+                        }
+                    }
                 }
             } else if (loader && k > 0 && issued < nk) {
                 if (xs + issued != g.skip_plane)             // plane k-1+TT_S into the stage of plane k-1
@@ -458,6 +527,17 @@ __device__ __forceinline__ bool tma_tile_body(TmaSmem& S, const TmaMaps& tm, con
             }
 #pragma unroll
             for (int n = 0; n < 3; ++n) { hp[n] = hc[n]; ep[n] = en[n]; }
+            if (VARIED) {                // rows of H(x) and, once its material has arrived, of E(x+1)
+                cell += NyNz;
+                if (own) rh = pair_rows8(g.rowsH, mv);
+                if (k + 1 < nk) {
+                    ok = mbar_wait_bounded(smem_u32(&S.full[rg.next()]), rg.next_ph(), g.wait_ns);
+                    if (ok) {
+                        mv = *reinterpret_cast<const uint2*>(&S.st[rg.next()].M[0][0] + ei);
+                        re = pair_rows8(g.rowsE, mv);
+                    }
+                }
+            }
         }
         // every read of the stage and of E_new(x-1) and every write of the plane buffers done; agree on a timeout
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the plane buffers' writes before their TMA stores
@@ -493,12 +573,12 @@ __device__ __forceinline__ void tt_done() {
     if (threadIdx.x == 32 * (TT_Y + 1)) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 // A TFSF face corrected in the core update meets the tile's columns (halo column included).
-template <bool IDX>
+template <bool IDX, bool VARIED>
 __device__ __forceinline__ bool tma_tile(TmaSmem& S, const TmaMaps& tm, const FusedGrid& g, uint32_t xs, uint32_t y0, uint32_t z0,
                                          TmaRing& rg) {
     bool tf = false;
     for (uint32_t f = 0; f < g.tf.n; ++f) tf |= g.tf.z[f] >= z0 && g.tf.z[f] <= z0 + TT_Z;
-    return tf ? tma_tile_body<IDX, true>(S, tm, g, xs, y0, z0, rg) : tma_tile_body<IDX, false>(S, tm, g, xs, y0, z0, rg);
+    return tf ? tma_tile_body<IDX, true, VARIED>(S, tm, g, xs, y0, z0, rg) : tma_tile_body<IDX, false, VARIED>(S, tm, g, xs, y0, z0, rg);
 }
 
 // Bound by DRAM on large grids (512^3: 1.114 ms a launch at 24 planes per CTA
@@ -511,7 +591,7 @@ __device__ __forceinline__ bool tma_tile(TmaSmem& S, const TmaMaps& tm, const Fu
 // registers: same time at 512^3, 4% slower at 256^3), loops unrolled 2 or 4
 // planes deep (slower: instruction fetch), TMA boxes without halo columns
 // (no change).
-template <bool IDX>
+template <bool IDX, bool VARIED>
 __global__ void __launch_bounds__(TT_THREADS, 2)
 k_fused_tma(const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmE,
             const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmD,
@@ -521,7 +601,7 @@ k_fused_tma(const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUt
     TmaSmem& S = tt_smem();
     tt_init(S);
     TmaRing rg;
-    (void)tma_tile<IDX>(S, TmaMaps{&tmH, &tmE, &tmM, &tmD, &tmE1, &tmH1}, g, xs, blockIdx.y * TT_Y, blockIdx.x * TT_Z, rg);
+    (void)tma_tile<IDX, VARIED>(S, TmaMaps{&tmH, &tmE, &tmM, &tmD, &tmE1, &tmH1}, g, xs, blockIdx.y * TT_Y, blockIdx.x * TT_Z, rg);
     tt_done();
 }
 
