@@ -74,7 +74,8 @@ namespace {
 // cells at 256^3 200 and 225, of 12 240 and 244, of 16 245 and 241, of 32 302
 // and 298; 8 cells at 250x240x250 199 and 199; 32 filters batched 680 and 679.
 constexpr size_t FIELD_SHIFT = 32;
-// Far field: a launch's angles, its blocks (148 SMs x 2 x 6 waves), the workspace an engine keeps between calls.
+// Far field: a launch's angles, about its blocks (12 per SM: four rounds of the three that fit), the workspace an engine
+// keeps between calls.
 constexpr uint32_t FF_SLAB = 1u << 18, FF_BLOCKS = 1776;
 constexpr size_t FF_KEEP = (size_t)64 << 20;
 constexpr size_t SWEEP_BYTES = (size_t)92 << 20;   // fields and material index of the largest grid that runs as sweeps
@@ -1431,7 +1432,6 @@ void alloc_fields(efs_engine* e, const uint32_t dims[3]) {
     e->tf = TfsfFace{0, {0, 0}};
     e->tf_n = 0;
     e->defer_n = 0;
-    // plane depth (x-planes per CTA) of the fused kernel; results do not depend on it
     e->cur = 0;
     e->alloc(e->volt, 3 * Nd * sizeof(float), true, FIELD_SHIFT);
     e->alloc(e->curr, 3 * Nd * sizeof(float), true, FIELD_SHIFT);

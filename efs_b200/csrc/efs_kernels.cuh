@@ -49,7 +49,7 @@ struct PmlRegion {
 // and so for y and z (zero beyond the grid), so the regions of a cell are three
 // loads that issue with its field loads.  (Walking the regions' bounds took
 // longer than the loads they gate: 86 x 87 x 71 with UPML on all faces.)
-constexpr uint32_t PML_AXIS_PAD = 80;   // zeros behind each axis: tiles overhang the grid
+constexpr uint32_t PML_AXIS_PAD = 1;    // zeros behind each axis: a pair's second cell may lie one beyond z
 struct PmlSet {
     int count;
     const uint32_t* xm; const uint32_t* ym; const uint32_t* zm;
@@ -770,7 +770,8 @@ __global__ void __launch_bounds__(256) k_energy_ranges(const float* __restrict__
 // Splitting the records over blocks is what a pattern of few angles needs
 // (61 x 73 angles filled 70 blocks, each with all points in series).
 //
-// Bound by the FMA pipe (70% active; 24 of its slots per angle and point).
+// Bound by the FMA pipe (72% active, ncu; 24 of its slots per angle and point;
+// the special-function pipe 50%, issue 48%).
 // Measured on B200, device time: 65,341 angles x 334,176 points 30.9 -> 20.5
 // ms, 4,453 angles x 22,410 points 0.34 -> 0.14 ms.
 // ---------------------------------------------------------------------------

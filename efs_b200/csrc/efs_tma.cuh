@@ -21,9 +21,9 @@
 // buffers, and the thread's own E_new(x).
 //
 // E values known before this kernel (UPML cells by k_pml_e, Mur targets by
-// k_mur_adopt) are staged in place of E_old and adopted as is where the
-// material index says so.  H of UPML cells is provisional here and rewritten
-// by k_pml_h.
+// k_mur_adopt, applied media by k_ade_adopt) are staged in place of E_old and
+// adopted as is where the material index says so.  H of UPML cells is
+// provisional here and rewritten by k_pml_h.
 //
 // Boundaries follow the reference's index-0 self reference: the x-1, y-1 and
 // z-1 neighbours of index 0 are the cell itself (the TMA zero fill outside

@@ -302,7 +302,9 @@ efs_status efs_debug_read(efs_engine* e, const char* name, uint32_t arg, float* 
 /* Diagnostics: launch the engine's core field-update kernels `reps` times
  * on its stream and return the mean device time per launch (CUDA events):
  * ms[0] = the fused E+H kernel, ms[1] = the UPML-cell passes around it (0
- * without UPML regions).  Advances the fields; meant for benchmarks only.
+ * without UPML regions); on a grid that runs as E and H sweeps, ms[0] = both
+ * sweeps, UPML cells included, also where efs_iterate runs all steps of a
+ * batch in one launch instead.  Advances the fields; meant for benchmarks only.
  * No counterpart in the reference. */
 efs_status efs_time_core(efs_engine* e, uint32_t reps, float* ms);
 
@@ -332,10 +334,12 @@ efs_status efs_set_plane_depth(efs_engine* e, uint32_t xchunk);
  *   0 steady-state accumulation and the UPML E pass (with the previous
  *     step's NF2FF samples in the same launch when they are paired),
  *   1 point operations before the core update (ADE, Mur pre, RLC pre),
- *   2 fused core update, 3 E-side point operations (TFSF, PBC, Mur
+ *   2 fused core update (or E sweep), 3 E-side point operations (TFSF, PBC, Mur
  *     post/apply, excitation, RLC, ADE apply), 4 UPML H pass and deferred H
- *     recompute (one launch), 5 H-side point operations, 6 NF2FF samples /
+ *     recompute (one launch; or H sweep), 5 H-side point operations, 6 NF2FF samples /
  *     accumulation and probe ring.
+ * A grid that efs_iterate steps in one launch per batch of steps is timed as
+ * E and H sweeps here (the same bits; its own steps are shorter).
  * No counterpart in the reference. */
 #define EFS_PHASES 7
 efs_status efs_time_phases(efs_engine* e, uint32_t steps, float* ms);

@@ -78,6 +78,24 @@ def test_batch_of_all_kinds(cuda_engine_cls, what):
         b.destroy()
 
 
+@pytest.mark.parametrize("plane", [0, 5, 19])
+def test_wait_runs_out_and_device_recovers(cuda_engine_cls, plane):
+    """A plane whose loads are never issued (efs_debug_set_wait, as in test_gpu_timeout.py): the waits give up by design."""
+    from efs_b200.engine import EfsError
+    N = (20, 18, 24)
+    g, o = build(cuda_engine_cls, N, "scattered", "plain", 0)
+    g.debugSetWait(2_000_000, skip_plane=plane)
+    g.iterate(1)
+    with pytest.raises(EfsError) as err:
+        g.sync()
+    assert err.value.code == 5                # EFS_ERR_TIMEOUT
+    g.debugSetWait()
+    fresh, o = build(cuda_engine_cls, N, "scattered", "plain", 6)
+    fresh.iterate(6)
+    o.iterate(6)
+    compare_fields(fresh, o, "after a timed-out wait on this device")
+
+
 def test_scattered_materials_cost_their_rows(cuda_engine_cls):
     """150^3, core update alone: a row of every cell and side read from L2 each step moves 1.7 times a constant material's
     52 bytes a cell (the rows' two 32-byte sectors, halos included), so 2.8 times its time leaves room for their latency."""
